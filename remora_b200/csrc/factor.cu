@@ -385,8 +385,9 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s) {
     if (n <= 0) return RC_SUCCESS;
     T* W = static_cast<T*>(workspace(s, (size_t)NB * NB * sizeof(T), 1));
     if (!W) return RC_ERR_ALLOC;
-    // FP64 panels run on the 128x128 DMMA tile, so one CTA owns every column of a panel
-    // row block and the panel solve can write in place; other types go through a buffer.
+    // An in-place FP64 product runs on a DMMA tile that spans the panel's 128 columns, so one
+    // CTA owns every column of its rows and the panel solve can write in place; other types
+    // go through a buffer.
     constexpr bool in_place = std::is_same<T, double>::value;
     T* tmp = nullptr;
     if (!in_place) {

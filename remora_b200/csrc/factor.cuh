@@ -5,7 +5,8 @@
 namespace rc {
 
 // Block size of the blocked TRSM / POTRF: one diagonal block per CTA, and the width of
-// the panel GEMMs (equal to the FP64 DMMA tile so in-place panel updates are race free).
+// the panel GEMMs (no wider than the in-place FP64 DMMA tiles, whose CTAs each own whole rows
+// or columns of what they overwrite).
 constexpr int kNB = 128;
 
 // Writes v into *info if *info is 0 or larger than v (first failing index wins).

@@ -5,18 +5,17 @@
 // include/remora/kernels/hip/gemm.hpp:46-112 and kernels/hip/syrk.hpp:44-85).
 //
 // Two kernels:
-//  * gemm_dmma_f64: the FP64 tensor-core path (DMMA, mma.sync m16n8k4 f64). 128x128x16
-//    CTA tiles, 8 warps of 64x32, a 3-stage cp.async pipeline. Operand tiles are staged
-//    in shared memory in one canonical layout ([k][m] and [k][n], rows padded by 4
-//    doubles so every fragment load of a half-warp hits 16 distinct 8-byte bank pairs);
-//    the transposition that a K-major operand needs happens in the 8-byte cp.async
-//    scatter, so all four transpose combinations share one inner loop.
+//  * gemm_dmma_f64: the FP64 tensor-core path (DMMA, mma.sync m16n8k4 f64), a family of
+//    CTA tiles from 128 x 128 down to 32 x 32 over one kernel template. Operand tiles are
+//    staged by 16-byte cp.async (8-byte where the alignment asks for it) in the order of
+//    their global layout, so all four transpose combinations run at the same rate.
 //  * gemm_simt: a generic strided FP32/FP64 kernel (64x64x16 tiles, 4x4 outer products
 //    per thread) for operands with no unit stride and for FP32.
 // Both honour a triangle mask (SYRK writes one triangle; whole tiles outside it exit at
 // once) and an abort word (a failed Cholesky pivot stops the trailing updates).
 #include "gemm.cuh"
 #include "tc_gemm.cuh"
+#include <cmath>
 #include <type_traits>
 
 namespace rc {
@@ -93,91 +92,119 @@ __global__ void __launch_bounds__(256) gemm_simt(int64_t m, int64_t n, int64_t k
 }
 
 // ------------------------------------------------------------------------------------
-// FP64 DMMA kernel: 128 x BN tiles (BN = 128 or 64 for skinny right-hand sides), k-step 16
-// staged through a 4-deep cp.async ring,
-// 8 warps. gridDim.z > 1 splits K: slice z covers [z * kchunk, (z + 1) * kchunk) and
-// writes its partial product (alpha = 1, beta = 0) to Cz + z * zstride; a second kernel
-// then reduces the slices into C.
-constexpr int DM = 128, DK = 16, DSTAGES = 4, DPAD = 4;
-constexpr int DLDA = DM + DPAD;
+// FP64 DMMA kernel. Tiles of BM x BN by a k-step of 16 staged through a cp.async ring, one
+// warp tile of 16 MI x 8 NI per warp. The pipe does 64 FMA per SM and cycle (36.9 TFLOP/s
+// measured on registers alone), so what a shape reaches depends on how evenly its tiles
+// load the SMs and on what a tile spends outside its k loop; pick_tile weighs both.
+// gridDim.z > 1 splits K: slice z covers [z * kchunk, (z + 1) * kchunk) and writes its
+// partial product (alpha = 1, beta = 0) to Cz + z * zstride; a second kernel then reduces
+// the slices into C.
+constexpr int DK = 16;
+constexpr int DKP = DK + 4;  // row stride of a K-major tile (doubles)
 
-template <int BN>
-struct DmmaCfg {
-    static constexpr int LDB = BN + DPAD;
-    static constexpr int WARPS_N = BN == 128 ? 4 : 2;  // warps along N
-    static constexpr int WARPS_M = 8 / WARPS_N;
-    static constexpr int WM = DM / WARPS_M, WN = BN / WARPS_N;  // warp tile
+template <int BM_, int BN_, int WARPS_M_, int WARPS_N_, int STAGES_, int OCC_>
+struct DmmaTile {
+    static constexpr int BM = BM_, BN = BN_, WARPS_M = WARPS_M_, WARPS_N = WARPS_N_, STAGES = STAGES_;
+    static constexpr int OCC = OCC_;  // CTAs per SM, by shared memory and registers
+    static constexpr int THREADS = 32 * WARPS_M * WARPS_N;
+    static constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N;
     static constexpr int MI = WM / 16, NI = WN / 8;
-    static constexpr size_t SMEM = (size_t)DSTAGES * DK * (DLDA + LDB) * sizeof(double);
+};
+// 64 x 64 with three CTAs per SM is the fastest at every size that fills the GPU: the CTAs'
+// barriers, fills and drains fall at different times, so the pipe always has work. 4096^3:
+// 4.08-4.12 ms (33.7 TFLOP/s), against 4.47-4.72 for one 128 x 128 CTA of 8 warps per SM,
+// 4.10-4.14 for two 128 x 64 of 4 warps, 4.17-4.26 for four 64 x 64 with a two-stage ring
+// and 4.71-4.88 for 32 x 32. Below about one tile per SM the smaller tiles win: 512^3 takes
+// 16.5 us with 32 x 32 and 32.8 us with 64 x 64.
+using TileM = DmmaTile<64, 64, 2, 2, 3, 3>;
+using TileS = DmmaTile<32, 32, 2, 2, 4, 5>;   // small products: latency counts
+using TileT = DmmaTile<64, 16, 4, 1, 4, 4>;   // up to 16 columns
+using TileP = DmmaTile<32, 128, 1, 4, 4, 2>;  // one CTA owns whole rows of a 128-column panel (in place)
+using TileQ = DmmaTile<128, 32, 4, 1, 4, 2>;  // one CTA owns whole columns of a 128-row block (in place)
+
+// Shared-memory tile of an operand with ROWS rows (the m or n direction), in the order of
+// its global layout, so that 16-byte copies keep it: K-major tiles are [row][k] with rows
+// of 20 doubles, the others [k][row] with rows of ROWS + 4 doubles. With either stride the
+// 16 lanes of a half-warp's fragment load (4 rows x 4 k) hit 16 distinct bank pairs.
+template <bool KM, int ROWS>
+struct OpTile {
+    static constexpr int SIZE = KM ? ROWS * DKP : DK * (ROWS + 4);
+    static __device__ __forceinline__ int at(int row, int k) { return KM ? row * DKP + k : k * (ROWS + 4) + row; }
 };
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool pred) {
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int bytes) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    const int bytes = pred ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 __device__ __forceinline__ void dmma_16x8x4(double (&d)[4], double a0, double a1, double b0) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
         : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
         : "d"(a0), "d"(a1), "d"(b0));
 }
 
-// Shared-memory tiles are k-rows of DLDA / LDB doubles; the row offset of element (k, c) is
-// c ^ dswz(k): when the global layout is K-major, consecutive lanes store consecutive k
-// rows, and the XOR spreads their 8-byte stores over all banks (without it the row strides
-// 132 and 68 put four lanes on each bank pair). The fragment loads of one 4-deep k step
-// share one XOR value, which only permutes columns inside groups of four.
-__device__ __forceinline__ int dswz(int k) { return (k >> 2) & 3; }
-
-// A_KMAJOR: A(i, k) is contiguous along k (A.cs == 1), else along i (A.rs == 1).
-// B_KMAJOR: B(k, j) is contiguous along k (B.rs == 1), else along j (B.cs == 1).
-template <bool A_KMAJOR, bool B_KMAJOR, int BN>
-__device__ __forceinline__ void dmma_load_tile(double* sA, double* sB, const View<const double>& A,
-                                               const View<const double>& B, int64_t m, int64_t n, int64_t k,
-                                               int64_t m0, int64_t n0, int64_t k0, int tid) {
-    constexpr int LDB = DmmaCfg<BN>::LDB;
+// Copy k-tile k0 of an operand (element (i, k) at p[i * ld + k] when KM, else p[i + k * ld])
+// into its shared tile; zero outside rows x k. V16: base and ld allow 16-byte copies (rows
+// r0 and k0 are even).
+template <bool KM, int ROWS, int THREADS, bool V16>
+__device__ __forceinline__ void load_operand(double* dst, const double* p, int64_t ld, int64_t rows, int64_t k,
+                                             int64_t r0, int64_t k0, int tid) {
+    constexpr int W = V16 ? 2 : 1;               // doubles per copy
+    constexpr int PER_ROW = (KM ? DK : ROWS) / W;  // copies per contiguous run
+    constexpr int COUNT = ROWS * DK / W;
+    const bool inside = r0 + ROWS <= rows && k0 + DK <= k;
 #pragma unroll
-    for (int r = 0; r < DM * DK / 256; ++r) {
-        int mm, kk;
-        if (A_KMAJOR) { kk = tid % DK; mm = tid / DK + (256 / DK) * r; } else { mm = tid % DM; kk = tid / DM + (256 / DM) * r; }
-        const int64_t gi = m0 + mm, gk = k0 + kk;
-        const bool ok = gi < m && gk < k;
-        cp_async8(sA + kk * DLDA + (mm ^ dswz(kk)), ok ? &A(gi, gk) : A.p, ok);
-    }
-#pragma unroll
-    for (int r = 0; r < BN * DK / 256; ++r) {
-        int nn, kk;
-        if (B_KMAJOR) { kk = tid % DK; nn = tid / DK + (256 / DK) * r; } else { nn = tid % BN; kk = tid / BN + (256 / BN) * r; }
-        const int64_t gj = n0 + nn, gk = k0 + kk;
-        const bool ok = gj < n && gk < k;
-        cp_async8(sB + kk * LDB + (nn ^ dswz(kk)), ok ? &B(gk, gj) : B.p, ok);
+    for (int e0 = 0; e0 < COUNT; e0 += THREADS) {
+        const int e = e0 + tid;
+        if (COUNT % THREADS != 0 && e >= COUNT) break;
+        const int c = (e % PER_ROW) * W, o = e / PER_ROW;  // along the run, across runs
+        const int row = KM ? o : c, kk = KM ? c : o;
+        int bytes = 8 * W;
+        const double* src = KM ? p + (r0 + row) * ld + k0 + kk : p + r0 + row + (k0 + kk) * ld;
+        if (!inside) {
+            const int64_t left = KM ? (r0 + row < rows ? k - (k0 + kk) : 0) : (k0 + kk < k ? rows - (r0 + row) : 0);
+            bytes = left >= W ? 8 * W : left > 0 ? 8 : 0;
+            if (bytes == 0) src = p;
+        }
+        if (V16) cp_async16(dst + OpTile<KM, ROWS>::at(row, kk), src, bytes);
+        else cp_async8(dst + OpTile<KM, ROWS>::at(row, kk), src, bytes);
     }
 }
 
-template <bool A_KMAJOR, bool B_KMAJOR, int BN>
-__global__ void __launch_bounds__(256, 1) gemm_dmma_f64(int64_t m, int64_t n, int64_t k, double alpha,
-                                                         View<const double> A, View<const double> B, double beta,
-                                                         View<double> C, Mask mask, int64_t off,
-                                                         const int* abort, int64_t kchunk, int64_t zstride) {
-    using Cfg = DmmaCfg<BN>;
-    constexpr int LDB = Cfg::LDB, MI = Cfg::MI, NI = Cfg::NI;
+template <bool A_KMAJOR, bool B_KMAJOR, class Tile>
+constexpr size_t dmma_smem() {
+    return (size_t)Tile::STAGES * (OpTile<A_KMAJOR, Tile::BM>::SIZE + OpTile<B_KMAJOR, Tile::BN>::SIZE) * sizeof(double);
+}
+
+// A_KMAJOR: A(i, k) is contiguous along k (A.cs == 1), else along i (A.rs == 1).
+// B_KMAJOR: B(k, j) is contiguous along k (B.rs == 1), else along j (B.cs == 1).
+template <bool A_KMAJOR, bool B_KMAJOR, class Tile, bool V16>
+__global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
+    gemm_dmma_f64(int64_t m, int64_t n, int64_t k, double alpha, View<const double> A, View<const double> B,
+                  double beta, View<double> C, Mask mask, int64_t off, const int* abort, int64_t kchunk,
+                  int64_t zstride) {
+    using TA = OpTile<A_KMAJOR, Tile::BM>;
+    using TB = OpTile<B_KMAJOR, Tile::BN>;
+    constexpr int BM = Tile::BM, BN = Tile::BN, MI = Tile::MI, NI = Tile::NI, ST = Tile::STAGES, T = Tile::THREADS;
     extern __shared__ __align__(16) double dsmem[];
     double* sA = dsmem;
-    double* sB = dsmem + DSTAGES * DK * DLDA;
-    // Grouped tile order: consecutive CTAs take kGroupM row tiles of one column tile before
-    // the next column tile, so that a wave holds a few A row blocks and B column blocks in L2
-    // instead of streaming all of B once per row of tiles.
-    constexpr int64_t kGroupM = 8;
+    double* sB = dsmem + ST * TA::SIZE;
+    // Grouped tile order: consecutive CTAs take a group of row tiles (1024 rows) of one
+    // column tile before the next column tile, so that a wave holds a few A row blocks and
+    // B column blocks in L2 instead of streaming all of B once per row of tiles.
+    constexpr int64_t kGroupM = 1024 / BM;
     const int64_t lin = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, per = kGroupM * gridDim.x;
     const int64_t first = lin / per * kGroupM, rest = (int64_t)gridDim.y - first;
     const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
-    const int64_t m0 = (first + r % gsz) * DM, n0 = r / gsz * BN;
-    if (aborted(abort) || tile_outside(mask, off, m0, n0, DM, BN)) return;
+    const int64_t m0 = (first + r % gsz) * BM, n0 = r / gsz * BN;
+    if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
     if (gridDim.z > 1) {  // K slice of a split-K product
         const int64_t kz = (int64_t)blockIdx.z * kchunk;
         A = A.sub(0, kz);
@@ -187,7 +214,13 @@ __global__ void __launch_bounds__(256, 1) gemm_dmma_f64(int64_t m, int64_t n, in
     }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int wm = (warp / Cfg::WARPS_N) * Cfg::WM, wn = (warp % Cfg::WARPS_N) * Cfg::WN;
+    const int wm = (warp / Tile::WARPS_N) * Tile::WM, wn = (warp % Tile::WARPS_N) * Tile::WN;
+    const int64_t lda = A_KMAJOR ? A.rs : A.cs, ldb = B_KMAJOR ? B.cs : B.rs;
+    auto load = [&](int kt) {
+        const int st = kt % ST;
+        load_operand<A_KMAJOR, BM, T, V16>(sA + st * TA::SIZE, A.p, lda, m, k, m0, (int64_t)kt * DK, tid);
+        load_operand<B_KMAJOR, BN, T, V16>(sB + st * TB::SIZE, B.p, ldb, n, k, n0, (int64_t)kt * DK, tid);
+    };
     double acc[MI][NI][4];
 #pragma unroll
     for (int a = 0; a < MI; ++a)
@@ -198,35 +231,27 @@ __global__ void __launch_bounds__(256, 1) gemm_dmma_f64(int64_t m, int64_t n, in
 
     const int KT = (int)((k + DK - 1) / DK);
 #pragma unroll
-    for (int s = 0; s < DSTAGES - 1; ++s) {
-        if (s < KT)
-            dmma_load_tile<A_KMAJOR, B_KMAJOR, BN>(sA + s * DK * DLDA, sB + s * DK * LDB, A, B, m, n, k, m0, n0,
-                                                   (int64_t)s * DK, tid);
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < KT) load(s);
         cp_async_commit();
     }
     for (int kt = 0; kt < KT; ++kt) {
-        cp_async_wait<DSTAGES - 2>();
+        cp_async_wait<ST - 2>();
         __syncthreads();
-        const int pf = kt + DSTAGES - 1;
-        if (pf < KT) {
-            const int st = pf % DSTAGES;
-            dmma_load_tile<A_KMAJOR, B_KMAJOR, BN>(sA + st * DK * DLDA, sB + st * DK * LDB, A, B, m, n, k, m0, n0,
-                                                   (int64_t)pf * DK, tid);
-        }
+        if (kt + ST - 1 < KT) load(kt + ST - 1);
         cp_async_commit();
-        const double* a_s = sA + (kt % DSTAGES) * DK * DLDA;
-        const double* b_s = sB + (kt % DSTAGES) * DK * LDB;
+        const double* a_s = sA + (kt % ST) * TA::SIZE;
+        const double* b_s = sB + (kt % ST) * TB::SIZE;
 #pragma unroll
         for (int ks = 0; ks < DK; ks += 4) {
             double af[MI][2], bf[NI];
-            const int sx = dswz(ks);  // == dswz(ks + t) for t < 4
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi) {
-                af[mi][0] = a_s[(ks + t) * DLDA + ((wm + mi * 16 + g) ^ sx)];
-                af[mi][1] = a_s[(ks + t) * DLDA + ((wm + mi * 16 + g + 8) ^ sx)];
+                af[mi][0] = a_s[TA::at(wm + mi * 16 + g, ks + t)];
+                af[mi][1] = a_s[TA::at(wm + mi * 16 + g + 8, ks + t)];
             }
 #pragma unroll
-            for (int ni = 0; ni < NI; ++ni) bf[ni] = b_s[(ks + t) * LDB + ((wn + ni * 8 + g) ^ sx)];
+            for (int ni = 0; ni < NI; ++ni) bf[ni] = b_s[TB::at(wn + ni * 8 + g, ks + t)];
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
@@ -234,24 +259,36 @@ __global__ void __launch_bounds__(256, 1) gemm_dmma_f64(int64_t m, int64_t n, in
         }
     }
     cp_async_wait<0>();
-    // Epilogue: element (g, 2t + c) and (g + 8, 2t + c) of each 16x8 accumulator tile.
+    // Epilogue: element (g, 2t + c) and (g + 8, 2t + c) of each 16x8 accumulator tile. The
+    // old C of 16 rows is fetched before any of it is written, so that its loads are all in
+    // flight at once.
 #pragma unroll
-    for (int mi = 0; mi < MI; ++mi)
+    for (int mi = 0; mi < MI; ++mi) {
+        double old[2][NI][2];
+        if (beta != 0.0) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int64_t i = m0 + wm + mi * 16 + g + 8 * h;
-            if (i >= m) continue;
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int64_t i = m0 + wm + mi * 16 + g + 8 * h, j = n0 + wn + ni * 8 + 2 * t + c;
+                        old[h][ni][c] = i < m && j < n && in_mask(mask, off, i, j) ? C(i, j) : 0.0;
+                    }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    const int64_t j = n0 + wn + ni * 8 + 2 * t + c;
-                    if (j >= n || !in_mask(mask, off, i, j)) continue;
+                    const int64_t i = m0 + wm + mi * 16 + g + 8 * h, j = n0 + wn + ni * 8 + 2 * t + c;
+                    if (i >= m || j >= n || !in_mask(mask, off, i, j)) continue;
                     double v = alpha * acc[mi][ni][2 * h + c];
-                    if (beta != 0.0) v = fma(beta, C(i, j), v);
+                    if (beta != 0.0) v = fma(beta, old[h][ni][c], v);
                     C(i, j) = v;
                 }
-        }
+    }
 }
 
 // C = alpha * sum_z P_z + beta * C over the split-K slices (column-major m x n, ld m each).
@@ -267,56 +304,108 @@ __global__ void splitk_reduce(int64_t m, int64_t n, int nz, const double* P, int
         }
 }
 
-template <bool AK, bool BK, int BN>
-int launch_dmma(int64_t m, int64_t n, int64_t k, double alpha, View<const double> A, View<const double> B,
-                double beta, View<double> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
-    const size_t smem = DmmaCfg<BN>::SMEM;
-    if (cudaFuncSetAttribute(gemm_dmma_f64<AK, BK, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+struct Shape {
+    int64_t m, n, k;
+    Mask mask;
+};
+
+// Cycles a product takes with a tile, per the model behind the choice of tiles: an SM works
+// on up to OCC tiles at a time, a k-step of which takes the pipe BM BN / 4 cycles each (it
+// reaches 94% of that with 64 x 64 tiles, 80% with the small ones), but never less than one
+// warp's own chain (its MMAs and ~400 cycles of barrier and fragment loads: 512^3 on 64 x 64
+// tiles, one per SM); a round of tiles pays a fixed fill and drain.
+template <class Tile>
+double tile_cycles(const Shape& s, int nz) {
+    const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
+    if (tm > 65535) return 1e200;  // more row tiles than grid.y holds
+    double tiles = (double)tm * tn;
+    if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));  // of a square, tm (tm + 1) / 2 tiles run
+    const double per_sm = ceil(tiles * nz / sm_count());
+    const double work = Tile::BM * Tile::BN / 4.0 / (Tile::MI * Tile::NI >= 8 ? 0.94 : 0.80);
+    const double chain = Tile::MI * Tile::NI * 4 * 32 + 400.0, ksteps = ceil((double)s.k / nz / DK);
+    const double full = floor(per_sm / Tile::OCC), rest = per_sm - full * Tile::OCC;
+    auto round = [&](double c) { return c <= 0 ? 0.0 : ksteps * (c * work > chain ? c * work : chain) + 3000.0; };
+    return full * round(Tile::OCC) + round(rest);
+}
+
+template <bool AK, bool BK, class Tile, bool V16>
+int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const double> B, double beta,
+                View<double> C, int64_t off, int nz, cudaStream_t s, const int* abort) {
+    constexpr size_t smem = dmma_smem<AK, BK, Tile>();
+    auto kernel = gemm_dmma_f64<AK, BK, Tile, V16>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return RC_ERR_CUDA;
-    dim3 grid(ceil_div(n, BN), ceil_div(m, DM));
-    // Long K: split it into nz slices when that packs the CTAs into the GPU's resident
-    // slots with less wave quantisation -- nz minimises ceil(tiles nz / slots) / nz (the
-    // time in units of one full-K tile) plus a small charge per slice for the reduction.
-    static int per_sm = 0;
-    if (per_sm == 0 &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemm_dmma_f64<AK, BK, BN>, 256, smem) != cudaSuccess)
-        return RC_ERR_CUDA;
-    const int64_t tiles = (int64_t)grid.x * grid.y, slots = (int64_t)(per_sm > 0 ? per_sm : 1) * sm_count();
-    int nz = 1;
-    if (mask == kFull && k >= 2048 && tiles < 4 * slots) {  // few waves: quantisation matters
-        double best = 1e30;
-        for (int z = 1; z <= 8 && (int64_t)z * 1024 <= k; ++z) {
-            const double cost = (double)((tiles * z + slots - 1) / slots) / z + 0.01 * (z - 1);
-            if (cost < best - 1e-9) {
-                best = cost;
-                nz = z;
-            }
-        }
-    }
+    dim3 grid(ceil_div(p.n, Tile::BN), ceil_div(p.m, Tile::BM));
     if (nz > 1) {
-        const int64_t kchunk = ((k + nz - 1) / nz + DK - 1) / DK * DK;
-        nz = (int)((k + kchunk - 1) / kchunk);
-        const int64_t zstride = m * n;
+        const int64_t kchunk = ((p.k + nz - 1) / nz + DK - 1) / DK * DK;
+        nz = (int)((p.k + kchunk - 1) / kchunk);
+        const int64_t zstride = p.m * p.n;
         double* P = static_cast<double*>(workspace(s, (size_t)nz * zstride * sizeof(double), 7));
         if (!P) return RC_ERR_ALLOC;
         grid.z = nz;
-        gemm_dmma_f64<AK, BK, BN><<<grid, 256, smem, s>>>(m, n, k, 1.0, A, B, 0.0, colmajor(P, m), kFull, 0, abort,
-                                                          kchunk, zstride);
+        kernel<<<grid, Tile::THREADS, smem, s>>>(p.m, p.n, p.k, 1.0, A, B, 0.0, colmajor(P, p.m), kFull, 0, abort,
+                                                 kchunk, zstride);
         RC_TRY(check_launch());
-        dim3 rg(ceil_div(m, 256) < 1024u ? ceil_div(m, 256) : 1024u, n < 65535 ? (unsigned)n : 65535u);
-        splitk_reduce<<<rg, 256, 0, s>>>(m, n, nz, P, zstride, alpha, beta, C);
+        dim3 rg(ceil_div(p.m, 256) < 1024u ? ceil_div(p.m, 256) : 1024u, p.n < 65535 ? (unsigned)p.n : 65535u);
+        splitk_reduce<<<rg, 256, 0, s>>>(p.m, p.n, nz, P, zstride, alpha, beta, C);
         return check_launch();
     }
-    gemm_dmma_f64<AK, BK, BN><<<grid, 256, smem, s>>>(m, n, k, alpha, A, B, beta, C, mask, off, abort, k, 0);
+    kernel<<<grid, Tile::THREADS, smem, s>>>(p.m, p.n, p.k, alpha, A, B, beta, C, p.mask, off, abort, p.k, 0);
     return check_launch();
 }
 
+enum TileId { kTileM, kTileS, kTileT, kTileP, kTileQ };
+
+template <bool AK, bool BK, bool V16>
+int launch_tile(TileId id, const Shape& p, double alpha, View<const double> A, View<const double> B, double beta,
+                View<double> C, int64_t off, int nz, cudaStream_t s, const int* abort) {
+    switch (id) {
+    case kTileM: return launch_dmma<AK, BK, TileM, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    case kTileS: return launch_dmma<AK, BK, TileS, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    case kTileT: return launch_dmma<AK, BK, TileT, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    case kTileP: return launch_dmma<AK, BK, TileP, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    default: return launch_dmma<AK, BK, TileQ, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    }
+}
+
+// The tile and K split of least modelled time. A product that writes over one of its own
+// operands (C on A with n <= 128, or on B with m <= 128) takes a tile that spans that
+// operand's rows or columns: each CTA has then read all of what it overwrites.
+void pick_tile(const Shape& p, bool c_on_a, bool c_on_b, bool may_split, TileId* id, int* nz) {
+    double best = 1e300;
+    auto look = [&](TileId t, double cycles, int z) {
+        if (cycles < best) {
+            best = cycles;
+            *id = t;
+            *nz = z;
+        }
+    };
+    if (c_on_a || c_on_b) {
+        *id = c_on_a ? kTileP : kTileQ;
+        *nz = 1;
+        return;
+    }
+    // A split pays a second launch and two passes over its partial products.
+    const int zmax = may_split ? 8 : 1;
+    for (int z = 1; z <= zmax && (z == 1 || (int64_t)z * 512 <= p.k); ++z) {
+        const double extra = z > 1 ? 6000.0 + 16.0 * z * p.m * p.n / 2500.0 : 0.0;
+        look(kTileM, tile_cycles<TileM>(p, z) + extra, z);
+        look(kTileS, tile_cycles<TileS>(p, z) + extra, z);
+        if (p.n <= 16) look(kTileT, tile_cycles<TileT>(p, z) + extra, z);
+    }
+}
+
 template <bool AK, bool BK>
-int launch_dmma_bn(int64_t m, int64_t n, int64_t k, double alpha, View<const double> A, View<const double> B,
-                   double beta, View<double> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
-    if (n <= 64) return launch_dmma<AK, BK, 64>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-    return launch_dmma<AK, BK, 128>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+int gemm_dmma(int64_t m, int64_t n, int64_t k, double alpha, View<const double> A, View<const double> B, double beta,
+              View<double> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
+    const Shape p{m, n, k, mask};
+    TileId id = kTileM;
+    int nz = 1;
+    pick_tile(p, C.p == A.p, C.p == B.p, mask == kFull && k >= 2048, &id, &nz);
+    auto even = [](const double* q, int64_t ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 2 == 0; };
+    if (even(A.p, AK ? A.rs : A.cs) && even(B.p, BK ? B.cs : B.rs))
+        return launch_tile<AK, BK, true>(id, p, alpha, A, B, beta, C, off, nz, s, abort);
+    return launch_tile<AK, BK, false>(id, p, alpha, A, B, beta, C, off, nz, s, abort);
 }
 
 // Scale (beta != 1) the masked part of C when k == 0 or alpha == 0.
@@ -343,10 +432,10 @@ int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T
     if constexpr (std::is_same<T, double>::value) {
         const bool a_k = A.cs == 1, a_m = A.rs == 1, b_k = B.rs == 1, b_n = B.cs == 1;
         if ((a_k || a_m) && (b_k || b_n)) {
-            if (a_k && b_k) return launch_dmma_bn<true, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            if (a_k) return launch_dmma_bn<true, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            if (b_k) return launch_dmma_bn<false, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            return launch_dmma_bn<false, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+            if (a_k && b_k) return gemm_dmma<true, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+            if (a_k) return gemm_dmma<true, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+            if (b_k) return gemm_dmma<false, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+            return gemm_dmma<false, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
         }
     }
     dim3 grid(ceil_div(n, 64), ceil_div(m, 64));
