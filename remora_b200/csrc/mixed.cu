@@ -1283,14 +1283,17 @@ int spd_solve_mixed(int prec, int64_t n, int64_t nrhs, const double* A, int64_t 
                 RC_TRY(M.col_reduce(Rm, ldm, nullptr, 0, 0, normR, M.dev_scalars));
                 RC_TRY(M.col_reduce(X, ldx, nullptr, 0, 0, normX, M.dev_scalars + nrhs));
                 worst = 0.0;
+                all = true;
                 for (int64_t j = 0; j < nrhs; ++j) {
                     const double eta = normR[j] / (normA * normX[j] + normB[j]);
-                    done[j] = !(eta > o.tol);
+                    all = all && !(eta > o.tol);
+                    // Where CG goes on for other columns, one stays in it until it meets the
+                    // recurrence's own bound: a column left within rounding of tol would pass
+                    // or fail the last check by the rounding of its residual alone.
+                    done[j] = !(eta > 0.5 * o.tol);
                     if (std::isfinite(eta)) worst = std::max(worst, eta);
                     else worst = INFINITY;
                 }
-                all = true;
-                for (char d : done) all = all && d;
                 if (!from_split || !(all || iters >= o.max_iter)) break;
             }
             if (iters > 0 && !all) sliced = false;
