@@ -21,321 +21,553 @@ namespace rc {
 namespace {
 
 constexpr int NB = kNB;
-constexpr int SLD = NB + 1;  // shared-memory row stride (doubles)
-constexpr size_t kBlockSmem = (size_t)NB * SLD * sizeof(double);
+constexpr int SLD = NB + 4;  // shared-memory row stride (doubles): DMMA fragment loads hit all banks
+constexpr int DB = 16;       // diagonal sub-block
+constexpr int NSUB = NB / DB;
+constexpr int LTD = 32;      // column stride of the sub-block's transposed copy
+constexpr int kDiagThreads = 512;
+
+// Shared memory of the diagonal-block kernels (doubles): S holds L in its strict lower
+// triangle, the reciprocals of L's diagonal on its diagonal and the strict part of inv(L)
+// transposed in its upper triangle (Inv(i, c), i >= c, at S[c * SLD + i]); ld L's diagonal,
+// rd its reciprocals, Lt the columns of the sub-block being factored, T16 / T32 / T64 the
+// scratch of the inverse's merges.
+constexpr int kOffLt = NB * SLD, kOffLd = kOffLt + NB * LTD / 2, kOffRd = kOffLd + NB, kOffT64 = kOffRd + NB,
+              kOffT32 = kOffT64 + 64 * (64 + 4), kOffT16 = kOffT32 + 32 * (32 + 4), kOffEnd = kOffT16 + 16 * (16 + 4);
+constexpr size_t kDiagSmem = kOffEnd * sizeof(double) + 16;
 
 __device__ __forceinline__ bool aborted(const int* abort) { return abort != nullptr && *(volatile const int*)abort != 0; }
 
-// In-place inversion of the unit/non-unit lower-triangular NB x NB matrix in S
-// (row-major, stride SLD), one thread per column: row i of the inverse only needs row i
-// of L and the rows < i of the inverse in the thread's own column.
-__device__ void invert_lower_inplace(double* S, bool unit) {
-    const int j = threadIdx.x;
-    for (int i = 0; i < NB; ++i) {
-        double x = 0.0;
-        if (j <= i && j < NB) {
-            const double dinv = unit ? 1.0 : 1.0 / S[i * SLD + i];
-            if (j == i) {
-                x = dinv;
-            } else {
-                double a0 = 0.0, a1 = 0.0;
-                int k = j;
-                for (; k + 1 < i; k += 2) {
-                    a0 = fma(S[i * SLD + k], S[k * SLD + j], a0);
-                    a1 = fma(S[i * SLD + k + 1], S[(k + 1) * SLD + j], a1);
-                }
-                if (k < i) a0 = fma(S[i * SLD + k], S[k * SLD + j], a0);
-                x = -(a0 + a1) * dinv;
-            }
+__device__ __forceinline__ void dmma_16x8x4(double (&d)[4], double a0, double a1, double b0) {
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a0), "d"(a1), "d"(b0));
+}
+
+// Tile (rows i0 .. i0 + 15, columns j0 .. j0 + 7) of S -= L(:, m0 : m0 + 16) L(:, m0 : m0 + 16)^T.
+__device__ __forceinline__ void syrk_tile(double* S, int i0, int j0, int m0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    double d[4] = {};
+#pragma unroll
+    for (int k = 0; k < DB; k += 4)
+        dmma_16x8x4(d, S[(i0 + g) * SLD + m0 + k + t], S[(i0 + g + 8) * SLD + m0 + k + t],
+                    S[(j0 + g) * SLD + m0 + k + t]);
+    double2* lo = reinterpret_cast<double2*>(S + (i0 + g) * SLD + j0 + 2 * t);
+    double2* hi = reinterpret_cast<double2*>(S + (i0 + g + 8) * SLD + j0 + 2 * t);
+    double2 a = *lo, b = *hi;
+    a.x -= d[0];
+    a.y -= d[1];
+    b.x -= d[2];
+    b.y -= d[3];
+    *lo = a;
+    *hi = b;
+}
+
+// The update of S by columns m0 .. m0 + 15 on the 16-row tiles from r0, columns from r0 up to
+// `width` 8-column tiles wide or to the diagonal, spread over n workers (number w).
+__device__ __forceinline__ void syrk_tiles(double* S, int r0, int width, int m0, int w, int n, int lane) {
+    int e = w;
+    for (int i0 = r0; i0 < NB; i0 += 16) {
+        const int diag = (i0 - r0) / 8 + 2, cnt = diag < width ? diag : width;
+        for (; e < cnt; e += n) syrk_tile(S, i0, r0 + 8 * e, m0, lane);
+        e -= cnt;
+    }
+}
+
+// One merge of the block inverse: with inv(A) (rows and columns J0 .. J0 + H) and inv(D)
+// (I0 .. I0 + H, I0 = J0 + H) in place, the off-diagonal block of inv([A 0; C D]) is
+// X = -inv(D) (C inv(A)). merge_t computes tile q of T = C inv(A), merge_x tile q of X (16 x 8
+// tiles, down the columns); both skip the zero blocks of the triangular operand and select
+// within its diagonal blocks.
+template <int H>
+__device__ __forceinline__ void merge_t(const double* S, double* T, int J0, int q, int lane) {
+    constexpr int TD = H + 4, ROWS = H / 16;
+    const int ti = 16 * (q % ROWS), tc = 8 * (q / ROWS);
+    const int g = lane >> 2, t = lane & 3, c = tc + g;
+    const double *a = S + (J0 + H + ti + g) * SLD + J0 + t, *v = S + (J0 + c) * SLD + J0 + t;  // v: inv(A)(k, c)
+    double d[4] = {};
+#pragma unroll
+    for (int k = 0; k < 8; k += 4)
+        dmma_16x8x4(d, a[tc + k], a[8 * SLD + tc + k], tc + k + t >= c ? v[tc + k] : 0.0);
+#pragma unroll 4
+    for (int k = tc + 8; k < H; k += 4) dmma_16x8x4(d, a[k], a[8 * SLD + k], v[k]);
+    *reinterpret_cast<double2*>(T + (ti + g) * TD + tc + 2 * t) = make_double2(d[0], d[1]);
+    *reinterpret_cast<double2*>(T + (ti + g + 8) * TD + tc + 2 * t) = make_double2(d[2], d[3]);
+}
+template <int H>
+__device__ __forceinline__ void merge_x(double* S, const double* T, int J0, int xi, int xc, int lane) {
+    constexpr int TD = H + 4;
+    const int I0 = J0 + H, g = lane >> 2, t = lane & 3, i = xi + g;
+    const double *a = S + (I0 + t) * SLD + I0 + i, *b = T + t * TD + xc + g;  // a: inv(D)(i, k)
+    double d[4] = {};
+#pragma unroll 4
+    for (int k = 0; k < xi; k += 4) dmma_16x8x4(d, a[k * SLD], a[k * SLD + 8], b[k * TD]);
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+        const int kk = xi + k;
+        dmma_16x8x4(d, k + t <= g ? a[kk * SLD] : 0.0, k + t <= g + 8 ? a[kk * SLD + 8] : 0.0, b[kk * TD]);
+    }
+    double* x = S + (J0 + xc + 2 * t) * SLD + I0 + i;  // X(i, c), transposed
+    x[0] = -d[0];
+    x[SLD] = -d[1];
+    x[8] = -d[2];
+    x[SLD + 8] = -d[3];
+}
+
+// x solved with the 16-block L, each lane its own x: x[m] /= L(m, m), x[q] -= L(q, m) x[m].
+// Columns of L in Lt, reciprocal diagonal in rd; wait(h) is called before the first use of
+// columns 8 h .. 8 h + 7. With x a unit vector this is a column of inv(L), with x a row of the
+// panel below L that row of the panel solve.
+template <class Wait>
+__device__ __forceinline__ void solve_sub_block(double (&x)[DB], const double* rd, const double* Lt, Wait wait) {
+#pragma unroll
+    for (int m = 0; m < DB; ++m) {
+        if (m % 8 == 0) wait(m / 8);
+        x[m] *= rd[m];
+        const double2* pair = reinterpret_cast<const double2*>(Lt + m * LTD);
+#pragma unroll
+        for (int q = (m + 1) & ~1; q < DB; q += 2) {
+            const double2 v = pair[q / 2];
+            if (q > m) x[q] = fma(-v.x, x[m], x[q]);
+            x[q + 1] = fma(-v.y, x[m], x[q + 1]);
         }
-        __syncthreads();
-        if (j <= i && j < NB) S[i * SLD + j] = x;
-    }
-    __syncthreads();
-}
-
-// Store the inverse (lower, zero above the diagonal) as an NB x NB block, column-major or
-// (row_major) row-major.
-template <class T>
-__device__ void store_block(const double* S, T* W, bool row_major = false) {
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int i = row_major ? e / NB : e % NB, j = row_major ? e % NB : e / NB;
-        W[e] = j <= i ? (T)S[i * SLD + j] : T(0);
     }
 }
 
-// One CTA per diagonal block: W_b = inverse of the lower-triangular block b of L.
+// The 32 x 32 blocks (bi, bj) of the lower triangle, by number 0 .. 9.
+__device__ __forceinline__ void lower_block(int q, int& bi, int& bj) {
+    bi = q < 1 ? 0 : q < 3 ? 1 : q < 6 ? 2 : 3;
+    bj = q - bi * (bi + 1) / 2;
+}
+
+// Half h (16 elements a lane, all loads before the stores) of block q of inv(L) to the NB x NB
+// block W. Row-major W: 8 rows x 4 columns a step (32-byte runs, at most two lanes per bank);
+// column-major: 32 rows of a column.
 template <class T>
-__global__ void __launch_bounds__(NB) trtri_blocks(int64_t m, View<const T> L, bool unit, T* W, int* info,
-                                                   const int* abort) {
-    extern __shared__ double S[];
+__device__ __forceinline__ void store_inverse(const double* S, T* W, bool row_major, int q, int h, int lane) {
+    int bi, bj;
+    lower_block(q, bi, bj);
+    const int i0 = 32 * bi + (row_major ? 16 * h + (lane >> 2) : lane);
+    const int c0 = 32 * bj + (row_major ? lane & 3 : 16 * h);
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+        v[u] = row_major ? S[(c0 + (u & 7) * 4) * SLD + i0 + (u >> 3) * 8] : S[(c0 + u) * SLD + i0];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int i = row_major ? i0 + (u >> 3) * 8 : i0, c = row_major ? c0 + (u & 7) * 4 : c0 + u;
+        if (i >= c) W[row_major ? i * NB + c : i + c * NB] = (T)v[u];
+    }
+}
+
+// Zeros above W's diagonal: part p of NSUB - 1, by 96 threads.
+template <class T>
+__device__ __forceinline__ void zero_upper(T* W, bool row_major, int p, int tid) {
+    constexpr int kPart = (NB * NB + NSUB - 2) / (NSUB - 1);
+    const int end = (p + 1) * kPart < NB * NB ? (p + 1) * kPart : NB * NB;
+#pragma unroll 4
+    for (int e = p * kPart + tid; e < end; e += 96) {
+        const int i = row_major ? e / NB : e % NB, c = row_major ? e % NB : e / NB;
+        if (i < c) W[e] = T(0);
+    }
+}
+
+// Element (i, c) of step u = 0 .. 31 of a lane in a 32 x 32 block of a matrix of either order:
+// 32 columns of a row a step where rows are contiguous, else 8 rows x 4 columns (64-byte runs;
+// the 16 lanes of a half-warp, 4 x 4, fall on distinct banks of S).
+__device__ __forceinline__ int block_row(bool rowmaj, int u, int lane) {
+    return rowmaj ? u : (u & 3) * 8 + (lane & 3) + ((lane >> 4) << 2);
+}
+__device__ __forceinline__ int block_col(bool rowmaj, int u, int lane) {
+    return rowmaj ? lane : (u >> 2) * 4 + ((lane >> 2) & 3);
+}
+
+// Block q of the diagonal block's lower triangle (the identity beyond its sz rows) into S by
+// one warp, 32 loads a lane in flight; unit: ones on the diagonal, which is not read.
+template <class T>
+__device__ __forceinline__ void load_block(const View<T>& A, int sz, bool rowmaj, bool unit, int q, double* S,
+                                           int lane) {
+    int bi, bj;
+    lower_block(q, bi, bj);
+    // (float columns: 32 rows a step, for the longer runs)
+    constexpr bool kRows32 = sizeof(T) == 4;
+    const int i0 = 32 * bi + (kRows32 && !rowmaj ? lane : block_row(rowmaj, 0, lane));
+    const int c0 = 32 * bj + (kRows32 && !rowmaj ? 0 : block_col(rowmaj, 0, lane));
+    auto di = [&](int u) { return rowmaj ? u : kRows32 ? 0 : (u & 3) * 8; };
+    auto dc = [&](int u) { return rowmaj ? 0 : kRows32 ? u : (u >> 2) * 4; };
+    const T* src = &A(i0, c0);
+    double v[32];
+#pragma unroll
+    for (int u = 0; u < 32; ++u) {
+        const int i = i0 + di(u), c = c0 + dc(u);
+        v[u] = i == c ? 1.0 : 0.0;
+        if (i < sz && (c < i || (c == i && !unit))) v[u] = (double)src[di(u) * A.rs + dc(u) * A.cs];
+    }
+#pragma unroll
+    for (int u = 0; u < 32; ++u) {
+        const int i = i0 + di(u), c = c0 + dc(u);
+        if (c <= i) S[i * SLD + c] = v[u];
+    }
+}
+
+// Half h of L's block q from S and ld back to A by one warp.
+template <class T>
+__device__ __forceinline__ void store_block(const View<T>& A, int sz, bool rowmaj, int q, int h, const double* S,
+                                            const double* ld, int lane) {
+    int bi, bj;
+    lower_block(q, bi, bj);
+    const int i0 = 32 * bi + block_row(rowmaj, 16 * h, lane), c0 = 32 * bj + block_col(rowmaj, 16 * h, lane);
+    T* dst = &A(i0, c0);
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int i = rowmaj ? i0 + u : i0 + (u & 3) * 8, c = rowmaj ? c0 : c0 + (u >> 2) * 4;
+        v[u] = *(i == c ? ld + i : S + i * SLD + c);
+    }
+    const int64_t r8 = 8 * A.rs, c4 = 4 * A.cs;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int i = rowmaj ? i0 + u : i0 + (u & 3) * 8, c = rowmaj ? c0 : c0 + (u >> 2) * 4;
+        if (i < sz && c <= i) dst[rowmaj ? u * A.rs : (u >> 2) * c4 + (u & 3) * r8] = (T)v[u];
+    }
+}
+
+// 1 / sqrt(d) for a normal d > 0: the hardware approximation (relative error e below 2^-20)
+// and one step of the third-order series of (1 - e)^(-1/2). Straight-line code, so that the
+// rank-1 update of the column before is scheduled into its latency; for a subnormal d the
+// approximation is infinite and the caller starts over with rsqrt().
+__device__ __forceinline__ double rsqrt_normal(double d) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-(d * r), r, 1.0);
+    return fma(r * e, fma(e, fma(e, 0.3125, 0.375), 0.5), r);
+}
+
+// Named barriers of potrf_diag: kBarChunk + h says that columns 8 h .. 8 h + 7 of the
+// sub-block being factored are in Lt and rd (warp 0 arrives, their readers wait).
+constexpr int kBarBackground = 1, kBarChunk = 2;
+__device__ __forceinline__ void named_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Right-looking factorisation of 16 columns of 32 rows by one warp, row `lane` in a (the
+// 16 x 16 block to factor and the 16 rows below it): a becomes L's row, column j of L goes to
+// Lt + j * LTD, L(j, j) to ld and its reciprocal to rd; every 8 columns it arrives at the chunk
+// barriers (`threads` participants). flags[0] = 1 + column of the first non-positive (or NaN)
+// pivot, 0 if there is none; after one the values are void. flags[1] = 1 where a pivot is too
+// small for rsqrt_normal, and the result is void.
+__device__ __forceinline__ void factor_sub_block(double (&a)[DB], double* Lt, double* ld, double* rd, int lane,
+                                                 int threads, volatile int* flags) {
+    int bad = 0;
+    bool tiny = false;
+    auto pivot = [&](double own, int j) {
+        const double d = __shfl_sync(0xffffffffu, own, j);
+        if (!(d > 0.0) && bad == 0) bad = j + 1;
+        tiny |= d < 1e-300;
+        return d;
+    };
+    double d = pivot(a[0], 0), r = rsqrt_normal(d);
+#pragma unroll
+    for (int j = 0; j < DB; ++j) {
+        const double l = lane == j ? d * r : a[j] * r;  // L(i, j); above the diagonal, unused
+        a[j] = l;
+        if (lane == j) {
+            rd[j] = r;
+            ld[j] = l;
+        }
+        double* colj = Lt + j * LTD;
+        colj[lane] = l;
+        if (j + 1 < DB) {
+            d = pivot(fma(-l, l, a[j + 1]), j + 1);  // row j + 1's own update of its diagonal
+            r = rsqrt_normal(d);
+        } else if (lane == 0) {
+            flags[0] = bad;
+            flags[1] = tiny && bad == 0;
+        }
+        __syncwarp();
+        if (j % 8 == 7) named_arrive(kBarChunk + j / 8, threads);
+        const double2* pair = reinterpret_cast<const double2*>(colj);
+#pragma unroll
+        for (int c = (j + 1) & ~1; c < DB; c += 2) {
+            const double2 v = pair[c / 2];
+            if (c > j) a[c] = fma(-l, v.x, a[c]);
+            a[c + 1] = fma(-l, v.y, a[c + 1]);
+        }
+    }
+}
+
+// The same for pivots of any size, on the rows in shared memory (row: this lane's) and with the
+// library's rsqrt: the way out for values next to underflow.
+__device__ __noinline__ void factor_sub_block_any(double* row, bool own, double* Lt, double* ld, double* rd, int lane,
+                                                  int threads, volatile int* flags) {
+    int bad = 0;
+#pragma unroll 1
+    for (int j = 0; j < DB; ++j) {
+        double d = __shfl_sync(0xffffffffu, own ? row[j] : 0.0, j);
+        if (!(d > 0.0)) {
+            if (bad == 0) bad = j + 1;
+            d = 1.0;
+        }
+        const double r = rsqrt(d), l = lane == j ? d * r : own ? row[j] * r : 0.0;
+        if (lane == j) {
+            rd[j] = r;
+            ld[j] = l;
+        }
+        if (own && lane > j) row[j] = l;
+        Lt[j * LTD + lane] = l;
+        if (j + 1 == DB && lane == 0) {
+            flags[0] = bad;
+            flags[1] = 0;
+        }
+        __syncwarp();
+        if (j % 8 == 7) named_arrive(kBarChunk + j / 8, threads);
+        if (own)
+            for (int c = j + 1; c < DB && c <= lane; ++c) row[c] = fma(-l, Lt[j * LTD + c], row[c]);
+    }
+}
+
+// One CTA per diagonal block: W_b = inverse of the lower-triangular block b of L. The 16-blocks
+// are inverted by a warp each and merged pairwise on DMMA (16-, 32-, then 64-blocks).
+// 64 blocks of an 8192-row FP64 triangle: 15 us (227 us with one thread per column and a
+// barrier per row).
+template <class T>
+__global__ void __launch_bounds__(kDiagThreads, 1) trtri_blocks(int64_t m, View<const T> L, bool unit, T* W, int* info,
+                                                                const int* abort) {
+    extern __shared__ __align__(16) double S[];
+    double *rd = S + kOffRd, *T64 = S + kOffT64, *T32 = S + kOffT32, *T16 = S + kOffT16;
     if (aborted(abort)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t r0 = (int64_t)blockIdx.x * NB;
     const int sz = (int)(m - r0 < NB ? m - r0 : NB);
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int i = e % NB, j = e / NB;
-        double v;
-        if (i < sz && j < sz && j <= i) v = (i == j && unit) ? 1.0 : (double)L(r0 + i, r0 + j);
-        else v = (i == j) ? 1.0 : 0.0;
-        S[i * SLD + j] = v;
+    T* Wb = W + (size_t)blockIdx.x * NB * NB;
+    const View<const T> A = L.sub(r0, r0);
+    if (warp < 10) load_block(A, sz, A.cs == 1, unit, warp, S, lane);
+    else if (warp < 13)
+        for (int p = 0; p < NSUB - 1; ++p) zero_upper(Wb, false, p, tid - 320);
+    __syncthreads();
+    if (tid < NB) {
+        const double d = S[tid * SLD + tid];
+        if (!unit && info != nullptr && tid < sz && d == 0.0) record_first(info, (int)(r0 + tid + 1));
+        rd[tid] = S[tid * SLD + tid] = 1.0 / d;
     }
     __syncthreads();
-    if (!unit && info != nullptr && threadIdx.x < sz && S[threadIdx.x * SLD + threadIdx.x] == 0.0)
-        record_first(info, (int)(r0 + threadIdx.x + 1));
-    invert_lower_inplace(S, unit);
-    store_block<T>(S, W + (size_t)blockIdx.x * NB * NB);
-}
-
-// In-CTA blocked factorisation of one NB x NB diagonal block (FP64 in shared memory S,
-// row-major, odd stride SLD so that both row and column walks are bank-conflict free).
-// Besides L (lower triangle of S) it keeps rd[i] = 1 / L(i, i) and builds inv(L) in the
-// strict upper triangle: Inv(i, c), i > c, is stored at S[c * SLD + i].
-constexpr int DB = 32;  // diagonal sub-block
-constexpr size_t kDiagSmem = kBlockSmem + (NB + 64 * 65) * sizeof(double) + 16;  // S, rd, T, flag
-
-// S[i][c] -= sum_{m in [C0, C0 + DB)} L(i, m) L(c, m) for C0 + DB <= c <= i < NB. Thread
-// (ty, tx) of 16 x 16 owns rows ty + 16 r and columns tx + 16 q with r, q >= (C0 + DB) / 16.
-template <int KB>
-__device__ void trailing_update(double* S) {
-    constexpr int C0 = DB * KB, R0 = (C0 + DB) / 16, G = NB / 16 - R0;
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    double acc[G][G];
+    if (warp < NSUB) {
+        const int c0 = DB * warp;
+        double* Lt = S + kOffLt + warp * DB * 16;  // columns of the sub-block, stride 16
+        if (lane < DB) {
 #pragma unroll
-    for (int r = 0; r < G; ++r)
+            for (int p = 0; p < DB; ++p) Lt[p * DB + lane] = S[(c0 + lane) * SLD + c0 + p];
+        }
+        __syncwarp();
+        double x[DB];
 #pragma unroll
-        for (int q = 0; q < G; ++q) acc[r][q] = 0.0;
-#pragma unroll 4
-    for (int m = C0; m < C0 + DB; ++m) {
-        double lr[G], lc[G];
+        for (int q = 0; q < DB; ++q) x[q] = q == lane ? 1.0 : 0.0;
 #pragma unroll
-        for (int r = 0; r < G; ++r) lr[r] = S[(ty + 16 * (R0 + r)) * SLD + m];
+        for (int p = 0; p < DB; ++p) {
+            x[p] *= rd[c0 + p];
 #pragma unroll
-        for (int q = 0; q < G; ++q) lc[q] = S[(tx + 16 * (R0 + q)) * SLD + m];
+            for (int q = p + 1; q < DB; ++q) x[q] = fma(-Lt[p * DB + q], x[p], x[q]);
+        }
 #pragma unroll
-        for (int r = 0; r < G; ++r)
-#pragma unroll
-            for (int q = 0; q <= r; ++q) acc[r][q] = fma(lr[r], lc[q], acc[r][q]);
+        for (int q = 0; q < DB; ++q)
+            if (q > lane) S[(c0 + lane) * SLD + c0 + q] = x[q];
     }
-#pragma unroll
-    for (int r = 0; r < G; ++r)
-#pragma unroll
-        for (int q = 0; q <= r; ++q) {
-            const int i = ty + 16 * (R0 + r), c = tx + 16 * (R0 + q);
-            if (c <= i) S[i * SLD + c] -= acc[r][q];
-        }
-}
-
-// One step of the recursive inverse, for blocks of H rows: with inv(A) (rows/columns
-// [J0, J0 + H)) and inv(D) ([I0, I0 + H), I0 = J0 + H) in place, the off-diagonal block of
-// inv([A 0; C D]) is X = -inv(D) (C inv(A)). Needs rd on the diagonal of S, so that
-// Inv(i, c) = S[c * SLD + i] for i >= c. NT threads (index t); thread (ty, tx) of
-// (NT / 16) x 16 computes rows ty + (NT / 16) r and columns tx + 16 q of the H x H
-// products; T is an H x H scratch (pitch 65). Phase 0: T = C inv(A); phase 1: X.
-template <int H, int NT>
-__device__ void inverse_merge(double* S, double* T, int J0, int t, int phase) {
-    constexpr int RY = NT / 16, NR = H / RY, NQ = H / 16;
-    const int I0 = J0 + H, ty = t / 16, tx = t % 16;
-    double acc[NR][NQ];
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[r][q] = 0.0;
-    // The triangular operand is walked in k-blocks matching this thread's row or column
-    // blocks: blocks that are entirely zero are skipped, full blocks need no mask, and only
-    // the diagonal block selects.
-    if (phase == 0) {  // T(i, c) = sum_{k >= c} C(i, k) inv(A)(k, c); columns c = tx + 16 q
-#pragma unroll
-        for (int kb = 0; kb < NQ; ++kb) {
-#pragma unroll 4
-            for (int kk = 0; kk < 16; ++kk) {
-                const int k = 16 * kb + kk;
-                double lr[NR];
-#pragma unroll
-                for (int r = 0; r < NR; ++r) lr[r] = S[(I0 + ty + RY * r) * SLD + J0 + k];
-#pragma unroll
-                for (int q = 0; q <= kb; ++q) {
-                    double v = S[(J0 + tx + 16 * q) * SLD + J0 + k];  // inv(A)(k, c)
-                    if (q == kb) v = kk >= tx ? v : 0.0;
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) acc[r][q] = fma(lr[r], v, acc[r][q]);
-                }
-            }
-        }
-    } else {           // X(i, c) = -sum_{k <= i} inv(D)(i, k) T(k, c); rows i = ty + RY r
-#pragma unroll
-        for (int kb = 0; kb < NR; ++kb) {
-#pragma unroll 4
-            for (int kk = 0; kk < RY; ++kk) {
-                const int k = RY * kb + kk;
-                double lc[NQ];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) lc[q] = T[k * 65 + tx + 16 * q];
-#pragma unroll
-                for (int r = kb; r < NR; ++r) {
-                    double v = S[(I0 + k) * SLD + I0 + ty + RY * r];  // inv(D)(i, k)
-                    if (r == kb) v = kk <= ty ? v : 0.0;
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) acc[r][q] = fma(v, lc[q], acc[r][q]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int i = ty + RY * r, c = tx + 16 * q;
-            if (phase == 0) T[i * 65 + c] = acc[r][q];
-            else S[(J0 + c) * SLD + I0 + i] = -acc[r][q];  // X(i, c) stored transposed
-        }
+    __syncthreads();
+    // four 16-merges (scratch: T16 and, for the others, T64), two 32-merges, the 64-merge
+    double* Tq = warp < 2 ? T16 : T64 + (warp >> 1) * 16 * 20;
+    if (warp < 8) merge_t<16>(S, Tq, 32 * (warp >> 1), warp & 1, lane);
+    __syncthreads();
+    if (warp < 8) merge_x<16>(S, Tq, 32 * (warp >> 1), 0, 8 * (warp & 1), lane);
+    __syncthreads();
+    Tq = warp < 8 ? T32 : T64;
+    merge_t<32>(S, Tq, 64 * (warp >> 3), warp & 7, lane);
+    __syncthreads();
+    merge_x<32>(S, Tq, 64 * (warp >> 3), 16 * (warp & 1), 8 * ((warp & 7) >> 1), lane);
+    __syncthreads();
+    for (int q = warp; q < 32; q += 16) merge_t<64>(S, T64, 0, q, lane);
+    __syncthreads();
+    for (int q = warp; q < 32; q += 16) merge_x<64>(S, T64, 0, 16 * (q & 3), 8 * (q >> 2), lane);
+    __syncthreads();
+    for (int q = warp; q < 20; q += 16) store_inverse(S, Wb, false, q >> 1, q & 1, lane);
 }
 
 // Factor the sz x sz lower diagonal block (A already offset to it) in FP64 and store
 // inv(L) into W (column-major, or row-major when w_row_major); g0 = global index of the
-// block for the pivot status. Blocked in shared memory over 32-column sub-blocks k:
-//   1. warp 0 factors the 32 x 32 diagonal sub-block right-looking with each lane's row
-//      in registers (a column step: a shuffle of the pivot, one reciprocal square root,
-//      the column broadcast through shared memory and independent FMAs, no CTA barrier);
-//   2. warp 0 inverts that sub-block (each lane a column, in registers) while warps 1-3
-//      solve the rows below it (each thread a row, in registers), both right-looking
-//      substitutions reading L through shared-memory broadcasts;
-//   3. all threads apply the rank-32 update to the trailing triangle (register tiles).
-// inv(L) is then merged from the 32-block inverses: two 64-blocks at once, then the
-// 128-block (X = -inv(D) C inv(A) at each merge).
+// block for the pivot status. One CTA; the critical path is warp 0's, over the 16-column
+// sub-blocks kb:
+//   A. warp 0 factors the 16 x 16 diagonal sub-block and solves the 16 rows below it,
+//      right-looking with each lane's row in registers. A column's chain is the shuffle of its
+//      pivot, the reciprocal square root, the scaling and the next pivot's own update; the
+//      column reaches the other lanes through shared memory and its rank-1 update runs in the
+//      shadow of that chain. Eight columns behind, warps 1-3 solve the other rows below (each
+//      thread a row, in registers) and warp 5 inverts the sub-block (each lane a column).
+//   C. all warps apply the panel's rank-16 update to the next 16 columns (DMMA).
+// The rest runs on the other warps in the shadow of A: the first loads, the trailing update
+// beyond the next panel, the merges of the block inverse (X = -inv(D) C inv(A) for 16-, 32-,
+// 64-blocks), so that after the last sub-block only the part of the inverse that depends on
+// it is left.
+// No DMMA work runs on the scheduler of warp 0 (warps 4, 8, 12) during A, and each role has a
+// loop of its own, so that warp 0's stays in the instruction cache of its scheduler (the same
+// schedule with the roles inside one loop ran the chain at half the speed, and on 32-column
+// sub-blocks, whose unrolled steps are four times the code, 40% of all stalls were waits for
+// instructions). Bound by latency: 128 dependent columns at ~180 cycles, ~1400 cycles a
+// sub-block for C and its barriers, 5000 for the first loads and 7000 for the last merges and
+// stores. In a factorisation of n = 1024: 26.5 us a block (46.7 with the merges and updates in
+// register tiles on the critical path); beside the mixed solve's trailing update 43.5 (61.8).
 template <class T>
-__global__ void __launch_bounds__(256, 1) potrf_diag(View<T> A, int sz, int64_t g0, T* W, int* info,
-                                                     bool w_row_major) {
-    extern __shared__ double S[];
-    double* rd = S + NB * SLD;
-    double* Tm = rd + NB;
-    int* fail = reinterpret_cast<int*>(Tm + 64 * 65);
-    if (aborted(info)) return;
+__global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz, int64_t g0, T* W, int* info,
+                                                              bool w_row_major) {
+    extern __shared__ __align__(16) double S[];
+    double *Lt = S + kOffLt, *ld = S + kOffLd, *rd = S + kOffRd;
+    double *T64 = S + kOffT64, *T32 = S + kOffT32, *T16 = S + kOffT16;
+    volatile int* flags = reinterpret_cast<int*>(S + kOffEnd);  // [0]: failing column, [1]: start over
+    const bool skip = aborted(info);  // looked at once the block's loads are under way
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool rowmaj = A.cs == 1;
-    // The block into shared memory, 16 loads per thread in flight at a time (the block was
-    // just written by the previous update and comes from L2: one round trip per batch).
-    constexpr int kPer = NB * NB / 256, kBatch = 16;
-    static_assert(kPer % kBatch == 0, "load batches");
+    auto sync_all = [] { named_sync(0, kDiagThreads); };
+    // The end of A for everybody: whether warp 0 has to start over (then once every thread has
+    // read the flag).
+    auto redo = [&] {
+        sync_all();
+        const bool r = flags[1] != 0;
+        if (r) sync_all();
+        return r;
+    };
+    // C by warps 1 .. 15: the next panel's update.
+    auto next_panel = [&](int c0) {
+        if (c0 + DB < NB) syrk_tiles(S, c0 + DB, 2, c0, warp - 1, kDiagThreads / 32 - 1, lane);
+        sync_all();
+    };
+    // Warps 1 .. 3 with rows at sub-block kb, beyond the 32 of warp 0; participants of its
+    // chunk barriers.
+    auto solvers = [](int kb) { return kb < 6 ? (NB - DB * kb - 1) / 32 : 0; };
+    auto participants = [&](int kb) { return 32 * (2 + solvers(kb)); };
+    if (warp < 10) load_block(A, sz, rowmaj, false, warp, S, lane);
+    if (skip) return;
+    sync_all();
+    if (warp == 0) {
 #pragma unroll 1
-    for (int b0 = 0; b0 < kPer; b0 += kBatch) {
-        double v[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            const int e = tid + 256 * (b0 + u);
-            const int i = rowmaj ? e / NB : e % NB, c = rowmaj ? e % NB : e / NB;
-            v[u] = (i < sz && c < sz && c <= i) ? (double)A(i, c) : (i == c ? 1.0 : 0.0);
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            const int e = tid + 256 * (b0 + u);
-            const int i = rowmaj ? e / NB : e % NB, c = rowmaj ? e % NB : e / NB;
-            S[i * SLD + c] = v[u];
-        }
-    }
-    if (tid == 0) *fail = 0;
-    __syncthreads();
-#pragma unroll 1
-    for (int kb = 0; kb < NB / DB; ++kb) {
-        const int c0 = DB * kb;
-        if (warp == 0) {  // 1. right-looking factor of the diagonal sub-block, row `lane` in registers
-            const int i = c0 + lane;
-            double a[DB];
-#pragma unroll
-            for (int c = 0; c < DB; ++c) a[c] = c <= lane ? S[i * SLD + c0 + c] : 0.0;
-            int bad = -1;  // first non-positive pivot (uniform across the warp); later steps run on 1
-            double* colj = Tm;  // column j of L, broadcast through shared memory
-#pragma unroll
-            for (int j = 0; j < DB; ++j) {
-                double d = __shfl_sync(0xffffffffu, a[j], j);
-                if (!(d > 0.0)) {  // also catches NaN
-                    if (bad < 0) bad = j;
-                    d = 1.0;
-                }
-                const double r = rsqrt(d);
-                const double l = lane == j ? d * r : a[j] * r;  // L(i, j); zero above the diagonal
-                a[j] = l;
-                if (lane == j) rd[c0 + j] = r;
-                colj[lane] = l;
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < DB; ++c) {
-                    if (c <= j) continue;
-                    // a(i, c) -= L(i, j) L(c, j); lanes above the diagonal only touch their
-                    // upper-triangle entries, which are neither read nor written back
-                    a[c] = fma(-l, colj[c], a[c]);
-                }
-                __syncwarp();
-            }
-            if (bad >= 0) {
-                if (lane == 0) {
-                    record_first(info, (int)(g0 + c0 + bad + 1));
-                    *fail = 1;
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < DB; ++c)
-                    if (c <= lane) S[i * SLD + c0 + c] = a[c];
-            }
-        }
-        __syncthreads();
-        if (*fail) return;
-        if (warp == 0) {  // 2a. inverse of the sub-block, column `lane` in registers
+        for (int kb = 0; kb < NSUB; ++kb) {
+            const int c0 = DB * kb;
+            double* row = S + (c0 + lane) * SLD + c0;
             double x[DB];
 #pragma unroll
-            for (int q = 0; q < DB; ++q) x[q] = q == lane ? 1.0 : 0.0;
-#pragma unroll
-            for (int m = 0; m < DB; ++m) {
-                x[m] *= rd[c0 + m];
-#pragma unroll
-                for (int q = m + 1; q < DB; ++q) x[q] = fma(-S[(c0 + q) * SLD + c0 + m], x[m], x[q]);
+            for (int c = 0; c < DB; c += 2) {
+                const double2 v = reinterpret_cast<const double2*>(row)[c / 2];
+                x[c] = v.x;
+                x[c + 1] = v.y;
             }
+            factor_sub_block(x, Lt, ld + c0, rd + c0, lane, participants(kb), flags);
+            __syncwarp();
+            if (!flags[1] && c0 + lane < NB) {
 #pragma unroll
-            for (int q = 0; q < DB; ++q)
-                if (q > lane) S[(c0 + lane) * SLD + c0 + q] = x[q];
-        } else if (tid - 32 < NB - c0 - DB) {  // 2b. one row below the sub-block per thread
-            const int i = c0 + DB + (tid - 32);
-            double r[DB];
-#pragma unroll
-            for (int c = 0; c < DB; ++c) r[c] = S[i * SLD + c0 + c];
-#pragma unroll
-            for (int j = 0; j < DB; ++j) {
-                r[j] *= rd[c0 + j];
-#pragma unroll
-                for (int c = j + 1; c < DB; ++c) r[c] = fma(-r[j], S[(c0 + c) * SLD + c0 + j], r[c]);
+                for (int q = 0; q < DB; ++q)
+                    if (q < lane) row[q] = x[q];
             }
-#pragma unroll
-            for (int c = 0; c < DB; ++c) S[i * SLD + c0 + c] = r[c];
+            if (redo()) {
+                factor_sub_block_any(row, c0 + lane < NB, Lt, ld + c0, rd + c0, lane, participants(kb), flags);
+                redo();
+            }
+            if (flags[0]) {
+                if (lane == 0) record_first(info, (int)(g0 + c0 + flags[0]));
+                return;
+            }
+            sync_all();
         }
-        __syncthreads();
-        if (kb == 0) trailing_update<0>(S);  // 3.
-        else if (kb == 1) trailing_update<1>(S);
-        else if (kb == 2) trailing_update<2>(S);
-        __syncthreads();
+    } else if (warp <= 3 || warp == 5) {
+#pragma unroll 1
+        for (int kb = 0; kb < NSUB; ++kb) {
+            const int c0 = DB * kb, row = c0 + 32 * warp + lane;
+            do {
+                if (warp != 5 && warp > solvers(kb)) continue;
+                double x[DB];
+                double2* src = reinterpret_cast<double2*>(S + row * SLD + c0);
+                if (warp == 5) {
+#pragma unroll
+                    for (int q = 0; q < DB; ++q) x[q] = q == lane ? 1.0 : 0.0;
+                } else if (row < NB) {
+#pragma unroll
+                    for (int c = 0; c < DB; c += 2) {
+                        const double2 v = src[c / 2];
+                        x[c] = v.x;
+                        x[c + 1] = v.y;
+                    }
+                }
+                const int threads = participants(kb);
+                solve_sub_block(x, rd + c0, Lt, [&](int h) { named_sync(kBarChunk + h, threads); });
+                if (flags[1]) continue;
+                if (warp == 5) {
+                    double* dst = S + (c0 + lane) * SLD + c0;
+#pragma unroll
+                    for (int q = 0; q < DB; ++q)
+                        if (q >= lane) dst[q] = x[q];
+                } else if (row < NB) {
+#pragma unroll
+                    for (int c = 0; c < DB; c += 2) src[c / 2] = make_double2(x[c], x[c + 1]);
+                }
+            } while (redo());
+            if (flags[0]) return;
+            next_panel(c0);
+        }
+    } else if (warp % 4 != 0) {  // the eight background warps 6, 7, 9, 10, 11, 13, 14, 15
+        constexpr int nbg = 8;
+        const int bg = warp - 5 - warp / 4;
+#pragma unroll 1
+        for (int kb = 0; kb < NSUB; ++kb) {
+            const int c0 = DB * kb;
+            // panel kb - 1's update right of this panel: rows and columns from c0 + 16
+            if (kb > 0) syrk_tiles(S, c0 + DB, NB, c0 - DB, bg, nbg, lane);
+            if (kb == 2 || kb == 4 || kb == 6) {  // the 32-block before this sub-block
+                if (bg < 2) merge_t<16>(S, T16, c0 - 32, bg, lane);
+                named_sync(kBarBackground, 32 * nbg);
+                if (bg < 2) merge_x<16>(S, T16, c0 - 32, 0, 8 * bg, lane);
+                if (kb == 4) {
+                    named_sync(kBarBackground, 32 * nbg);
+                    merge_x<32>(S, T32, 0, 16 * (bg & 1), 8 * (bg >> 1), lane);
+                }
+            } else if (kb == 3 || kb == 7) {
+                merge_t<32>(S, T32, kb == 3 ? 0 : 64, bg, lane);
+                if (kb == 7) {
+                    if (bg < 2) merge_t<16>(S, T16, 96, bg, lane);
+                    // rows 64 .. 95 of the 64-merge need no part of the last 32 rows
+                    for (int q = bg; q < 16; q += nbg) merge_x<64>(S, T64, 0, 16 * (q & 1), 8 * (q >> 1), lane);
+                }
+            }
+            if (kb == 5 || kb == 6)  // T of the 64-merge, half of its columns each
+                for (int q = bg; q < 16; q += nbg) merge_t<64>(S, T64, 0, 16 * (kb - 5) + q, lane);
+            while (redo()) {}
+            if (flags[0]) return;
+            next_panel(c0);
+        }
+    } else {  // warps 4, 8, 12
+#pragma unroll 1
+        for (int kb = 0; kb < NSUB; ++kb) {
+            if (kb < NSUB - 1) zero_upper(W, w_row_major, kb, 32 * (warp / 4 - 1) + lane);
+            if (kb == NSUB - 1)  // the inverse's final blocks (0, 0), (1, 0), (1, 1), (2, 2)
+                for (int q = warp / 4 - 1; q < 8; q += 3) store_inverse(S, W, w_row_major, q < 6 ? q >> 1 : 5, q & 1, lane);
+            while (redo()) {}
+            if (flags[0]) return;
+            next_panel(DB * kb);
+        }
     }
-    // L back to global memory (lower part).
-    for (int e = tid; e < NB * NB; e += 256) {
-        const int i = rowmaj ? e / NB : e % NB, c = rowmaj ? e % NB : e / NB;
-        if (i < sz && c <= i) A(i, c) = (T)S[i * SLD + c];
+    // What depends on the last sub-blocks: the last 16-, the last 32-merge and the lower half
+    // of the 64-merge (warps 0-7); meanwhile L goes back to global memory.
+    if (warp < 8) {
+        if (warp < 2) merge_x<16>(S, T16, 96, 0, 8 * warp, lane);
+        named_sync(kBarBackground, 256);
+        merge_x<32>(S, T32, 64, 16 * (warp & 1), 8 * (warp >> 1), lane);
+        named_sync(kBarBackground, 256);
+        merge_x<64>(S, T64, 0, 32, 8 * warp, lane);
+        merge_x<64>(S, T64, 0, 48, 8 * warp, lane);
+    } else {
+        for (int q = warp - 8; q < 20; q += 8) store_block(A, sz, rowmaj, q >> 1, q & 1, S, ld, lane);
     }
     __syncthreads();
-    // inv(L): the inverse's diagonal replaces L's, then 32-blocks -> 64-blocks (two merges,
-    // 128 threads each) -> the 128-block.
-    if (tid < NB) S[tid * SLD + tid] = rd[tid];
-    __syncthreads();
-    double* Th = Tm + (tid >= 128 ? 32 * 65 : 0);
-    inverse_merge<32, 128>(S, Th, tid >= 128 ? 64 : 0, tid & 127, 0);
-    __syncthreads();
-    inverse_merge<32, 128>(S, Th, tid >= 128 ? 64 : 0, tid & 127, 1);
-    __syncthreads();
-    inverse_merge<64, 256>(S, Tm, 0, tid, 0);
-    __syncthreads();
-    inverse_merge<64, 256>(S, Tm, 0, tid, 1);
-    __syncthreads();
-    for (int e = tid; e < NB * NB; e += 256) {
-        const int i = w_row_major ? e / NB : e % NB, c = w_row_major ? e % NB : e / NB;
-        const double v = S[c * SLD + i];
-        W[e] = (T)(i >= c ? v : 0.0);
-    }
+    if (warp < 12)  // the blocks of the inverse that are not stored yet
+        store_inverse(S, W, w_row_major, warp < 4 ? 3 + (warp >> 1) : 6 + ((warp - 4) >> 1), warp & 1, lane);
 }
 
 template <class K>
@@ -356,8 +588,8 @@ int trsm_left(bool upper, bool unit, int64_t m, int64_t n, T alpha, View<const T
     T* tmp = static_cast<T*>(workspace(s, (size_t)NB * n * sizeof(T), 2));
     if (!W || !tmp) return RC_ERR_ALLOC;
     const View<const T> L = upper ? A.t() : A;
-    RC_TRY(set_smem(trtri_blocks<T>, kBlockSmem));
-    trtri_blocks<T><<<(unsigned)nblk, NB, kBlockSmem, s>>>(m, L, unit, W, info, abort);
+    RC_TRY(set_smem(trtri_blocks<T>, kDiagSmem));
+    trtri_blocks<T><<<(unsigned)nblk, kDiagThreads, kDiagSmem, s>>>(m, L, unit, W, info, abort);
     RC_TRY(check_launch());
     if (alpha != T(1)) RC_TRY(copy2d<T, T>(m, n, alpha, View<const T>{B.p, B.rs, B.cs}, B, s, abort));
     const View<T> Tv = colmajor(tmp, (int64_t)NB);
@@ -405,7 +637,7 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s) {
         const int64_t w = (n - k0) < kOuter ? n - k0 : kOuter;
         for (int64_t j0 = k0; j0 < k0 + w; j0 += NB) {
             const int jb = (int)((k0 + w - j0) < NB ? k0 + w - j0 : NB);
-            potrf_diag<T><<<1, 256, kDiagSmem, s>>>(A.sub(j0, j0), jb, j0, W, info, false);
+            potrf_diag<T><<<1, kDiagThreads, kDiagSmem, s>>>(A.sub(j0, j0), jb, j0, W, info, false);
             RC_TRY(check_launch());
             const int64_t rows = n - j0 - jb;
             if (rows <= 0) continue;
@@ -433,7 +665,7 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s) {
 template <class T>
 int potrf_diag_block(View<T> A, int sz, int64_t g0, T* W, bool w_row_major, int* info, cudaStream_t s) {
     RC_TRY(set_smem(potrf_diag<T>, kDiagSmem));
-    potrf_diag<T><<<1, 256, kDiagSmem, s>>>(A, sz, g0, W, info, w_row_major);
+    potrf_diag<T><<<1, kDiagThreads, kDiagSmem, s>>>(A, sz, g0, W, info, w_row_major);
     return check_launch();
 }
 
@@ -461,8 +693,8 @@ int trsm_preinv(bool trans, int64_t m, int64_t n, View<const T> L, const T* Winv
 template <class T>
 int trtri_blocks_launch(int64_t m, View<const T> L, bool unit, T* W, int* info, const int* abort, cudaStream_t s) {
     if (m <= 0) return RC_SUCCESS;
-    RC_TRY(set_smem(trtri_blocks<T>, kBlockSmem));
-    trtri_blocks<T><<<(unsigned)((m + NB - 1) / NB), NB, kBlockSmem, s>>>(m, L, unit, W, info, abort);
+    RC_TRY(set_smem(trtri_blocks<T>, kDiagSmem));
+    trtri_blocks<T><<<(unsigned)((m + NB - 1) / NB), kDiagThreads, kDiagSmem, s>>>(m, L, unit, W, info, abort);
     return check_launch();
 }
 
