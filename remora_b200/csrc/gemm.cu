@@ -4,13 +4,14 @@
 // (include/remora/hip/cublas_backend.hpp:121-166, :389-431, called from
 // include/remora/kernels/hip/gemm.hpp:46-112 and kernels/hip/syrk.hpp:44-85).
 //
-// Two kernels:
+// Three kernels:
 //  * gemm_dmma_f64: the FP64 tensor-core path (DMMA, mma.sync m16n8k4 f64), a family of
 //    CTA tiles from 128 x 128 down to 32 x 32 over one kernel template. Operand tiles are
 //    staged by 16-byte cp.async (8-byte where the alignment asks for it) in the order of
 //    their global layout, so all four transpose combinations run at the same rate.
-//  * gemm_simt: a generic strided FP32/FP64 kernel (64x64x16 tiles, 4x4 outer products
-//    per thread) for operands with no unit stride and for FP32.
+//  * sgemm_simt: FP32 on the FMA units, register tiles of packed pairs.
+//  * gemm_simt: a generic strided kernel (64x64x16 tiles, 4x4 outer products per thread) for
+//    operands with no unit stride.
 // Both honour a triangle mask (SYRK writes one triangle; whole tiles outside it exit at
 // once) and an abort word (a failed Cholesky pivot stops the trailing updates).
 #include "gemm.cuh"
@@ -89,6 +90,208 @@ __global__ void __launch_bounds__(256) gemm_simt(int64_t m, int64_t n, int64_t k
             C(i, j) = v;
         }
     }
+}
+
+// ------------------------------------------------------------------------------------
+// FP32 kernel on the FMA units (68.6 TFLOP/s measured on registers alone), exact FP32
+// accumulation in ascending k. Operand tiles go through registers into shared memory as
+// [k][m] and [k][n], two buffers, the next tile's loads in flight under the current one's
+// products. A thread owns GM x GN groups of 4 x 4 elements of C, so that one 16-byte fragment
+// load feeds 4 GN (4 GM) products; a warp is 4 (m) x 8 (n) threads, whose fragment loads cover
+// 64 and 128 distinct bytes. Products are packed pairs along n (fma.rn.f32x2): half the issue
+// slots, the rest of which hold the fragment loads.
+template <int BM_, int BN_, int GM_, int GN_, int OCC_>
+struct SimtTile {
+    static constexpr int BM = BM_, BN = BN_, GM = GM_, GN = GN_, OCC = OCC_, BK = 16;
+    static constexpr int WARPS_M = BM / (16 * GM), WARPS_N = BN / (32 * GN), THREADS = 32 * WARPS_M * WARPS_N;
+    static constexpr int LDA = BM + 4, LDB = BN + 4;
+};
+// 128 x 64 with three CTAs of 4 warps per SM: 4096^3 in 2.65 ms (52 TFLOP/s; the 64 x 64 tile
+// of one 4 x 4 group a thread and one barrier-bound buffer took 6.2), 1024^3 in 68 us (153). The
+// variants 128 x 128 of 8 warps (2.59-2.75 ms, 115 us), of 4 warps (2.60-2.63, 115) and 64 x 64
+// of 2 warps (2.75-2.80, 73) are no better on large products and worse on middle ones. Below
+// about a tile per SM the 32 x 32 tile wins: 512^3 in 19 us (37 with 128 x 64).
+using SimtL = SimtTile<128, 64, 2, 2, 3>;
+using SimtS = SimtTile<32, 32, 1, 1, 12>;
+
+// One thread's share of a 16-deep operand tile: groups of 4 elements along the contiguous
+// direction (k when KM, else the row direction), zero outside rows x k. V16: 16-byte loads are
+// aligned.
+template <bool KM, int ROWS, int THREADS, bool V16>
+struct SimtLoader {
+    static constexpr int COUNT = ROWS * 16 / 4, PER = (COUNT + THREADS - 1) / THREADS;
+    static constexpr int RUN = (KM ? 16 : ROWS) / 4;  // groups per contiguous run
+    static __device__ __forceinline__ void load(float4 (&v)[PER], const float* p, int64_t ld, int64_t rows, int64_t k,
+                                                int64_t r0, int64_t k0, int tid) {
+        const bool inside = r0 + ROWS <= rows && k0 + 16 <= k;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int q = tid + e * THREADS, c = q % RUN * 4, o = q / RUN;
+            const int row = KM ? o : c, kk = KM ? c : o;
+            v[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (COUNT % THREADS != 0 && q >= COUNT) continue;
+            const float* src = KM ? p + (r0 + row) * ld + k0 + kk : p + r0 + row + (k0 + kk) * ld;
+            if (V16 && inside) {
+                v[e] = *reinterpret_cast<const float4*>(src);
+            } else {
+                const int64_t left = KM ? (r0 + row < rows ? k - (k0 + kk) : 0) : (k0 + kk < k ? rows - (r0 + row) : 0);
+                if (left > 0) v[e].x = src[0];
+                if (left > 1) v[e].y = src[1];
+                if (left > 2) v[e].z = src[2];
+                if (left > 3) v[e].w = src[3];
+            }
+        }
+    }
+    static __device__ __forceinline__ void store(const float4 (&v)[PER], float* dst, int ldt, int tid) {
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int q = tid + e * THREADS, c = q % RUN * 4, o = q / RUN;
+            if (COUNT % THREADS != 0 && q >= COUNT) continue;
+            if (KM) {
+                dst[c * ldt + o] = v[e].x;
+                dst[(c + 1) * ldt + o] = v[e].y;
+                dst[(c + 2) * ldt + o] = v[e].z;
+                dst[(c + 3) * ldt + o] = v[e].w;
+            } else {
+                *reinterpret_cast<float4*>(dst + o * ldt + c) = v[e];
+            }
+        }
+    }
+};
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+template <bool A_KMAJOR, bool B_KMAJOR, class Tile, bool V16>
+__global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
+    sgemm_simt(int64_t m, int64_t n, int64_t k, float alpha, View<const float> A, View<const float> B, float beta,
+               View<float> C, Mask mask, int64_t off, const int* abort) {
+    constexpr int BM = Tile::BM, BN = Tile::BN, GM = Tile::GM, GN = Tile::GN, BK = Tile::BK;
+    constexpr int LDA = Tile::LDA, LDB = Tile::LDB;
+    using LA = SimtLoader<A_KMAJOR, BM, Tile::THREADS, V16>;
+    using LB = SimtLoader<B_KMAJOR, BN, Tile::THREADS, V16>;
+    __shared__ __align__(16) float sA[2][BK * LDA];
+    __shared__ __align__(16) float sB[2][BK * LDB];
+    constexpr int64_t kGroupM = 1024 / BM;  // grouped tile order, as gemm_dmma_f64
+    const int64_t lin = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, per = kGroupM * gridDim.x;
+    const int64_t first = lin / per * kGroupM, rest = (int64_t)gridDim.y - first;
+    const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
+    const int64_t m0 = (first + r % gsz) * BM, n0 = r / gsz * BN;
+    if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tm = (warp / Tile::WARPS_N) * 16 + (lane >> 3) * 4, tn = (warp % Tile::WARPS_N) * 32 + (lane & 7) * 4;
+    const int64_t lda = A_KMAJOR ? A.rs : A.cs, ldb = B_KMAJOR ? B.cs : B.rs;
+    uint64_t acc[GM * 4][GN * 2];
+#pragma unroll
+    for (int i = 0; i < GM * 4; ++i)
+#pragma unroll
+        for (int j = 0; j < GN * 2; ++j) acc[i][j] = 0;
+    float4 va[LA::PER], vb[LB::PER];
+    LA::load(va, A.p, lda, m, k, m0, 0, tid);
+    LB::load(vb, B.p, ldb, n, k, n0, 0, tid);
+    LA::store(va, sA[0], LDA, tid);
+    LB::store(vb, sB[0], LDB, tid);
+    __syncthreads();
+    const int KT = (int)((k + BK - 1) / BK);
+    for (int kt = 0; kt < KT; ++kt) {
+        const bool more = kt + 1 < KT;
+        if (more) {
+            LA::load(va, A.p, lda, m, k, m0, (int64_t)(kt + 1) * BK, tid);
+            LB::load(vb, B.p, ldb, n, k, n0, (int64_t)(kt + 1) * BK, tid);
+        }
+        const float *a_s = sA[kt & 1] + tm, *b_s = sB[kt & 1] + tn;
+#pragma unroll
+        for (int kk = 0; kk < BK; ++kk) {
+            float4 a[GM];
+            ulonglong2 b[GN];
+#pragma unroll
+            for (int q = 0; q < GM; ++q) a[q] = *reinterpret_cast<const float4*>(a_s + kk * LDA + q * (BM / GM));
+#pragma unroll
+            for (int q = 0; q < GN; ++q) b[q] = *reinterpret_cast<const ulonglong2*>(b_s + kk * LDB + q * (BN / GN));
+#pragma unroll
+            for (int q = 0; q < GM; ++q) {
+                const float ai[4] = {a[q].x, a[q].y, a[q].z, a[q].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint64_t aa = pack2(ai[i], ai[i]);
+#pragma unroll
+                    for (int j = 0; j < GN; ++j) {
+                        fma2(acc[4 * q + i][2 * j], aa, b[j].x);
+                        fma2(acc[4 * q + i][2 * j + 1], aa, b[j].y);
+                    }
+                }
+            }
+        }
+        if (more) {
+            LA::store(va, sA[(kt + 1) & 1], LDA, tid);
+            LB::store(vb, sB[(kt + 1) & 1], LDB, tid);
+            __syncthreads();
+        }
+    }
+    // Epilogue: 4 x 4 group by group; the old C of a group is fetched before any of it is
+    // written; 16-byte accesses along C's contiguous direction where the group lies inside.
+    const bool colC = C.rs == 1, vecC = (colC || C.cs == 1) && (colC ? C.cs : C.rs) % 4 == 0 &&
+                                        reinterpret_cast<uintptr_t>(C.p) % 16 == 0;
+    const int64_t ci = colC ? C.cs : C.rs;
+#pragma unroll
+    for (int gm = 0; gm < GM; ++gm)
+#pragma unroll
+        for (int gn = 0; gn < GN; ++gn) {
+            const int64_t i0 = m0 + tm + gm * (BM / GM), j0 = n0 + tn + gn * (BN / GN);
+            float v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(v[i][2 * j]), "=f"(v[i][2 * j + 1]) : "l"(acc[4 * gm + i][2 * gn + j]));
+            const bool inside = i0 + 4 <= m && j0 + 4 <= n &&
+                                (mask == kFull || (mask == kLower ? i0 - (j0 + 3) >= off : (i0 + 3) - j0 <= off));
+            if (vecC && inside) {
+                float4* c4[4];
+                float4 old[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    c4[q] = reinterpret_cast<float4*>(C.p + (colC ? i0 + (j0 + q) * ci : (i0 + q) * ci + j0));
+                    if (beta != 0.f) old[q] = *c4[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float w[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) w[u] = alpha * (colC ? v[u][q] : v[q][u]);
+                    if (beta != 0.f) {
+                        w[0] = fmaf(beta, old[q].x, w[0]);
+                        w[1] = fmaf(beta, old[q].y, w[1]);
+                        w[2] = fmaf(beta, old[q].z, w[2]);
+                        w[3] = fmaf(beta, old[q].w, w[3]);
+                    }
+                    *c4[q] = make_float4(w[0], w[1], w[2], w[3]);
+                }
+            } else {
+                float old[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        old[i][j] = beta != 0.f && i0 + i < m && j0 + j < n && in_mask(mask, off, i0 + i, j0 + j)
+                                        ? C(i0 + i, j0 + j) : 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (i0 + i >= m || j0 + j >= n || !in_mask(mask, off, i0 + i, j0 + j)) continue;
+                        float w = alpha * v[i][j];
+                        if (beta != 0.f) w = fmaf(beta, old[i][j], w);
+                        C(i0 + i, j0 + j) = w;
+                    }
+            }
+        }
 }
 
 // ------------------------------------------------------------------------------------
@@ -408,6 +611,44 @@ int gemm_dmma(int64_t m, int64_t n, int64_t k, double alpha, View<const double> 
     return launch_tile<AK, BK, false>(id, p, alpha, A, B, beta, C, off, nz, s, abort);
 }
 
+// Cycles an FP32 product takes with a tile (the FMA units do BM BN BK / 128 a k-step, of which
+// a tile reaches the share eff: 0.78 measured at 4096^3 and 0.40 at 1024^3; a k-step of a lone tile takes
+// `chain` cycles: 1900 and 800 measured at 512^3; see tile_cycles).
+template <class Tile>
+double simt_cycles(const Shape& s, double eff, double chain) {
+    const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
+    if (tm > 65535) return 1e200;
+    double tiles = (double)tm * tn;
+    if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));
+    const double per_sm = ceil(tiles / sm_count()), work = Tile::BM * Tile::BN * Tile::BK / 128.0 / eff;
+    const double ksteps = ceil((double)s.k / Tile::BK), full = floor(per_sm / Tile::OCC), rest = per_sm - full * Tile::OCC;
+    auto round = [&](double c) { return c <= 0 ? 0.0 : ksteps * (c * work > chain ? c * work : chain) + 3000.0; };
+    return full * round(Tile::OCC) + round(rest);
+}
+
+template <bool AK, bool BK, class Tile>
+int launch_sgemm(const Shape& p, float alpha, View<const float> A, View<const float> B, float beta, View<float> C,
+                 int64_t off, cudaStream_t s, const int* abort) {
+    auto aligned = [](const float* q, int64_t ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
+    const dim3 grid(ceil_div(p.n, Tile::BN), ceil_div(p.m, Tile::BM));
+    if (aligned(A.p, AK ? A.rs : A.cs) && aligned(B.p, BK ? B.cs : B.rs))
+        sgemm_simt<AK, BK, Tile, true><<<grid, Tile::THREADS, 0, s>>>(p.m, p.n, p.k, alpha, A, B, beta, C, p.mask, off,
+                                                                      abort);
+    else
+        sgemm_simt<AK, BK, Tile, false><<<grid, Tile::THREADS, 0, s>>>(p.m, p.n, p.k, alpha, A, B, beta, C, p.mask,
+                                                                       off, abort);
+    return check_launch();
+}
+
+template <bool AK, bool BK>
+int sgemm(int64_t m, int64_t n, int64_t k, float alpha, View<const float> A, View<const float> B, float beta,
+          View<float> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
+    const Shape p{m, n, k, mask};
+    if (simt_cycles<SimtL>(p, 0.78, 1900.0) <= simt_cycles<SimtS>(p, 0.40, 800.0))
+        return launch_sgemm<AK, BK, SimtL>(p, alpha, A, B, beta, C, off, s, abort);
+    return launch_sgemm<AK, BK, SimtS>(p, alpha, A, B, beta, C, off, s, abort);
+}
+
 // Scale (beta != 1) the masked part of C when k == 0 or alpha == 0.
 template <class T>
 __global__ void scale_masked(int64_t m, int64_t n, T beta, View<T> C, Mask mask, int64_t off, const int* abort) {
@@ -429,14 +670,18 @@ int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T
         scale_masked<T><<<grid, 256, 0, s>>>(m, n, beta, C, mask, off, abort);
         return check_launch();
     }
-    if constexpr (std::is_same<T, double>::value) {
-        const bool a_k = A.cs == 1, a_m = A.rs == 1, b_k = B.rs == 1, b_n = B.cs == 1;
-        if ((a_k || a_m) && (b_k || b_n)) {
-            if (a_k && b_k) return gemm_dmma<true, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            if (a_k) return gemm_dmma<true, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            if (b_k) return gemm_dmma<false, true>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-            return gemm_dmma<false, false>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-        }
+    const bool a_k = A.cs == 1, a_m = A.rs == 1, b_k = B.rs == 1, b_n = B.cs == 1;
+    if ((a_k || a_m) && (b_k || b_n)) {
+        auto run = [&](auto ak, auto bk) {
+            if constexpr (std::is_same<T, double>::value)
+                return gemm_dmma<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+            else
+                return sgemm<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+        };
+        if (a_k && b_k) return run(std::true_type{}, std::true_type{});
+        if (a_k) return run(std::true_type{}, std::false_type{});
+        if (b_k) return run(std::false_type{}, std::true_type{});
+        return run(std::false_type{}, std::false_type{});
     }
     dim3 grid(ceil_div(n, 64), ceil_div(m, 64));
     gemm_simt<T><<<grid, 256, 0, s>>>(m, n, k, alpha, A, B, beta, C, mask, off, abort);
