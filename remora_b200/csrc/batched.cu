@@ -8,15 +8,27 @@
 //  * persistent CTAs (a multiple of the SM count) pull systems from an atomic work
 //    counter over an order sorted by decreasing n, so the large systems start first and
 //    the small ones fill the tail -- no inter-CTA waiting, only one atomicAdd per system;
-//  * per system, a right-looking Cholesky in NB-column steps: the NB x NB diagonal block
-//    is factored in shared memory (one element per thread-slot, one barrier per column),
-//    the panel below is solved row-parallel against it and kept in shared memory, and the
-//    trailing lower triangle is updated in 4 x 4 register tiles read from that panel;
-//  * then the forward and backward substitutions for the right-hand side, in shared
-//    memory;
+//  * per system, a left-looking Cholesky in 32-column panels on DMMA, in FP64 also for float
+//    matrices: the panel's rows, as 32 x 32 warp tiles in registers, subtract the product of
+//    the columns before them (fragments straight from global memory, which L2 and L1 hold:
+//    each element of L is read once per panel to its right, where a right-looking update
+//    would read and write the whole trailing triangle per panel), and are solved with the
+//    inverse of the panel's diagonal block;
+//  * one warp factors and inverts the diagonal block (diag.cuh) while the others update the
+//    rows below it;
+//  * the right-hand side's forward substitution is part of the panels; the backward
+//    substitution walks the panels with the kept inverses;
 //  * a failing pivot records its 1-based index in info[i] and the CTA moves on.
-// The tile configuration (NB, threads) is chosen per (precision, size bucket) by a small
-// autotuner that times every candidate on the caller's batch once and caches the winner.
+// The warps per CTA are chosen per (precision, size bucket) by a small autotuner that times
+// every candidate on the caller's batch once and caches the winner.
+//
+// 1024 systems of 16 to 512 rows: 1.04 ms in FP64, 1.00 ms in FP32 (12.3 and 10.4 ms with FMA
+// tiles over a right-looking update and one barrier per column), 11.9 GFLOP of which the DMMA
+// pipe could do in 0.35 ms. What is left is latency: a 512-row system alone takes 0.52 ms, its
+// 16 panels ~35K cycles each for the loads, the 32 dependent columns and three barriers. Tiles
+// kept in registers from their update to their solve (which spill at two CTAs per SM) took
+// 1.8 ms; the code is kept small (one form of each tile) because the phases of a panel are
+// bound by instruction fetch before anything else.
 #include <algorithm>
 #include <map>
 #include <memory>
@@ -26,182 +38,331 @@
 #include <vector>
 
 #include "common.cuh"
+#include "diag.cuh"
 
 namespace rc {
 namespace {
 
 constexpr int kMaxN = 512;
 
-template <class T, int NB>
+constexpr int PB = 32;      // panel width
+constexpr int DLD = PB + 4;  // row stride of the diagonal block in shared memory
+constexpr int kPacked = PB * (PB + 1) / 2;
+
+// Shared memory (doubles): two diagonal blocks (this panel's and the next's), the scratch of
+// their factorisation, the right-hand side y (then L^-1 b, then the solution), a panel's part
+// of it and the packed inverses of the diagonal blocks of a matrix of up to nmax rows.
 struct BatchedSmem {
-    static constexpr int LD = NB + 1;
-    static constexpr size_t bytes = (size_t)(NB * LD + kMaxN * LD + kMaxN) * sizeof(T);
+    static constexpr int D = 0, Lt = D + 2 * PB * DLD, T16 = Lt + kDB * kLTD, ld = T16 + 16 * 20, rd = ld + PB,
+                         flags = rd + PB, y = flags + 2, t = y + kMaxN + PB, inv = t + PB;
+    static size_t bytes(int nmax) { return (size_t)(inv + (nmax + PB - 1) / PB * kPacked) * sizeof(double); }
 };
 
-template <class T, int NB, int THREADS>
-__global__ void __launch_bounds__(THREADS) batched_chol_solve(int count, const int* __restrict__ order,
-                                                             const int* __restrict__ sizes, T* const* __restrict__ Aptr,
-                                                             T* const* __restrict__ bptr, int* __restrict__ info,
-                                                             int* __restrict__ next) {
-    constexpr int LD = NB + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* D = reinterpret_cast<T*>(smem_raw);  // NB x LD diagonal block, row-major
-    T* P = D + NB * LD;                      // up to kMaxN x LD panel rows, row-major
-    T* x = P + kMaxN * LD;                   // right-hand side / solution
-    __shared__ int s_work, s_fail;
-    const int tid = threadIdx.x;
+// P = C - L(rows, 0 : k0) L(k0 : k0 + 32, 0 : k0)^T on the 32-row tile at r0 of the panel at k0, in
+// place, by one warp. Rows past the matrix stand on its last row and are not stored. The
+// fragments of two k-steps ahead are in flight; the last two fetches read columns of the panel
+// itself, which exist (n > r0 >= k0 + 32), and are not used.
+template <class T>
+__device__ __forceinline__ void update_tile(T* A, int n, int k0, int r0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = r0 + 8 * u + g < n ? r0 + 8 * u + g : n - 1;
+    double acc[2][4][4] = {};
+    const T *a = A + (int64_t)t * n, *b = a + k0 + g;
+    const int64_t step = 4 * (int64_t)n;
+    T av[4][4], bv[4][4];  // three of the four stages are live at a time
+    auto fetch = [&](int st) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            av[st][u] = a[row[u]];
+            bv[st][u] = b[8 * u];
+        }
+        a += step;
+        b += step;
+    };
+    fetch(0);
+    fetch(1);
+#pragma unroll 1
+    for (int k = 0; k < k0; k += 16)
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+            fetch((st + 2) & 3);
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+                    dmma_16x8x4(acc[mi][ni], (double)av[st][2 * mi], (double)av[st][2 * mi + 1], (double)bv[st][ni]);
+        }
+    T* c = A + (int64_t)(k0 + 2 * t) * n;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) {
+        T old[2][4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) old[e][u] = c[e * n + row[u]];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (r0 + 8 * u + g < n) c[e * n + row[u]] = (T)((double)old[e][u] - acc[u >> 1][ni][2 * (u & 1) + e]);
+        c += 8 * (int64_t)n;
+    }
+}
+
+// X = P inv(L_kk)^T on one tile, in place (all of it is loaded before any is stored), and
+// y(rows) -= X y(k0 : k0 + 32): the forward substitution of the right-hand side. D holds the
+// diagonal block's inverse, yp = y + k0.
+template <class T>
+__device__ __forceinline__ void solve_tile(T* A, const double* D, const double* yp, double* y, int n, int k0, int r0,
+                                           int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = r0 + 8 * u + g < n ? r0 + 8 * u + g : n - 1;
+    T av[8][4];
+    const T* p = A + (int64_t)(k0 + t) * n;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) av[q][u] = p[row[u]];
+        p += 4 * (int64_t)n;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi) {
+        double acc[4][4] = {};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = 4 * q + t;
+#pragma unroll
+            for (int ni = q / 2; ni < 4; ++ni) {  // inv(c, k), c = 8 ni + g: zero below the diagonal
+                double v = D[k * DLD + 8 * ni + g];
+                if (ni == q / 2) v = k <= 8 * ni + g ? v : 0.0;
+                dmma_16x8x4(acc[ni], (double)av[q][2 * mi], (double)av[q][2 * mi + 1], v);
+            }
+        }
+        T* c = A + (int64_t)(k0 + 2 * t) * n;
+        double dot[2] = {};
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    dot[h] = fma(acc[ni][2 * h + e], yp[8 * ni + 2 * t + e], dot[h]);
+                    if (r0 + 16 * mi + 8 * h + g < n) c[e * n + row[2 * mi + h]] = (T)acc[ni][2 * h + e];
+                }
+            c += 8 * (int64_t)n;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            dot[h] += __shfl_xor_sync(0xffffffffu, dot[h], 1);
+            dot[h] += __shfl_xor_sync(0xffffffffu, dot[h], 2);
+            if (t == 0 && r0 + 16 * mi + 8 * h + g < n) y[r0 + 16 * mi + 8 * h + g] -= dot[h];
+        }
+    }
+}
+
+// Factor the 32 x 32 block in D by one warp and build its inverse: two 16-column sub-blocks, then
+// one merge. flags[0]: 1 + the failing column of the block, or 0.
+__device__ __forceinline__ void factor_block(double* D, double* Lt, double* T16, double* ld, double* rd,
+                                             volatile int* flags, int lane) {
+#pragma unroll 1
+    for (int c0 = 0; c0 < PB; c0 += kDB) {
+        const bool mine = c0 + lane < PB;
+        double* row = D + (mine ? c0 + lane : c0) * DLD + c0;
+        double x[kDB];
+#pragma unroll
+        for (int c = 0; c < kDB; c += 2) {
+            const double2 v = reinterpret_cast<const double2*>(row)[c / 2];
+            x[c] = v.x;
+            x[c + 1] = v.y;
+        }
+        factor_sub_block(x, Lt, ld + c0, rd + c0, lane, flags, [](int) {});
+        __syncwarp();
+        if (flags[1]) {
+            factor_sub_block_any(row, mine, Lt, ld + c0, rd + c0, lane, flags, [](int) {});
+        } else if (mine) {
+#pragma unroll
+            for (int q = 0; q < kDB; ++q)
+                if (q < lane) row[q] = x[q];
+        }
+        __syncwarp();
+        if (flags[0]) {
+            if (lane == 0) flags[0] = flags[0] + c0;
+            return;
+        }
+        // this sub-block's inverse, and the update of the next one
+#pragma unroll
+        for (int q = 0; q < kDB; ++q) x[q] = q == lane ? 1.0 : 0.0;
+        solve_sub_block(x, rd + c0, Lt, [](int) {});
+        if (lane < kDB) {
+#pragma unroll
+            for (int q = 0; q < kDB; ++q)
+                if (q >= lane) row[q] = x[q];
+        }
+        if (c0 == 0) {
+            syrk_tile<DLD>(D, kDB, kDB, 0, lane);
+            syrk_tile<DLD>(D, kDB, kDB + 8, 0, lane);
+        }
+        __syncwarp();
+    }
+    merge_t<16, DLD>(D, T16, 0, 0, lane);
+    merge_t<16, DLD>(D, T16, 0, 1, lane);
+    __syncwarp();
+    merge_x<16, DLD>(D, T16, 0, 0, 0, lane);
+    merge_x<16, DLD>(D, T16, 0, 0, 8, lane);
+    __syncwarp();
+}
+
+// D -= L(rows, ka : kb) L(rows, ka : kb)^T on tiles q, q + 1 (of the six 16 x 8 tiles on and
+// below the diagonal: 0, 1 in rows 0 .. 15, 2 .. 5 in rows 16 .. 31) of the diagonal block at r0;
+// first: D starts from the matrix (the identity beyond its n rows).
+template <class T>
+__device__ __forceinline__ void diag_tiles(const T* A, int n, int r0, int ka, int kb, int q, bool first, double* D,
+                                           int lane) {
+    const int g = lane >> 2, t = lane & 3, i0 = q < 2 ? 0 : 16, j0 = q < 4 ? 0 : 16;
+    auto row = [&](int i) { return A + (r0 + i < n ? r0 + i : n - 1) + (int64_t)(ka + t) * n; };
+    const T *a0 = row(i0 + g), *a1 = row(i0 + g + 8), *b0 = row(j0 + g), *b1 = row(j0 + g + 8);
+    double acc[2][4] = {};
+    const int64_t step = 4 * (int64_t)n;
+#pragma unroll 4
+    for (int k = ka; k < kb; k += 4) {
+        const double x0 = (double)*a0, x1 = (double)*a1, y0 = (double)*b0, y1 = (double)*b1;
+        a0 += step;
+        a1 += step;
+        b0 += step;
+        b1 += step;
+        dmma_16x8x4(acc[0], x0, x1, y0);
+        dmma_16x8x4(acc[1], x0, x1, y1);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = i0 + g + 8 * (e >> 1), c = j0 + 8 * h + 2 * t + (e & 1);
+            double v = r == c ? 1.0 : 0.0;
+            if (!first) v = D[r * DLD + c];
+            else if (c <= r && r0 + r < n) v = (double)A[(r0 + r) + (int64_t)(r0 + c) * n];
+            D[r * DLD + c] = r0 + r < n ? v - acc[h][e] : v;
+        }
+}
+
+template <class T, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) batched_chol_solve(int count, const int* __restrict__ order,
+                                                                       const int* __restrict__ sizes,
+                                                                       T* const* __restrict__ Aptr,
+                                                                       T* const* __restrict__ bptr,
+                                                                       int* __restrict__ info, int* __restrict__ next) {
+    extern __shared__ __align__(16) double sm[];
+    using M = BatchedSmem;
+    double *D = sm + M::D, *ld = sm + M::ld, *rd = sm + M::rd, *y = sm + M::y, *tv = sm + M::t, *inv = sm + M::inv;
+    volatile int* flags = reinterpret_cast<int*>(sm + M::flags);
+    __shared__ int s_work;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int THREADS = 32 * NW;
     while (true) {
         __syncthreads();
         if (tid == 0) s_work = atomicAdd(next, 1);
         __syncthreads();
-        const int w = s_work;
-        if (w >= count) break;
-        const int sys = order[w];
+        if (s_work >= count) break;
+        const int sys = order[s_work];
         const int n = sizes[sys];
         T* A = Aptr[sys];  // column-major, ld = n
         T* b = bptr[sys];
-        if (tid == 0) s_fail = 0;
-        for (int r = tid; r < n; r += THREADS) x[r] = b[r];
-        __syncthreads();
-        for (int k = 0; k < n; k += NB) {
-            const int kb = min(NB, n - k);
-            // 1. diagonal block into shared memory (lower part)
-            for (int e = tid; e < kb * kb; e += THREADS) {
-                const int r = e % kb, c = e / kb;
-                D[r * LD + c] = c <= r ? A[(k + r) + (size_t)(k + c) * n] : T(0);
+        for (int i = tid; i < n + PB; i += THREADS) y[i] = i < n ? (double)b[i] : 0.0;
+        int failed = 0;
+        for (int k0 = 0; k0 < n; k0 += PB) {
+            // The diagonal block: the last panel's update (the earlier ones' came with that
+            // panel's, below).
+            double *Dk = D + (k0 / PB & 1) * PB * DLD, *Dn = D + (~(k0 / PB) & 1) * PB * DLD;
+            for (int q = warp; q < 3; q += NW)
+                diag_tiles(A, n, k0, k0 > 0 ? k0 - PB : 0, k0, 2 * q, k0 == 0, Dk, lane);
+            __syncthreads();
+            const int r1 = k0 + PB, tiles = r1 < n ? (n - r1 + 31) / 32 : 0;
+            if (warp == 0) {
+                factor_block(Dk, sm + M::Lt, sm + M::T16, ld, rd, flags, lane);
+                double v = 0.0;  // y(k0 : k0 + 32) solved with the block
+#pragma unroll 8
+                for (int k = 0; k < PB; ++k)
+                    if (k <= lane) v = fma(Dk[k * DLD + lane], y[k0 + k], v);
+                __syncwarp();
+                y[k0 + lane] = v;
+            } else if (tiles > 0) {  // the rows below it, and the next diagonal block's update so far
+                for (int q = warp - 1; q < tiles + 3; q += NW - 1) {
+                    if (q < 3) diag_tiles(A, n, r1, 0, k0, 2 * q, true, Dn, lane);
+                    else if (k0 > 0) update_tile(A, n, k0, r1 + 32 * (q - 3), lane);
+                }
             }
             __syncthreads();
-            // 2. factor it: per column, the pivot, the column scaling, the rank-1 update
-            for (int j = 0; j < kb; ++j) {
-                const T d = D[j * LD + j];
-                if (!(d > T(0))) {
-                    if (tid == 0) s_fail = k + j + 1;
-                    break;  // uniform: every thread read the same d
-                }
-                const T sq = sqrt(d);
-                __syncthreads();
-                for (int r = j + tid; r < kb; r += THREADS) D[r * LD + j] = r == j ? sq : D[r * LD + j] / sq;
-                __syncthreads();
-                const int t = kb - j - 1;
-                for (int e = tid; e < t * t; e += THREADS) {
-                    const int r = j + 1 + e / t, c = j + 1 + e % t;
-                    if (c <= r) D[r * LD + c] -= D[r * LD + j] * D[c * LD + j];
-                }
-                __syncthreads();
+            if (flags[0]) {
+                failed = k0 + flags[0];
+                break;
             }
-            __syncthreads();
-            if (s_fail) break;
-            for (int e = tid; e < kb * kb; e += THREADS) {
-                const int r = e % kb, c = e / kb;
-                if (c <= r) A[(k + r) + (size_t)(k + c) * n] = D[r * LD + c];
-            }
-            // 3. panel rows below: solve x L_kk^T = a row by row (forward substitution)
-            const int m = n - k - kb;
-            for (int r = tid; r < m; r += THREADS) {
-                T* pr = P + r * LD;
-                for (int c = 0; c < kb; ++c) {
-                    T v = A[(k + kb + r) + (size_t)(k + c) * n];
-                    for (int q = 0; q < c; ++q) v -= pr[q] * D[c * LD + q];
-                    pr[c] = v / D[c * LD + c];
-                }
-                for (int c = 0; c < kb; ++c) A[(k + kb + r) + (size_t)(k + c) * n] = pr[c];
-            }
-            __syncthreads();
-            // 4. trailing update of the lower triangle, 4 x 4 tiles
-            const int tiles = (m + 3) / 4;
-            const int ntile = tiles * (tiles + 1) / 2;
-            for (int t = tid; t < ntile; t += THREADS) {
-                // t -> (tr, tc) with tc <= tr, row-major over the lower triangle of tiles
-                int tr = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-                while ((tr + 1) * (tr + 2) / 2 <= t) ++tr;
-                while (tr * (tr + 1) / 2 > t) --tr;
-                const int tc = t - tr * (tr + 1) / 2;
-                const int r0 = 4 * tr, c0 = 4 * tc;
-                T acc[4][4] = {};
-                for (int q = 0; q < kb; ++q) {
-                    T pr[4], pc[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        pr[u] = r0 + u < m ? P[(r0 + u) * LD + q] : T(0);
-                        pc[u] = c0 + u < m ? P[(c0 + u) * LD + q] : T(0);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) acc[u][v] += pr[u] * pc[v];
-                }
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int c = c0 + v;
-                    if (c >= m) continue;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int r = r0 + u;
-                        if (r >= m || r < c) continue;
-                        A[(k + kb + r) + (size_t)(k + kb + c) * n] -= acc[u][v];
-                    }
-                }
+            for (int q = warp; q < tiles; q += NW) solve_tile(A, Dk, y + k0, y, n, k0, r1 + 32 * q, lane);
+            // the diagonal block and its inverse (packed by rows)
+            double* pk = inv + (k0 / PB) * kPacked;
+            for (int e = tid; e < PB * PB; e += THREADS) {
+                const int r = e % PB, c = e / PB;
+                if (c > r) continue;
+                pk[r * (r + 1) / 2 + c] = Dk[c * DLD + r];
+                if (k0 + r < n) A[(k0 + r) + (int64_t)(k0 + c) * n] = (T)(r == c ? ld[r] : Dk[r * DLD + c]);
             }
             __syncthreads();
         }
-        if (s_fail) {
-            if (tid == 0) info[sys] = s_fail;
+        if (failed) {
+            if (tid == 0) info[sys] = failed;
             continue;
         }
-        // 5. L y = b, then L^T x = y (one barrier per column), x in shared memory
-        for (int j = 0; j < n; ++j) {
-            if (tid == 0) x[j] /= A[j + (size_t)j * n];
+        // L^T x = y, panel by panel from the last: x_p = inv(L_pp)^T (y_p - L(below, p)^T x(below)).
+        // A warp sums 32 / NW columns, its lanes along the rows.
+        for (int k0 = (n - 1) / PB * PB; k0 >= 0; k0 -= PB) {
+            constexpr int NC = PB / NW;
+            double part[NC] = {};
+            const int c0 = k0 + NC * warp;
+#pragma unroll 2
+            for (int i = k0 + PB + lane; i < n; i += 32) {
+                const double xi = y[i];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) part[c] = fma((double)A[i + (int64_t)(c0 + c) * n], xi, part[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) part[c] += __shfl_xor_sync(0xffffffffu, part[c], off);
+                if (lane == c) tv[NC * warp + c] = y[c0 + c] - part[c];
+            }
             __syncthreads();
-            const T yj = x[j];
-            for (int r = j + 1 + tid; r < n; r += THREADS) x[r] -= A[r + (size_t)j * n] * yj;
-            __syncthreads();
-        }
-        for (int j = n - 1; j >= 0; --j) {
-            // x_j = (y_j - sum_{r > j} L_rj x_r) / L_jj: a block reduction per column
-            T part = T(0);
-            for (int r = j + 1 + tid; r < n; r += THREADS) part += A[r + (size_t)j * n] * x[r];
-            for (int off = 16; off > 0; off >>= 1) part += __shfl_down_sync(0xffffffffu, part, off);
-            __shared__ T red[32];
-            if ((tid & 31) == 0) red[tid >> 5] = part;
-            __syncthreads();
-            if (tid == 0) {
-                T s = T(0);
-                for (int q = 0; q < THREADS / 32; ++q) s += red[q];
-                x[j] = (x[j] - s) / A[j + (size_t)j * n];
+            if (warp == 0) {
+                const double* pk = inv + (k0 / PB) * kPacked;
+                double v = 0.0;
+#pragma unroll 8
+                for (int r = 0; r < PB; ++r)
+                    if (r >= lane) v = fma(pk[r * (r + 1) / 2 + lane], tv[r], v);
+                y[k0 + lane] = v;
             }
             __syncthreads();
         }
-        for (int r = tid; r < n; r += THREADS) b[r] = x[r];
+        for (int i = tid; i < n; i += THREADS) b[i] = (T)y[i];
         if (tid == 0) info[sys] = 0;
     }
 }
 
 struct Config {
-    int nb, threads;
+    int warps;
 };
 
 template <class T>
 using KernelFn = void (*)(int, const int*, const int*, T* const*, T* const*, int*, int*);
 
 template <class T>
-KernelFn<T> kernel_for(Config c, size_t* smem) {
-    if (c.nb == 32 && c.threads == 256) {
-        *smem = BatchedSmem<T, 32>::bytes;
-        return batched_chol_solve<T, 32, 256>;
-    }
-    if (c.nb == 32 && c.threads == 128) {
-        *smem = BatchedSmem<T, 32>::bytes;
-        return batched_chol_solve<T, 32, 128>;
-    }
-    if (c.nb == 16 && c.threads == 256) {
-        *smem = BatchedSmem<T, 16>::bytes;
-        return batched_chol_solve<T, 16, 256>;
-    }
-    *smem = BatchedSmem<T, 16>::bytes;
-    return batched_chol_solve<T, 16, 128>;
+KernelFn<T> kernel_for(Config c) {
+    return c.warps == 8 ? batched_chol_solve<T, 8> : batched_chol_solve<T, 4>;
 }
 
-const Config kCandidates[] = {{32, 256}, {32, 128}, {16, 256}, {16, 128}};
+const Config kCandidates[] = {{8}, {4}};
 
 // A plan: the device copy of sizes and order, the chosen configuration, the captured
 // graph (work-counter reset + the persistent kernel) for one set of pointer arrays.
@@ -213,7 +374,7 @@ struct Plan {
     const int* info = nullptr;
     std::vector<int> sizes;
     int* d_buf = nullptr;  // [next | order (count) | sizes (count)]
-    Config cfg{32, 256};
+    Config cfg{8};
     cudaGraphExec_t exec = nullptr;
     ~Plan() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -235,16 +396,16 @@ int size_bucket(const std::vector<int>& sizes) {
 
 template <class T>
 int launch_plain(const Plan& p, Config c, cudaStream_t s) {
-    size_t smem = 0;
-    auto fn = kernel_for<T>(c, &smem);
+    const size_t smem = BatchedSmem::bytes(*std::max_element(p.sizes.begin(), p.sizes.end()));
+    auto fn = kernel_for<T>(c);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return RC_ERR_CUDA;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, c.threads, smem) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * c.warps, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     const int grid = std::min(sm_count() * per_sm, std::max(p.count, 1));
     if (cudaMemsetAsync(p.d_buf, 0, sizeof(int), s) != cudaSuccess) return RC_ERR_CUDA;
-    fn<<<grid, c.threads, smem, s>>>(p.count, p.d_buf + 1, p.d_buf + 1 + p.count, (T* const*)p.A, (T* const*)p.b,
+    fn<<<grid, 32 * c.warps, smem, s>>>(p.count, p.d_buf + 1, p.d_buf + 1 + p.count, (T* const*)p.A, (T* const*)p.b,
                                     const_cast<int*>(p.info), p.d_buf);
     return check_launch();
 }

@@ -14,6 +14,7 @@
 //    kernel of the factorization returns at once.
 #include "factor.cuh"
 #include "assign.cuh"
+#include "diag.cuh"
 #include "gemm.cuh"
 #include <type_traits>
 
@@ -22,9 +23,9 @@ namespace {
 
 constexpr int NB = kNB;
 constexpr int SLD = NB + 4;  // shared-memory row stride (doubles): DMMA fragment loads hit all banks
-constexpr int DB = 16;       // diagonal sub-block
+constexpr int DB = kDB;      // diagonal sub-block
+constexpr int LTD = kLTD;    // column stride of the sub-block's transposed copy
 constexpr int NSUB = NB / DB;
-constexpr int LTD = 32;      // column stride of the sub-block's transposed copy
 constexpr int kDiagThreads = 512;
 
 // Shared memory of the diagonal-block kernels (doubles): S holds L in its strict lower
@@ -38,99 +39,14 @@ constexpr size_t kDiagSmem = kOffEnd * sizeof(double) + 16;
 
 __device__ __forceinline__ bool aborted(const int* abort) { return abort != nullptr && *(volatile const int*)abort != 0; }
 
-__device__ __forceinline__ void dmma_16x8x4(double (&d)[4], double a0, double a1, double b0) {
-    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a0), "d"(a1), "d"(b0));
-}
-
-// Tile (rows i0 .. i0 + 15, columns j0 .. j0 + 7) of S -= L(:, m0 : m0 + 16) L(:, m0 : m0 + 16)^T.
-__device__ __forceinline__ void syrk_tile(double* S, int i0, int j0, int m0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    double d[4] = {};
-#pragma unroll
-    for (int k = 0; k < DB; k += 4)
-        dmma_16x8x4(d, S[(i0 + g) * SLD + m0 + k + t], S[(i0 + g + 8) * SLD + m0 + k + t],
-                    S[(j0 + g) * SLD + m0 + k + t]);
-    double2* lo = reinterpret_cast<double2*>(S + (i0 + g) * SLD + j0 + 2 * t);
-    double2* hi = reinterpret_cast<double2*>(S + (i0 + g + 8) * SLD + j0 + 2 * t);
-    double2 a = *lo, b = *hi;
-    a.x -= d[0];
-    a.y -= d[1];
-    b.x -= d[2];
-    b.y -= d[3];
-    *lo = a;
-    *hi = b;
-}
-
 // The update of S by columns m0 .. m0 + 15 on the 16-row tiles from r0, columns from r0 up to
 // `width` 8-column tiles wide or to the diagonal, spread over n workers (number w).
 __device__ __forceinline__ void syrk_tiles(double* S, int r0, int width, int m0, int w, int n, int lane) {
     int e = w;
     for (int i0 = r0; i0 < NB; i0 += 16) {
         const int diag = (i0 - r0) / 8 + 2, cnt = diag < width ? diag : width;
-        for (; e < cnt; e += n) syrk_tile(S, i0, r0 + 8 * e, m0, lane);
+        for (; e < cnt; e += n) syrk_tile<SLD>(S, i0, r0 + 8 * e, m0, lane);
         e -= cnt;
-    }
-}
-
-// One merge of the block inverse: with inv(A) (rows and columns J0 .. J0 + H) and inv(D)
-// (I0 .. I0 + H, I0 = J0 + H) in place, the off-diagonal block of inv([A 0; C D]) is
-// X = -inv(D) (C inv(A)). merge_t computes tile q of T = C inv(A), merge_x tile q of X (16 x 8
-// tiles, down the columns); both skip the zero blocks of the triangular operand and select
-// within its diagonal blocks.
-template <int H>
-__device__ __forceinline__ void merge_t(const double* S, double* T, int J0, int q, int lane) {
-    constexpr int TD = H + 4, ROWS = H / 16;
-    const int ti = 16 * (q % ROWS), tc = 8 * (q / ROWS);
-    const int g = lane >> 2, t = lane & 3, c = tc + g;
-    const double *a = S + (J0 + H + ti + g) * SLD + J0 + t, *v = S + (J0 + c) * SLD + J0 + t;  // v: inv(A)(k, c)
-    double d[4] = {};
-#pragma unroll
-    for (int k = 0; k < 8; k += 4)
-        dmma_16x8x4(d, a[tc + k], a[8 * SLD + tc + k], tc + k + t >= c ? v[tc + k] : 0.0);
-#pragma unroll 4
-    for (int k = tc + 8; k < H; k += 4) dmma_16x8x4(d, a[k], a[8 * SLD + k], v[k]);
-    *reinterpret_cast<double2*>(T + (ti + g) * TD + tc + 2 * t) = make_double2(d[0], d[1]);
-    *reinterpret_cast<double2*>(T + (ti + g + 8) * TD + tc + 2 * t) = make_double2(d[2], d[3]);
-}
-template <int H>
-__device__ __forceinline__ void merge_x(double* S, const double* T, int J0, int xi, int xc, int lane) {
-    constexpr int TD = H + 4;
-    const int I0 = J0 + H, g = lane >> 2, t = lane & 3, i = xi + g;
-    const double *a = S + (I0 + t) * SLD + I0 + i, *b = T + t * TD + xc + g;  // a: inv(D)(i, k)
-    double d[4] = {};
-#pragma unroll 4
-    for (int k = 0; k < xi; k += 4) dmma_16x8x4(d, a[k * SLD], a[k * SLD + 8], b[k * TD]);
-#pragma unroll
-    for (int k = 0; k < 16; k += 4) {
-        const int kk = xi + k;
-        dmma_16x8x4(d, k + t <= g ? a[kk * SLD] : 0.0, k + t <= g + 8 ? a[kk * SLD + 8] : 0.0, b[kk * TD]);
-    }
-    double* x = S + (J0 + xc + 2 * t) * SLD + I0 + i;  // X(i, c), transposed
-    x[0] = -d[0];
-    x[SLD] = -d[1];
-    x[8] = -d[2];
-    x[SLD + 8] = -d[3];
-}
-
-// x solved with the 16-block L, each lane its own x: x[m] /= L(m, m), x[q] -= L(q, m) x[m].
-// Columns of L in Lt, reciprocal diagonal in rd; wait(h) is called before the first use of
-// columns 8 h .. 8 h + 7. With x a unit vector this is a column of inv(L), with x a row of the
-// panel below L that row of the panel solve.
-template <class Wait>
-__device__ __forceinline__ void solve_sub_block(double (&x)[DB], const double* rd, const double* Lt, Wait wait) {
-#pragma unroll
-    for (int m = 0; m < DB; ++m) {
-        if (m % 8 == 0) wait(m / 8);
-        x[m] *= rd[m];
-        const double2* pair = reinterpret_cast<const double2*>(Lt + m * LTD);
-#pragma unroll
-        for (int q = (m + 1) & ~1; q < DB; q += 2) {
-            const double2 v = pair[q / 2];
-            if (q > m) x[q] = fma(-v.x, x[m], x[q]);
-            x[q + 1] = fma(-v.y, x[m], x[q + 1]);
-        }
     }
 }
 
@@ -232,17 +148,6 @@ __device__ __forceinline__ void store_block(const View<T>& A, int sz, bool rowma
     }
 }
 
-// 1 / sqrt(d) for a normal d > 0: the hardware approximation (relative error e below 2^-20)
-// and one step of the third-order series of (1 - e)^(-1/2). Straight-line code, so that the
-// rank-1 update of the column before is scheduled into its latency; for a subnormal d the
-// approximation is infinite and the caller starts over with rsqrt().
-__device__ __forceinline__ double rsqrt_normal(double d) {
-    double r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-(d * r), r, 1.0);
-    return fma(r * e, fma(e, fma(e, 0.3125, 0.375), 0.5), r);
-}
-
 // Named barriers of potrf_diag: kBarChunk + h says that columns 8 h .. 8 h + 7 of the
 // sub-block being factored are in Lt and rd (warp 0 arrives, their readers wait).
 constexpr int kBarBackground = 1, kBarChunk = 2;
@@ -251,82 +156,6 @@ __device__ __forceinline__ void named_sync(int id, int threads) {
 }
 __device__ __forceinline__ void named_arrive(int id, int threads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// Right-looking factorisation of 16 columns of 32 rows by one warp, row `lane` in a (the
-// 16 x 16 block to factor and the 16 rows below it): a becomes L's row, column j of L goes to
-// Lt + j * LTD, L(j, j) to ld and its reciprocal to rd; every 8 columns it arrives at the chunk
-// barriers (`threads` participants). flags[0] = 1 + column of the first non-positive (or NaN)
-// pivot, 0 if there is none; after one the values are void. flags[1] = 1 where a pivot is too
-// small for rsqrt_normal, and the result is void.
-__device__ __forceinline__ void factor_sub_block(double (&a)[DB], double* Lt, double* ld, double* rd, int lane,
-                                                 int threads, volatile int* flags) {
-    int bad = 0;
-    bool tiny = false;
-    auto pivot = [&](double own, int j) {
-        const double d = __shfl_sync(0xffffffffu, own, j);
-        if (!(d > 0.0) && bad == 0) bad = j + 1;
-        tiny |= d < 1e-300;
-        return d;
-    };
-    double d = pivot(a[0], 0), r = rsqrt_normal(d);
-#pragma unroll
-    for (int j = 0; j < DB; ++j) {
-        const double l = lane == j ? d * r : a[j] * r;  // L(i, j); above the diagonal, unused
-        a[j] = l;
-        if (lane == j) {
-            rd[j] = r;
-            ld[j] = l;
-        }
-        double* colj = Lt + j * LTD;
-        colj[lane] = l;
-        if (j + 1 < DB) {
-            d = pivot(fma(-l, l, a[j + 1]), j + 1);  // row j + 1's own update of its diagonal
-            r = rsqrt_normal(d);
-        } else if (lane == 0) {
-            flags[0] = bad;
-            flags[1] = tiny && bad == 0;
-        }
-        __syncwarp();
-        if (j % 8 == 7) named_arrive(kBarChunk + j / 8, threads);
-        const double2* pair = reinterpret_cast<const double2*>(colj);
-#pragma unroll
-        for (int c = (j + 1) & ~1; c < DB; c += 2) {
-            const double2 v = pair[c / 2];
-            if (c > j) a[c] = fma(-l, v.x, a[c]);
-            a[c + 1] = fma(-l, v.y, a[c + 1]);
-        }
-    }
-}
-
-// The same for pivots of any size, on the rows in shared memory (row: this lane's) and with the
-// library's rsqrt: the way out for values next to underflow.
-__device__ __noinline__ void factor_sub_block_any(double* row, bool own, double* Lt, double* ld, double* rd, int lane,
-                                                  int threads, volatile int* flags) {
-    int bad = 0;
-#pragma unroll 1
-    for (int j = 0; j < DB; ++j) {
-        double d = __shfl_sync(0xffffffffu, own ? row[j] : 0.0, j);
-        if (!(d > 0.0)) {
-            if (bad == 0) bad = j + 1;
-            d = 1.0;
-        }
-        const double r = rsqrt(d), l = lane == j ? d * r : own ? row[j] * r : 0.0;
-        if (lane == j) {
-            rd[j] = r;
-            ld[j] = l;
-        }
-        if (own && lane > j) row[j] = l;
-        Lt[j * LTD + lane] = l;
-        if (j + 1 == DB && lane == 0) {
-            flags[0] = bad;
-            flags[1] = 0;
-        }
-        __syncwarp();
-        if (j % 8 == 7) named_arrive(kBarChunk + j / 8, threads);
-        if (own)
-            for (int c = j + 1; c < DB && c <= lane; ++c) row[c] = fma(-l, Lt[j * LTD + c], row[c]);
-    }
 }
 
 // One CTA per diagonal block: W_b = inverse of the lower-triangular block b of L. The 16-blocks
@@ -378,18 +207,18 @@ __global__ void __launch_bounds__(kDiagThreads, 1) trtri_blocks(int64_t m, View<
     __syncthreads();
     // four 16-merges (scratch: T16 and, for the others, T64), two 32-merges, the 64-merge
     double* Tq = warp < 2 ? T16 : T64 + (warp >> 1) * 16 * 20;
-    if (warp < 8) merge_t<16>(S, Tq, 32 * (warp >> 1), warp & 1, lane);
+    if (warp < 8) merge_t<16, SLD>(S, Tq, 32 * (warp >> 1), warp & 1, lane);
     __syncthreads();
-    if (warp < 8) merge_x<16>(S, Tq, 32 * (warp >> 1), 0, 8 * (warp & 1), lane);
+    if (warp < 8) merge_x<16, SLD>(S, Tq, 32 * (warp >> 1), 0, 8 * (warp & 1), lane);
     __syncthreads();
     Tq = warp < 8 ? T32 : T64;
-    merge_t<32>(S, Tq, 64 * (warp >> 3), warp & 7, lane);
+    merge_t<32, SLD>(S, Tq, 64 * (warp >> 3), warp & 7, lane);
     __syncthreads();
-    merge_x<32>(S, Tq, 64 * (warp >> 3), 16 * (warp & 1), 8 * ((warp & 7) >> 1), lane);
+    merge_x<32, SLD>(S, Tq, 64 * (warp >> 3), 16 * (warp & 1), 8 * ((warp & 7) >> 1), lane);
     __syncthreads();
-    for (int q = warp; q < 32; q += 16) merge_t<64>(S, T64, 0, q, lane);
+    for (int q = warp; q < 32; q += 16) merge_t<64, SLD>(S, T64, 0, q, lane);
     __syncthreads();
-    for (int q = warp; q < 32; q += 16) merge_x<64>(S, T64, 0, 16 * (q & 3), 8 * (q >> 2), lane);
+    for (int q = warp; q < 32; q += 16) merge_x<64, SLD>(S, T64, 0, 16 * (q & 3), 8 * (q >> 2), lane);
     __syncthreads();
     for (int q = warp; q < 20; q += 16) store_inverse(S, Wb, false, q >> 1, q & 1, lane);
 }
@@ -453,6 +282,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
         for (int kb = 0; kb < NSUB; ++kb) {
             const int c0 = DB * kb;
             double* row = S + (c0 + lane) * SLD + c0;
+            auto arrive = [&](int h) { named_arrive(kBarChunk + h, participants(kb)); };
             double x[DB];
 #pragma unroll
             for (int c = 0; c < DB; c += 2) {
@@ -460,7 +290,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
                 x[c] = v.x;
                 x[c + 1] = v.y;
             }
-            factor_sub_block(x, Lt, ld + c0, rd + c0, lane, participants(kb), flags);
+            factor_sub_block(x, Lt, ld + c0, rd + c0, lane, flags, arrive);
             __syncwarp();
             if (!flags[1] && c0 + lane < NB) {
 #pragma unroll
@@ -468,7 +298,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
                     if (q < lane) row[q] = x[q];
             }
             if (redo()) {
-                factor_sub_block_any(row, c0 + lane < NB, Lt, ld + c0, rd + c0, lane, participants(kb), flags);
+                factor_sub_block_any(row, c0 + lane < NB, Lt, ld + c0, rd + c0, lane, flags, arrive);
                 redo();
             }
             if (flags[0]) {
@@ -521,23 +351,23 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
             // panel kb - 1's update right of this panel: rows and columns from c0 + 16
             if (kb > 0) syrk_tiles(S, c0 + DB, NB, c0 - DB, bg, nbg, lane);
             if (kb == 2 || kb == 4 || kb == 6) {  // the 32-block before this sub-block
-                if (bg < 2) merge_t<16>(S, T16, c0 - 32, bg, lane);
+                if (bg < 2) merge_t<16, SLD>(S, T16, c0 - 32, bg, lane);
                 named_sync(kBarBackground, 32 * nbg);
-                if (bg < 2) merge_x<16>(S, T16, c0 - 32, 0, 8 * bg, lane);
+                if (bg < 2) merge_x<16, SLD>(S, T16, c0 - 32, 0, 8 * bg, lane);
                 if (kb == 4) {
                     named_sync(kBarBackground, 32 * nbg);
-                    merge_x<32>(S, T32, 0, 16 * (bg & 1), 8 * (bg >> 1), lane);
+                    merge_x<32, SLD>(S, T32, 0, 16 * (bg & 1), 8 * (bg >> 1), lane);
                 }
             } else if (kb == 3 || kb == 7) {
-                merge_t<32>(S, T32, kb == 3 ? 0 : 64, bg, lane);
+                merge_t<32, SLD>(S, T32, kb == 3 ? 0 : 64, bg, lane);
                 if (kb == 7) {
-                    if (bg < 2) merge_t<16>(S, T16, 96, bg, lane);
+                    if (bg < 2) merge_t<16, SLD>(S, T16, 96, bg, lane);
                     // rows 64 .. 95 of the 64-merge need no part of the last 32 rows
-                    for (int q = bg; q < 16; q += nbg) merge_x<64>(S, T64, 0, 16 * (q & 1), 8 * (q >> 1), lane);
+                    for (int q = bg; q < 16; q += nbg) merge_x<64, SLD>(S, T64, 0, 16 * (q & 1), 8 * (q >> 1), lane);
                 }
             }
             if (kb == 5 || kb == 6)  // T of the 64-merge, half of its columns each
-                for (int q = bg; q < 16; q += nbg) merge_t<64>(S, T64, 0, 16 * (kb - 5) + q, lane);
+                for (int q = bg; q < 16; q += nbg) merge_t<64, SLD>(S, T64, 0, 16 * (kb - 5) + q, lane);
             while (redo()) {}
             if (flags[0]) return;
             next_panel(c0);
@@ -556,12 +386,12 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
     // What depends on the last sub-blocks: the last 16-, the last 32-merge and the lower half
     // of the 64-merge (warps 0-7); meanwhile L goes back to global memory.
     if (warp < 8) {
-        if (warp < 2) merge_x<16>(S, T16, 96, 0, 8 * warp, lane);
+        if (warp < 2) merge_x<16, SLD>(S, T16, 96, 0, 8 * warp, lane);
         named_sync(kBarBackground, 256);
-        merge_x<32>(S, T32, 64, 16 * (warp & 1), 8 * (warp >> 1), lane);
+        merge_x<32, SLD>(S, T32, 64, 16 * (warp & 1), 8 * (warp >> 1), lane);
         named_sync(kBarBackground, 256);
-        merge_x<64>(S, T64, 0, 32, 8 * warp, lane);
-        merge_x<64>(S, T64, 0, 48, 8 * warp, lane);
+        merge_x<64, SLD>(S, T64, 0, 32, 8 * warp, lane);
+        merge_x<64, SLD>(S, T64, 0, 48, 8 * warp, lane);
     } else {
         for (int q = warp - 8; q < 20; q += 8) store_block(A, sz, rowmaj, q >> 1, q & 1, S, ld, lane);
     }
