@@ -644,7 +644,10 @@ template <bool AK, bool BK>
 int sgemm(int64_t m, int64_t n, int64_t k, float alpha, View<const float> A, View<const float> B, float beta,
           View<float> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
     const Shape p{m, n, k, mask};
-    if (simt_cycles<SimtL>(p, 0.78, 1900.0) <= simt_cycles<SimtS>(p, 0.40, 800.0))
+    // A product that writes over one of its own operands (C on B with m <= 128, on A with n <= 64)
+    // takes the tile that spans that operand's rows or columns, as in pick_tile.
+    const bool in_place = C.p == A.p || C.p == B.p;
+    if (in_place || simt_cycles<SimtL>(p, 0.78, 1900.0) <= simt_cycles<SimtS>(p, 0.40, 800.0))
         return launch_sgemm<AK, BK, SimtL>(p, alpha, A, B, beta, C, off, s, abort);
     return launch_sgemm<AK, BK, SimtS>(p, alpha, A, B, beta, C, off, s, abort);
 }

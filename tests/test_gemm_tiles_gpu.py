@@ -54,3 +54,15 @@ def test_syrk_tiles_exact(cuda, n, k, upper, shift, dtype):
     full = C - A @ A.T
     want = np.triu(full) + np.tril(C, -1) if upper else np.tril(full) + np.triu(C, 1)
     assert np.array_equal(Cd.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("n", [5, 33, 64, 500])
+def test_gemm_in_place_left(cuda, n, dtype):
+    """B <- L B over its own operand with 64 rows, as the factorisations' block rows do: no tile
+    may overwrite rows that another one still reads."""
+    rs = np.random.default_rng(n)
+    L, B = rs.integers(-4, 5, (64, 64)).astype(np.float64), rs.integers(-4, 5, (64, n)).astype(np.float64)
+    Ld, Bd = _dev(L, True, 0, dtype), _dev(B, False, 0, dtype)
+    ops.gemm(Ld, Bd, Bd, 1.0, 0.0)
+    assert np.array_equal(Bd.cpu().numpy(), L @ B)
