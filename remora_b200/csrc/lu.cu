@@ -2,7 +2,8 @@
 // any strided view of the logical n x n matrix.
 //
 // getrf (kernels/getrf.hpp:50-59; CPU algorithm kernels/default/getrf.hpp:41-181):
-// blocked right-looking LU with 64-column panels. One CTA factors a panel column by
+// blocked right-looking LU with 64-column panels. A panel (of up to 4096 rows on one
+// thread-block cluster, beyond that on a cooperative grid or one CTA) is factored column by
 // column -- pivot = the row of largest |A(i, j)| at or below the diagonal (the lowest
 // row among equals, as the reference's strictly-larger scan), the swap of the two rows
 // across the panel, the division of the column by the pivot (in double, as the
@@ -22,11 +23,18 @@
 // and the row right of the diagonal is cleared. After the block the whole trailing square
 // (both triangles, which later swaps read) is updated by a DMMA GEMM with the block's
 // columns. piv as for getrf (identity where no swap happened); the rank goes to *rank.
+#include <cooperative_groups.h>
+
+#include <atomic>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 
+#include "diag.cuh"
 #include "factor.cuh"
 #include "gemm.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace rc {
 namespace {
@@ -88,7 +96,7 @@ __global__ void __launch_bounds__(kLuThreads) getrf_panel_kernel(int64_t n, View
             }
         }
         block_argmax(best, bi, sv, si);
-        const int64_t p = bi;
+        const int64_t p = bi == INT64_MAX ? c : bi;  // nothing but NaN: the row itself
         const double pv = (double)A(p, c);
         if (pv == 0.0) {  // also all-zero columns: the first row is the pivot, value 0
             if (threadIdx.x == 0) {
@@ -246,9 +254,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
             }
         }
         block_argmax(best, bi, sv, si);
-        const int64_t p = bi;
+        const int64_t p = bi == INT64_MAX ? c : bi;  // nothing but NaN: the row itself
         const int owner = (int)((p - k0) / chunk);
-        const double* pr = sc.cand_row + ((size_t)j * G + owner) * nb;
+        const double* pr = bi == INT64_MAX ? sc.crow + (size_t)j * nb : sc.cand_row + ((size_t)j * G + owner) * nb;
         for (int col = threadIdx.x; col < nb; col += kCoopThreads) prow[col] = __ldcg(pr + col);
         __syncthreads();
         const double pv = prow[j];
@@ -328,21 +336,425 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     }
 }
 
-// The row swaps piv[k0 .. k0 + nb) in order, on the columns outside the panel.
+// The panel factorisation on one thread-block cluster: CTA r of the G (a power of two, at most
+// 16) holds rows [k0 + 256 r, k0 + 256 (r + 1)) of the panel, a thread per row, in shared memory
+// P (row stride kClLd). The panel is walked in 16-column strips, whose rows are in registers,
+// rotated so that a[0] is the column to eliminate. Per column every CTA sends its candidate
+// (largest |a[0]|, the lowest row among equals) and that row into every CTA's shared memory by
+// st.async and waits for theirs on its own mbarrier (two in turn, by the column's parity: what is
+// sent for a column is sent after its sender has read all of the column before last); then all
+// agree on the pivot, the two rows swap within the strip, and every row is divided and updated. Per strip, the swaps of the panel's other columns
+// (and of the strip's own finished ones) are gathered through distributed shared memory, the
+// strip's 16 rows of U are solved, and the columns to the right are updated on DMMA. Each element
+// sees the pivot, division and update order of getrf_panel_kernel, a strip's sixteen products
+// summed before they are subtracted.
+// Bound by latency: of a column's ~2400 cycles (8 CTAs) the two-level search for the candidate
+// takes ~1000, sending and waiting ~600 (cluster barriers instead: 860, with 16 CTAs 1400
+// instead of 720), the agreed pivot, the division and the update ~700. 2048 x 64: 104 us (385 on
+// the cooperative grid, whose columns cost a grid barrier and two round trips through L2).
+constexpr int kClThreads = 256, kStrip = 16, kClLd = kLuNB + 4, kClMax = 16;
+
 template <class T>
-__global__ void lu_swap_kernel(int64_t n, View<T> A, int64_t k0, int nb, const int* piv, const int* info) {
-    if (*(volatile const int*)info != 0) return;
-    for (int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; col < n - nb;
-         col += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t cc = col < k0 ? col : col + nb;
-        for (int j = 0; j < nb; ++j) {
-            const int64_t r = k0 + j, p = piv[r];
-            if (p != r) {
-                const T t = A(r, cc);
-                A(r, cc) = A(p, cc);
-                A(p, cc) = t;
+struct ClusterSmem {
+    T P[kClThreads * kClLd];
+    T cand_row[2][kClMax][kStrip];  // by column parity and CTA
+    T crow[2][kStrip];              // row c before the swap
+    uint64_t cand_key[2][kClMax][2];  // (hi, lo) of |a[0]|; the row
+    uint64_t bar[2];
+    int late;                       // a wait ran out
+    int from_all[2 * kStrip], from_strip[2 * kStrip][kStrip], dest[2 * kStrip];
+    T mine[8][kStrip], top[kStrip];  // the warps' candidate rows; row c
+    T U[kStrip][kLuNB];
+    unsigned whi[8], wlo[8];
+    int widx[8];
+    int pivots[kStrip];
+    // the inverse of L11 (read and written in pairs)
+    alignas(16) double L[kLuNB * kClLd];
+    alignas(16) double Lt[4][kDB * kLTD];
+    alignas(16) double T16[2][16 * 20];
+    alignas(16) double T32[32 * 36];
+    double rd[kLuNB];
+};
+
+// Largest (hi, lo), the smallest idx among equals, over a warp; lanes without a candidate have
+// hi = 0 and idx = INT_MAX.
+__device__ __forceinline__ void warp_best(unsigned& hi, unsigned& lo, int& idx) {
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi), at = __ballot_sync(0xffffffffu, hi == mh);
+    if ((at & (at - 1)) == 0) {  // one lane has it
+        const int src = __ffs((int)at) - 1;
+        lo = __shfl_sync(0xffffffffu, lo, src);
+        idx = __shfl_sync(0xffffffffu, idx, src);
+        hi = mh;
+        return;
+    }
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    idx = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? idx : INT_MAX);
+    hi = mh;
+    lo = ml;
+}
+
+__device__ __forceinline__ uint32_t peer_address(const void* p, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void send(uint32_t to, uint64_t v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to), "l"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send(uint32_t to, double v, uint32_t bar) {
+    send(to, (uint64_t)__double_as_longlong(v), bar);
+}
+__device__ __forceinline__ void send(uint32_t to, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(to),
+                 "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
+}
+// Whether phase `parity` of the mbarrier completed within `limit` cycles.
+__device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity, long long limit) {
+    const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+    const long long t0 = clock64();
+    while (true) {
+        uint32_t ok;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(b), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (clock64() - t0 > limit) return false;
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kClThreads, 1)
+    getrf_panel_cluster_kernel(int64_t n, View<T> A, int64_t k0, int nb, int* piv, int* info, T* linv, int* err,
+                               uint64_t limit_ns) {
+    extern __shared__ __align__(16) unsigned char cl_smem[];
+    ClusterSmem<T>& sm = *reinterpret_cast<ClusterSmem<T>*>(cl_smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int G = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (*(volatile int*)info != 0) return;  // the same for the whole cluster
+    const int m = (int)(n - k0);             // rows of the panel; rows are numbered from k0 here
+    const int base = rank * kClThreads, row = base + tid;
+    const long long limit = (long long)(limit_ns * 2u);
+    if (tid == 0) {
+        for (int q = 0; q < 2; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&sm.bar[q])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sm.late = 0;
+    }
+    T* const prow_mem = sm.P + tid * kClLd;
+    if (A.cs == 1) {  // rows contiguous: lanes along the columns
+        for (int r = warp; r < kClThreads; r += 8)
+            for (int col = lane; col < kLuNB; col += 32)
+                sm.P[r * kClLd + col] = base + r < m && col < nb ? A(k0 + base + r, k0 + col) : T(0);
+    } else {
+#pragma unroll 32
+        for (int col = 0; col < kLuNB; ++col) prow_mem[col] = row < m && col < nb ? A(k0 + row, k0 + col) : T(0);
+    }
+    cluster.sync();  // every CTA runs before any writes to another's shared memory
+    const unsigned bytes = (unsigned)(G * (kStrip * sizeof(T) + 16) + kStrip * sizeof(T));  // sent to a CTA per column
+    unsigned turn = 0;                                                                     // columns so far
+    for (int j0 = 0; j0 < nb; j0 += kStrip) {
+        const int w = nb - j0 < kStrip ? nb - j0 : kStrip;
+        T a[kStrip];
+        {
+            const T* src = prow_mem + j0;
+#pragma unroll
+            for (int q = 0; q < kStrip; ++q) a[q] = src[q];
+        }
+#pragma unroll 1
+        for (int jj = 0; jj < w; ++jj, ++turn) {
+            const int c = j0 + jj, par = turn & 1;
+            if (tid == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&sm.bar[par])),
+                             "r"(bytes)
+                             : "memory");
+            // the CTA's candidate
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs((double)a[0]));
+            const bool valid = row >= c && row < m && bits <= 0x7ff0000000000000ull;  // not NaN
+            unsigned hi = valid ? (unsigned)(bits >> 32) + 1u : 0u, lo = valid ? (unsigned)bits : 0u;
+            int idx = valid ? row : INT_MAX;
+            warp_best(hi, lo, idx);
+            if (lane == 0) {
+                sm.whi[warp] = hi;
+                sm.wlo[warp] = lo;
+                sm.widx[warp] = idx;
+            }
+            if (row == idx) {
+#pragma unroll
+                for (int q = 0; q < kStrip; ++q) sm.mine[warp][q] = a[q];
+            }
+            if (row == c) {
+#pragma unroll
+                for (int q = 0; q < kStrip; ++q) sm.top[q] = a[q];
+            }
+            __syncthreads();
+            hi = lane < 8 ? sm.whi[lane] : 0u;
+            lo = lane < 8 ? sm.wlo[lane] : 0u;
+            idx = lane < 8 ? sm.widx[lane] : INT_MAX;
+            warp_best(hi, lo, idx);
+            const int from_warp = idx == INT_MAX ? 0 : (idx - base) >> 5;
+            {  // thread (dest, e) sends element e to CTA dest
+                const int dest = tid / kStrip, e = tid % kStrip;
+                if (dest < G) {
+                    const uint32_t bar = peer_address(&sm.bar[par], dest);
+                    send(peer_address(&sm.cand_row[par][rank][e], dest), sm.mine[from_warp][e], bar);
+                    if (rank == 0) send(peer_address(&sm.crow[par][e], dest), sm.top[e], bar);
+                    if (e == 0) send(peer_address(&sm.cand_key[par][rank][0], dest), (uint64_t)hi << 32 | lo, bar);
+                    if (e == 1) send(peer_address(&sm.cand_key[par][rank][1], dest), (uint64_t)idx, bar);
+                }
+            }
+            if (!wait_phase(&sm.bar[par], turn >> 1 & 1, limit)) sm.late = 1;
+            hi = lane < G ? (unsigned)(sm.cand_key[par][lane][0] >> 32) : 0u;
+            lo = lane < G ? (unsigned)sm.cand_key[par][lane][0] : 0u;
+            idx = lane < G ? (int)sm.cand_key[par][lane][1] : INT_MAX;
+            warp_best(hi, lo, idx);
+            if (idx != INT_MAX && (idx < c || idx >= m)) idx = INT_MAX;  // after a late wait only
+            const int p = idx == INT_MAX ? c : idx;  // nothing but NaN: the row itself
+            const T* pr = idx == INT_MAX ? sm.crow[par] : sm.cand_row[par][p / kClThreads];
+            const double pv = (double)pr[0];
+            if (pv == 0.0) {  // also all-zero columns: the first row is the pivot, value 0
+                if (rank == 0 && tid == 0) {
+                    piv[k0 + c] = (int)(k0 + c);
+                    record_first(info, (int)(k0 + c + 1));
+                }
+                if (sm.late && err && atomicCAS(err, 0, RC_ERR_TIMEOUT) == 0) atomicExch(err + 1, 501);
+                cluster.sync();
+                return;  // the whole cluster
+            }
+            if (tid == 0) {
+                sm.pivots[jj] = p;
+                if (rank == 0) piv[k0 + c] = (int)(k0 + p);
+            }
+            if (row == p || row == c) {
+                const T* from = row == p ? sm.crow[par] : pr;
+#pragma unroll
+                for (int q = 0; q < kStrip; ++q) a[q] = from[q];
+            }
+            T l = a[0];
+            if (row > c) {
+                l = (T)((double)a[0] / pv);
+#pragma unroll
+                for (int q = 1; q < kStrip; ++q) a[q] -= l * pr[q];
+            }
+            // column c is final but for the strip's later swaps; the next one moves to a[0]
+            prow_mem[c] = l;
+#pragma unroll
+            for (int q = 0; q + 1 < kStrip; ++q) a[q] = a[q + 1];
+            // (columns past the strip's width rotate in: never a[0], their updates unused)
+            if (row == c) {  // U's row right of the diagonal, kept as the rotation leaves it
+#pragma unroll
+                for (int q = 0; q + 1 < kStrip; ++q)
+                    if (jj + 1 + q < w) prow_mem[c + 1 + q] = a[q];
             }
         }
+        cluster.sync();  // P's strip and the pivots are final everywhere
+        // The swaps of the other columns, and of the strip's own columns by the later pivots
+        // (entries right of a row's diagonal were swapped in registers): destination rows are
+        // j0 .. j0 + w and the pivots beyond them; each traces its content back through the swaps.
+        {
+            int pv[kStrip];
+#pragma unroll
+            for (int i = 0; i < kStrip; ++i) pv[i] = i < w ? sm.pivots[i] : -1;
+            for (int e = tid; e < 2 * kStrip * kStrip; e += kClThreads) {
+                const int d = e % (2 * kStrip), j = e / (2 * kStrip);
+                int r = d < w ? j0 + d : -1;
+                if (d >= kStrip) {
+                    r = d - kStrip < w ? sm.pivots[d - kStrip] : -1;
+                    if (r < j0 + w) r = -1;
+#pragma unroll
+                    for (int i = 0; i < kStrip; ++i)
+                        if (i < d - kStrip && pv[i] == r) r = -1;
+                }
+                int from = r, from_j = r;
+#pragma unroll
+                for (int i = kStrip - 1; i >= 0; --i) {
+                    if (i == j) from_j = from;  // column j takes the swaps after its own
+                    if (i < w) from = from == j0 + i ? pv[i] : from == pv[i] ? j0 + i : from;
+                }
+                sm.from_strip[d][j] = r >= j0 && r < j0 + j ? r : from_j;  // U's rows are final
+                if (j == 0) {
+                    sm.from_all[d] = from;
+                    sm.dest[d] = r;
+                }
+            }
+        }
+        __syncthreads();
+        T moved[4][2];
+        int dst[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int d = warp + 8 * q, r = sm.dest[d];
+            dst[q] = r >= 0 && r / kClThreads == rank ? r : -1;
+            if (dst[q] < 0) continue;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = lane + 32 * h;
+                const int from = col >= j0 && col < j0 + w ? sm.from_strip[d][col - j0] : sm.from_all[d];
+                const ClusterSmem<T>* peer = cluster.map_shared_rank(&sm, from / kClThreads);
+                moved[q][h] = peer->P[(from % kClThreads) * kClLd + col];
+            }
+        }
+        cluster.sync();  // all gathered
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (dst[q] >= 0)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) sm.P[(dst[q] - base) * kClLd + lane + 32 * h] = moved[q][h];
+        __syncthreads();
+        const int j1 = j0 + w, right = nb - j1;
+        if (right <= 0) break;
+        // U(strip, right) = inv(L11) A(strip, right), a thread per column
+        if (rank == 0 && tid < right) {
+            T u[kStrip];
+            T* col = sm.P + j0 * kClLd + j1 + tid;
+            const T* l11 = sm.P + j0 * kClLd + j0;
+#pragma unroll
+            for (int i = 0; i < kStrip; ++i) u[i] = col[i * kClLd];
+#pragma unroll
+            for (int k = 0; k < kStrip; ++k)
+#pragma unroll
+                for (int i = k + 1; i < kStrip; ++i) u[i] -= l11[i * kClLd + k] * u[k];
+#pragma unroll
+            for (int i = 0; i < kStrip; ++i) col[i * kClLd] = sm.U[i][tid] = u[i];
+        }
+        cluster.sync();
+        if (rank != 0) {
+            const ClusterSmem<T>* first = cluster.map_shared_rank(&sm, 0);
+            for (int e = tid; e < kStrip * right; e += kClThreads) sm.U[e / right][e % right] = first->U[e / right][e % right];
+            __syncthreads();
+        }
+        // P(:, right) -= L(:, strip) U on the rows below the strip: 16 x 8 tiles
+        const int g = lane >> 2, t = lane & 3;
+        for (int ti = warp; ti < kClThreads / 16; ti += 8) {
+            if (base + 16 * ti < j1) continue;
+            const T* l0 = sm.P + (16 * ti + g) * kClLd + j0 + t;
+            double lf[4][2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                lf[k][0] = (double)l0[4 * k];
+                lf[k][1] = (double)l0[8 * kClLd + 4 * k];
+            }
+            for (int tj = 0; tj < right; tj += 8) {
+                double d[4] = {};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) dmma_16x8x4(d, lf[k][0], lf[k][1], (double)sm.U[4 * k + t][tj + g]);
+                T* x = sm.P + (16 * ti + g) * kClLd + j1 + tj + 2 * t;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    T& v = x[(e >> 1) * 8 * kClLd + (e & 1)];
+                    if (tj + 2 * t + (e & 1) < right) v = (T)((double)v - d[e]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    cluster.sync();  // no CTA leaves while its shared memory may be read
+    if (tid == 0 && sm.late && err && atomicCAS(err, 0, RC_ERR_TIMEOUT) == 0) atomicExch(err + 1, 501);
+    if (A.cs == 1) {
+        for (int r = warp; r < kClThreads; r += 8)
+            for (int col = lane; col < nb; col += 32)
+                if (base + r < m) A(k0 + base + r, k0 + col) = sm.P[r * kClLd + col];
+    } else if (row < m) {
+#pragma unroll 32
+        for (int col = 0; col < kLuNB; ++col)
+            if (col < nb) A(k0 + row, k0 + col) = prow_mem[col];
+    }
+    if (rank != 0) return;
+    // inv(L11), unit lower (the identity beyond nb), for U12 = inv(L11) A12 right of the panel:
+    // 16-blocks by a warp each, then merges (diag.cuh)
+#pragma unroll 8
+    for (int e = tid; e < kLuNB * kLuNB; e += kClThreads) {
+        const int i = e / kLuNB, j = e % kLuNB;
+        if (j <= i) sm.L[i * kClLd + j] = i == j ? 1.0 : i < nb ? (double)sm.P[i * kClLd + j] : 0.0;
+    }
+    if (tid < kLuNB) sm.rd[tid] = 1.0;
+    __syncthreads();
+    if (warp < 4) {
+        const int c0 = kDB * warp;
+        double* Lt = sm.Lt[warp];
+        if (lane < kDB)
+#pragma unroll
+            for (int p = 0; p < kDB; ++p) Lt[p * kLTD + lane] = sm.L[(c0 + lane) * kClLd + c0 + p];
+        __syncwarp();
+        double x[kDB];
+#pragma unroll
+        for (int q = 0; q < kDB; ++q) x[q] = q == lane ? 1.0 : 0.0;
+        solve_sub_block(x, sm.rd, Lt, [](int) {});
+        if (lane < kDB)
+#pragma unroll
+            for (int q = 0; q < kDB; ++q)
+                if (q >= lane) sm.L[(c0 + lane) * kClLd + c0 + q] = x[q];
+    }
+    __syncthreads();
+    if (warp < 4) merge_t<16, kClLd>(sm.L, sm.T16[warp >> 1], 32 * (warp >> 1), warp & 1, lane);
+    __syncthreads();
+    if (warp < 4) merge_x<16, kClLd>(sm.L, sm.T16[warp >> 1], 32 * (warp >> 1), 0, 8 * (warp & 1), lane);
+    __syncthreads();
+    merge_t<32, kClLd>(sm.L, sm.T32, 0, warp, lane);
+    __syncthreads();
+    merge_x<32, kClLd>(sm.L, sm.T32, 0, 16 * (warp & 1), 8 * (warp >> 1), lane);
+    __syncthreads();
+#pragma unroll 8
+    for (int e = tid; e < kLuNB * kLuNB; e += kClThreads) {  // (only used when nb == kLuNB)
+        const int i = e / kLuNB, j = e % kLuNB;
+        linv[e] = i >= j ? (T)sm.L[j * kClLd + i] : T(0);
+    }
+}
+
+// The row swaps piv[k0 .. k0 + nb) on the columns outside the panel, 32 columns a CTA. The rows
+// they touch (the panel's nb and the pivots beyond them) trace their content back through the
+// swaps, a thread per row; then all of it is gathered into shared memory and written back.
+// 64 swaps on 1984 columns of a column-major matrix: 14 us (49 with a thread per column that makes
+// them one after the other).
+constexpr int kSwapCols = 32;
+template <class T>
+__global__ void __launch_bounds__(256) lu_swap_kernel(int64_t n, View<T> A, int64_t k0, int nb, const int* piv,
+                                                      const int* info) {
+    __shared__ int64_t src[2 * kLuNB], dst[2 * kLuNB];
+    __shared__ int64_t p[kLuNB];
+    __shared__ T tile[2 * kLuNB][kSwapCols + 1];
+    if (*(volatile const int*)info != 0) return;
+    const int tid = threadIdx.x;
+    if (tid < nb) p[tid] = piv[k0 + tid];
+    __syncthreads();
+    if (tid < 2 * kLuNB) {
+        int64_t r = -1;
+        if (tid < nb) r = k0 + tid;
+        else if (tid >= kLuNB && tid - kLuNB < nb) {
+            r = p[tid - kLuNB];
+            if (r < k0 + nb) r = -1;
+#pragma unroll 16
+            for (int i = 0; i < kLuNB; ++i)
+                if (i < tid - kLuNB && p[i] == r) r = -1;
+        }
+        int64_t from = r;
+#pragma unroll 16
+        for (int i = kLuNB - 1; i >= 0; --i)
+            if (i < nb) from = from == k0 + i ? p[i] : from == p[i] ? k0 + i : from;
+        dst[tid] = from == r ? -1 : r;  // rows that keep their content are left alone
+        src[tid] = from;
+    }
+    __syncthreads();
+    const int64_t cols = n - nb;
+    const bool along_rows = A.cs == 1;  // a row's columns are contiguous
+    for (int64_t cb = (int64_t)blockIdx.x * kSwapCols; cb < cols; cb += (int64_t)gridDim.x * kSwapCols) {
+        auto each = [&](auto body) {
+#pragma unroll 4
+            for (int e = tid; e < 2 * kLuNB * kSwapCols; e += 256) {
+                const int d = along_rows ? e / kSwapCols : e % (2 * kLuNB);
+                const int c = along_rows ? e % kSwapCols : e / (2 * kLuNB);
+                if (dst[d] >= 0 && cb + c < cols) body(d, c, cb + c < k0 ? cb + c : cb + c + nb);
+            }
+        };
+        each([&](int d, int c, int64_t col) { tile[d][c] = A(src[d], col); });
+        __syncthreads();
+        each([&](int d, int c, int64_t col) { A(dst[d], col) = tile[d][c]; });
+        __syncthreads();
     }
 }
 
@@ -450,6 +862,44 @@ View<T> view_of(int row_major, T* A, int64_t lda) {
     return row_major ? View<T>{A, lda, 1} : View<T>{A, 1, lda};
 }
 
+template <class T>
+void cluster_config(int G, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)G;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->gridDim = dim3((unsigned)G);
+    cfg->blockDim = dim3(kClThreads);
+    cfg->dynamicSmemBytes = sizeof(ClusterSmem<T>);
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+}
+
+// CTAs of the cluster that holds a panel of `rows` rows, 0 where none does: more than 4096 rows,
+// or a device that cannot run such a cluster (asked once per size).
+template <class T>
+int cluster_size(int64_t rows) {
+    static std::atomic<int> fits[5];  // 0: not asked, 1: yes, 2: no
+    int g = 1, lg = 0;
+    for (; g < kClMax && (int64_t)g * kClThreads < rows; g *= 2) ++lg;
+    if ((int64_t)g * kClThreads < rows) return 0;
+    int f = fits[lg].load(std::memory_order_relaxed);
+    if (f == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        cluster_config<T>(g, &cfg, &attr);
+        int num = 0;
+        auto kernel = getrf_panel_cluster_kernel<T>;
+        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(ClusterSmem<T>)) == cudaSuccess &&
+                        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&num, kernel, &cfg) == cudaSuccess && num > 0;
+        if (!ok) cudaGetLastError();
+        f = ok ? 1 : 2;
+        fits[lg].store(f, std::memory_order_relaxed);
+    }
+    return f == 1 ? g : 0;
+}
+
 // The panel on a cooperative grid of about 256 rows per CTA (a grid barrier costs more the
 // more CTAs meet at it, the column work per CTA grows with its rows), at most one CTA per
 // SM; on one CTA when the panel's rows do not fit the grid's shared memory (n above ~56K).
@@ -463,6 +913,19 @@ int getrf_panel(int64_t n, View<T> A, int64_t k0, int nb, int* piv, int* info, T
     const int sms = sm_count();
     int G = (int)((rows + kCoopRows - 1) / kCoopRows);
     if (G > sms) G = sms;
+    const int cl = cluster_size<T>(rows);
+    if (cl > 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        cluster_config<T>(cl, &cfg, &attr);
+        cfg.stream = s;
+        if (cudaLaunchKernelEx(&cfg, getrf_panel_cluster_kernel<T>, n, A, k0, nb, piv, info, linv, error_word(),
+                               wait_limit_ns()) != cudaSuccess)
+            return RC_ERR_CUDA;
+        RC_TRY(check_launch());
+        *have_inv = true;
+        return RC_SUCCESS;
+    }
     const int chunk = (int)((rows + G - 1) / G);
     if (chunk > kCoopMaxChunk || sms <= 0) {
         getrf_panel_kernel<T><<<1, kLuThreads, 0, s>>>(n, A, k0, nb, piv, info);
@@ -510,8 +973,8 @@ int getrf(int row_major, int64_t n, T* Ap, int64_t lda, int* piv, int* info, cud
         RC_TRY(getrf_panel<T>(n, A, k0, nb, piv, info, linv, &have_inv, s));
         if (n > nb) {
             const int64_t cols = n - nb;
-            lu_swap_kernel<T><<<ceil_div(cols, 256) < 1024u ? ceil_div(cols, 256) : 1024u, 256, 0, s>>>(n, A, k0, nb,
-                                                                                                      piv, info);
+            const unsigned grid = ceil_div(cols, kSwapCols) < 4096u ? ceil_div(cols, kSwapCols) : 4096u;
+            lu_swap_kernel<T><<<grid, 256, 0, s>>>(n, A, k0, nb, piv, info);
             RC_TRY(check_launch());
         }
         const int64_t r = n - k0 - nb;
