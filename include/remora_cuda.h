@@ -357,6 +357,10 @@ int rc_potrf_backward_f64(size_t n, const double* L, size_t ldl, const double* L
 int rc_trsm_backward_f64(int trans, size_t n, size_t nrhs, const double* L, size_t ldl,
                          const double* X, size_t ldx, double* Xbar, size_t ldxb, double* Lbar,
                          size_t ldlb, void* stream);
+/* rc_nll_adjoint_f64: the adjoint of f(K) = 1/2 y^T K^-1 y + 1/2 log det K from K = L L^T and
+ * a = K^-1 y: Kbar = 1/2 (L^-T L^-1 - a a^T), full and symmetric; L's lower triangle is read. */
+int rc_nll_adjoint_f64(size_t n, const double* L, size_t ldl, const double* a, double* Kbar, size_t ldkb,
+                       void* stream);
 /* Gaussian-process RBF kernel around the differentiated Cholesky: X is n x d row-major
  * (d <= 16), ls the d lengthscales. rc_rbf_kernel_f64 writes
  * K_ij = exp(-1/2 sum_q ((x_iq - x_jq) / ls_q)^2) + noise [i == j]; the gradient call

@@ -101,6 +101,7 @@ SIGNATURES: dict[str, list] = {
     "rc_syrk_emu64": [_Z, _Z, c_double, _P, _Z, c_double, _P, _Z, _P],
     "rc_potrf_backward_f64": [_Z, _P, _Z, _P, _Z, _P, _Z, _P],
     "rc_trsm_backward_f64": [_I, _Z, _Z, _P, _Z, _P, _Z, _P, _Z, _P, _Z, _P],
+    "rc_nll_adjoint_f64": [_Z, _P, _Z, _P, _P, _Z, _P],
     "rc_rbf_kernel_f64": [_Z, _I, _P, _P, c_double, _P, _Z, _P],
     "rc_rbf_lengthscale_grad_f64": [_Z, _I, _P, _P, _P, _Z, _P, _P],
     "rc_copy2d_f64": [_I, _Z, _Z, c_double, _P, _Z, _P, _Z, _P],

