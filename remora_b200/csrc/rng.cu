@@ -9,7 +9,7 @@
 // along the storage's contiguous direction so each warp store is one or four 128-byte
 // segments (16-byte vector stores for aligned row-major rows), a bounds check on both
 // indices (the reference writes past the matrix when cols % 64 != 0, :172, :186), and
-// a grid that strides over rows so row counts above 65535 launch.
+// threads that keep their place along the contiguous direction and walk the other one.
 #include "common.cuh"
 #include <cmath>
 
@@ -56,6 +56,58 @@ __device__ __forceinline__ float uniform1(uint32_t x, float low, float range) {
     return nextafterf(__fmaf_rn(unit_float(x), range, low), low);
 }
 
+// The fills are bound by instruction issue, so the normal transform's functions cover just the
+// arguments it has. 2^28 normals (16384 x 16384, row-major): 705 -> 449 us; the general
+// library functions branch around cases that do not occur here.
+
+// Bit pattern of nextafter(unit_float(x), 0): one less than the float's for x > 0, else 0.
+__device__ __forceinline__ int unit_below(uint32_t x) {
+    return max(__float_as_int(__uint2float_rn(x)) - ((32 << 23) + 1), 0);
+}
+
+// sqrt(-2 log(u)) for the float u of bit pattern 0 (infinity) or 2^-32 <= u < 1, one float down. The
+// logarithm is e log 2 + log(1 + f), 1 + f in [sqrt(1/2), sqrt(2)), log(1 + f) = f - f^2 / 2 +
+// f^3 P(f) with a P of degree 7 fitted to the relative error by iteratively reweighted least
+// squares (Lawson): within 0.9 ulp. The root of t is t rsqrt(t) with one Newton correction.
+__device__ __forceinline__ float sqrt_m2log(int bits) {
+    const int d = bits - 0x3f3504f3, e = d >> 23;  // 0x3f3504f3: sqrt(1/2)
+    const float f = __int_as_float(bits - (e << 23)) - 1.0f;
+    float p = -0x1.38b6p-4f;
+    p = __fmaf_rn(p, f, 0x1.055bd2p-3f);
+    p = __fmaf_rn(p, f, -0x1.0d855cp-3f);
+    p = __fmaf_rn(p, f, 0x1.22da10p-3f);
+    p = __fmaf_rn(p, f, -0x1.547240p-3f);
+    p = __fmaf_rn(p, f, 0x1.99a008p-3f);
+    p = __fmaf_rn(p, f, -0x1.000228p-2f);
+    p = __fmaf_rn(p, f, 0x1.555554p-2f);
+    p = __fmaf_rn(p, f, -0.5f);
+    p = __fmaf_rn(p, f * f, f);
+    // e as a float: 1.5 2^23 + e has the bits of 1.5 2^23, plus e
+    const float ef = __int_as_float(e + 0x4b400000) - 12582912.0f;
+    const float t = -2.0f * __fmaf_rn(ef, 0x1.62e43p-1f, p);
+    float y;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(t));
+    const float r = t * y;
+    const float root = __fmaf_rn(__fmaf_rn(-r, r, t), 0.5f * y, r);
+    return bits == 0 ? __int_as_float(0x7f800000) : root;
+}
+
+// Sine and cosine of q = 2 pi u rounded to a float, 0 <= u < 1: q less the nearest multiple of pi / 2
+// (in two parts, Cody and Waite), then polynomials on [-pi/4, pi/4] fitted as above: within 1.5
+// ulp.
+__device__ __forceinline__ void sincos_2pi(float u, float* sine, float* cosine) {
+    const float q = (2.0f * 3.14159265358979323846f) * u;
+    const float biased = __fmaf_rn(u, 4.0f, 12582912.0f), kf = biased - 12582912.0f;
+    const int k = __float_as_int(biased);
+    const float r = __fmaf_rn(-kf, -0x1.777a5cp-25f, __fmaf_rn(-kf, 0x1.921fb6p+0f, q)), z = r * r;
+    const float ps = __fmaf_rn(__fmaf_rn(-0x1.994386p-13f, z, 0x1.11073ap-7f), z, -0x1.555546p-3f);
+    const float pc = __fmaf_rn(__fmaf_rn(0x1.99eb4ap-16f, z, -0x1.6c0c32p-10f), z, 0x1.55554ap-5f);
+    const float s = __fmaf_rn(ps * z, r, r), c = __fmaf_rn(z, __fmaf_rn(z, pc, -0.5f), 1.0f);
+    const bool odd = k & 1;
+    *sine = __int_as_float(__float_as_int(odd ? c : s) ^ ((k << 30) & 0x80000000));
+    *cosine = __int_as_float(__float_as_int(odd ? s : c) ^ (((k + 1) << 30) & 0x80000000));
+}
+
 enum Kind { kBits = 0, kUniform = 1, kNormal = 2, kDiscreteF = 3, kDiscreteI = 4 };
 
 template <int K>
@@ -74,15 +126,10 @@ __device__ __forceinline__ void transform(uint4 x, float a, float b, int ia, uin
         v[2] = uniform1(x.z, a, range); v[3] = uniform1(x.w, a, range);
     } else if constexpr (K == kNormal) {
         // Box-Muller on the four uniforms in [0,1] (random.hpp:119-132); a = mean, b = stddev.
-        const float u0 = uniform1(x.x, 0.f, 1.f), u1 = uniform1(x.y, 0.f, 1.f);
-        const float u2 = uniform1(x.z, 0.f, 1.f), u3 = uniform1(x.w, 0.f, 1.f);
-        const float r0 = sqrtf(-2.0f * logf(u0));
-        const float r1 = sqrtf(-2.0f * logf(u1));
-        const float two_pi = 2.0f * 3.14159265358979323846f;
+        const float g0 = b * sqrt_m2log(unit_below(x.x)), g1 = b * sqrt_m2log(unit_below(x.y));
         float s0, c0, s1, c1;
-        sincosf(two_pi * u2, &s0, &c0);
-        sincosf(two_pi * u3, &s1, &c1);
-        const float g0 = b * r0, g1 = b * r1;
+        sincos_2pi(__int_as_float(unit_below(x.z)), &s0, &c0);
+        sincos_2pi(__int_as_float(unit_below(x.w)), &s1, &c1);
         v[0] = __fmaf_rn(g0, s0, a); v[1] = __fmaf_rn(g0, c0, a);
         v[2] = __fmaf_rn(g1, s1, a); v[3] = __fmaf_rn(g1, c1, a);
     } else if constexpr (K == kDiscreteF) {
@@ -95,54 +142,56 @@ __device__ __forceinline__ void transform(uint4 x, float a, float b, int ia, uin
     }
 }
 
-// Row-major: thread x walks 4-column groups of one row (contiguous), grid.y strides rows.
+// Row-major: a thread keeps its 4-column group and walks rows, so what of the stream's rounds
+// depends on the columns alone is computed once; a warp stores 128 consecutive elements.
 template <int K>
 __global__ void __launch_bounds__(256) fill_rowmajor(typename Out<K>::type* __restrict__ A, uint64_t ld,
                                                       uint64_t rows, uint64_t cols, uint4 key, float a,
                                                       float b, int ia, uint32_t N, bool vec_ok) {
     using T = typename Out<K>::type;
     const uint64_t groups = (cols + 3) / 4;
-    for (uint64_t i = blockIdx.y; i < rows; i += gridDim.y) {
-        T* row = A + i * ld;
-        for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups;
-             g += (uint64_t)gridDim.x * blockDim.x) {
-            const uint64_t j = 4 * g;
-            uint4 ctr = make_uint4((uint32_t)(i & 0xffffu), (uint32_t)(i >> 32), (uint32_t)(j & 0xffffu),
-                                   (uint32_t)(j >> 32));
+    for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups;
+         g += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t j = 4 * g;
+        const uint32_t cz = (uint32_t)(j & 0xffffu), cw = (uint32_t)(j >> 32);
+        T* out = A + blockIdx.y * ld + j;
+        for (uint64_t i = blockIdx.y; i < rows; i += gridDim.y, out += gridDim.y * ld) {
             T v[4];
-            transform<K>(threefry(ctr, key), a, b, ia, N, v);
+            transform<K>(threefry(make_uint4((uint32_t)(i & 0xffffu), (uint32_t)(i >> 32), cz, cw), key), a, b, ia, N,
+                         v);
             if (vec_ok && j + 3 < cols) {
                 uint4 packed;
                 memcpy(&packed, v, sizeof(packed));
-                reinterpret_cast<uint4*>(row + j)[0] = packed;
+                reinterpret_cast<uint4*>(out)[0] = packed;
             } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    if (j + c < cols) row[j + c] = v[c];
+                    if (j + c < cols) out[c] = v[c];
             }
         }
     }
 }
 
-// Column-major: thread x walks rows (contiguous), each thread writes the 4 columns of its
-// group, so every store instruction of a warp covers 32 consecutive elements of one column.
+// Column-major: a thread keeps its row and walks 4-column groups, so every store instruction of
+// a warp covers 32 consecutive elements of one column.
 template <int K>
 __global__ void __launch_bounds__(256) fill_colmajor(typename Out<K>::type* __restrict__ A, uint64_t ld,
                                                       uint64_t rows, uint64_t cols, uint4 key, float a,
                                                       float b, int ia, uint32_t N) {
     using T = typename Out<K>::type;
     const uint64_t groups = (cols + 3) / 4;
-    for (uint64_t g = blockIdx.y; g < groups; g += gridDim.y) {
-        const uint64_t j = 4 * g;
-        for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows;
-             i += (uint64_t)gridDim.x * blockDim.x) {
-            uint4 ctr = make_uint4((uint32_t)(i & 0xffffu), (uint32_t)(i >> 32), (uint32_t)(j & 0xffffu),
-                                   (uint32_t)(j >> 32));
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t cx = (uint32_t)(i & 0xffffu), cy = (uint32_t)(i >> 32);
+        T* out = A + i + 4 * blockIdx.y * ld;
+        for (uint64_t g = blockIdx.y; g < groups; g += gridDim.y, out += 4 * gridDim.y * ld) {
+            const uint64_t j = 4 * g;
             T v[4];
-            transform<K>(threefry(ctr, key), a, b, ia, N, v);
+            transform<K>(threefry(make_uint4(cx, cy, (uint32_t)(j & 0xffffu), (uint32_t)(j >> 32)), key), a, b, ia, N,
+                         v);
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                if (j + c < cols) A[i + (j + c) * ld] = v[c];
+                if (j + c < cols) out[c * ld] = v[c];
         }
     }
 }
@@ -164,17 +213,18 @@ int launch_fill(const uint32_t key[4], size_t rows, size_t cols, void* Av, size_
     T* A = static_cast<T*>(Av);
     const uint4 k = make_uint4(key[0], key[1], key[2], key[3]);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const unsigned threads = 256;
+    // Along x a block covers the contiguous direction; along y, threads of as many blocks as fill
+    // the SMs four times over share the steps of the other one: enough that the last ones to
+    // finish cost little, few enough that their prologues do.
+    constexpr unsigned threads = 256;
+    const uint64_t groups = (cols + 3) / 4, along = row_major ? groups : rows, steps = row_major ? rows : groups;
+    const unsigned gx = ceil_div(along, threads) < 65535u ? ceil_div(along, threads) : 65535u;
+    const uint64_t share = ceil_div((uint64_t)sm_count() * 32, gx);
+    const dim3 grid(gx, (unsigned)(steps < share ? steps : share));
     if (row_major) {
-        const uint64_t groups = (cols + 3) / 4;
         const bool vec_ok = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (ld % 4 == 0);
-        dim3 grid(ceil_div(groups, threads) < 65535u ? ceil_div(groups, threads) : 65535u,
-                  rows < 65535 ? (unsigned)rows : 65535u);
         fill_rowmajor<K><<<grid, threads, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N, vec_ok);
     } else {
-        const uint64_t groups = (cols + 3) / 4;
-        dim3 grid(ceil_div(rows, threads) < 65535u ? ceil_div(rows, threads) : 65535u,
-                  groups < 65535 ? (unsigned)groups : 65535u);
         fill_colmajor<K><<<grid, threads, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N);
     }
     return check_launch();
