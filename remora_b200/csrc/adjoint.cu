@@ -18,6 +18,7 @@
 #include "assign.cuh"
 #include "factor.cuh"
 #include "gemm.cuh"
+#include "strip.cuh"
 
 namespace rc {
 namespace {
@@ -124,9 +125,7 @@ int trsm_backward(bool trans, int64_t n, int64_t nrhs, View<const double> L, Vie
 // a 64-bit library result 7.2e-15 -> 2.5e-15.
 int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> Kbar, cudaStream_t s) {
     if (n <= 0) return RC_SUCCESS;
-    // Trailing updates of depth 512 as in the factorisation; the 128-row steps inside a panel
-    // are products with at most 384 rows.
-    constexpr int64_t kPanel = 512;
+    constexpr int64_t kPanel = kStripRows;  // trailing updates as deep as the factorisation's
     double* w = static_cast<double*>(workspace(s, (size_t)n * n * sizeof(double), 8));
     double* W = static_cast<double*>(workspace(s, (size_t)ceil_div(n, kNB) * kNB * kNB * sizeof(double), 1));
     if (!w || !W) return RC_ERR_ALLOC;
@@ -141,15 +140,7 @@ int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> K
     RC_TRY(trtri_blocks_launch<double>(n, L, false, W, nullptr, nullptr, s));
     for (int64_t p = 0; p < n; p += kPanel) {
         const int64_t pe = n - p < kPanel ? n : p + kPanel;
-        for (int64_t r = p; r < pe; r += kNB) {
-            const int64_t sz = pe - r < kNB ? pe - r : kNB, cols = r + sz;
-            const View<const double> Wb = {W + r / kNB * kNB * kNB, 1, kNB};
-            // in place, on a DMMA tile that spans the block's rows
-            RC_TRY(gemm<double>(sz, cols, sz, 1.0, Wb, C_(X.sub(r, 0)), 0.0, X.sub(r, 0), kFull, 0, s));
-            if (cols < pe)
-                RC_TRY(gemm<double>(pe - cols, cols, sz, -1.0, L.sub(cols, r), C_(X.sub(r, 0)), 1.0, X.sub(cols, 0),
-                                    kFull, 0, s));
-        }
+        RC_TRY(strip_solve<double>(false, pe - p, pe, L.sub(p, p), W + p * kNB, false, X.sub(p, 0), s, nullptr));
         const View<const double> Xp = C_(X.sub(p, 0));
         RC_TRY(gemm<double>(pe, pe, pe - p, 0.5, Xp.t(), Xp, 1.0, Kbar, kLower, 0, s));
         if (pe < n)

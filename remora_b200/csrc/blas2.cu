@@ -179,8 +179,9 @@ int trsv_abi(int upper, int trans, int unit, size_t n, const T* A, size_t lda, T
         Av = Av.t();
         up = !up;
     }
-    return rc::trsm_left<T>(up, unit != 0, (int64_t)n, 1, T(1), Av, rc::View<T>{x, (int64_t)incx, (int64_t)n * (int64_t)incx},
-                            nullptr, static_cast<cudaStream_t>(stream));
+    // a strided vector is a row-major n x 1 matrix
+    const rc::View<T> xv{x, (int64_t)incx, incx == 1 ? (int64_t)n : 1};
+    return rc::trsm_left<T>(up, unit != 0, (int64_t)n, 1, T(1), Av, xv, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 template <class T>

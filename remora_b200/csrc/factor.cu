@@ -16,6 +16,7 @@
 #include "assign.cuh"
 #include "diag.cuh"
 #include "gemm.cuh"
+#include "strip.cuh"
 #include <type_traits>
 
 namespace rc {
@@ -148,6 +149,29 @@ __device__ __forceinline__ void store_block(const View<T>& A, int sz, bool rowma
     }
 }
 
+// The same as calls: inlined, the FP32 instance's conversions took registers from the dependent
+// chain of potrf_diag (44 us a block, 36 with calls; 29 in FP64).
+__device__ __noinline__ void load_block_call(const View<float>& A, int sz, bool rowmaj, int q, double* S, int lane) {
+    load_block(A, sz, rowmaj, false, q, S, lane);
+}
+__device__ __noinline__ void store_block_call(const View<float>& A, int sz, bool rowmaj, int q, int h, const double* S,
+                                              const double* ld, int lane) {
+    store_block(A, sz, rowmaj, q, h, S, ld, lane);
+}
+__device__ __noinline__ void store_inverse_call(const double* S, float* W, bool row_major, int q, int h, int lane) {
+    store_inverse(S, W, row_major, q, h, lane);
+}
+__device__ __forceinline__ void load_block_call(const View<double>& A, int sz, bool rowmaj, int q, double* S, int lane) {
+    load_block(A, sz, rowmaj, false, q, S, lane);
+}
+__device__ __forceinline__ void store_block_call(const View<double>& A, int sz, bool rowmaj, int q, int h,
+                                                 const double* S, const double* ld, int lane) {
+    store_block(A, sz, rowmaj, q, h, S, ld, lane);
+}
+__device__ __forceinline__ void store_inverse_call(const double* S, double* W, bool row_major, int q, int h, int lane) {
+    store_inverse(S, W, row_major, q, h, lane);
+}
+
 // Named barriers of potrf_diag: kBarChunk + h says that columns 8 h .. 8 h + 7 of the
 // sub-block being factored are in Lt and rd (warp 0 arrives, their readers wait).
 constexpr int kBarBackground = 1, kBarChunk = 2;
@@ -274,7 +298,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
     // chunk barriers.
     auto solvers = [](int kb) { return kb < 6 ? (NB - DB * kb - 1) / 32 : 0; };
     auto participants = [&](int kb) { return 32 * (2 + solvers(kb)); };
-    if (warp < 10) load_block(A, sz, rowmaj, false, warp, S, lane);
+    if (warp < 10) load_block_call(A, sz, rowmaj, warp, S, lane);
     if (skip) return;
     sync_all();
     if (warp == 0) {
@@ -377,7 +401,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
         for (int kb = 0; kb < NSUB; ++kb) {
             if (kb < NSUB - 1) zero_upper(W, w_row_major, kb, 32 * (warp / 4 - 1) + lane);
             if (kb == NSUB - 1)  // the inverse's final blocks (0, 0), (1, 0), (1, 1), (2, 2)
-                for (int q = warp / 4 - 1; q < 8; q += 3) store_inverse(S, W, w_row_major, q < 6 ? q >> 1 : 5, q & 1, lane);
+                for (int q = warp / 4 - 1; q < 8; q += 3) store_inverse_call(S, W, w_row_major, q < 6 ? q >> 1 : 5, q & 1, lane);
             while (redo()) {}
             if (flags[0]) return;
             next_panel(DB * kb);
@@ -393,11 +417,11 @@ __global__ void __launch_bounds__(kDiagThreads, 1) potrf_diag(View<T> A, int sz,
         merge_x<64, SLD>(S, T64, 0, 32, 8 * warp, lane);
         merge_x<64, SLD>(S, T64, 0, 48, 8 * warp, lane);
     } else {
-        for (int q = warp - 8; q < 20; q += 8) store_block(A, sz, rowmaj, q >> 1, q & 1, S, ld, lane);
+        for (int q = warp - 8; q < 20; q += 8) store_block_call(A, sz, rowmaj, q >> 1, q & 1, S, ld, lane);
     }
     __syncthreads();
     if (warp < 12)  // the blocks of the inverse that are not stored yet
-        store_inverse(S, W, w_row_major, warp < 4 ? 3 + (warp >> 1) : 6 + ((warp - 4) >> 1), warp & 1, lane);
+        store_inverse_call(S, W, w_row_major, warp < 4 ? 3 + (warp >> 1) : 6 + ((warp - 4) >> 1), warp & 1, lane);
 }
 
 template <class K>
@@ -409,67 +433,71 @@ int set_smem(K kernel, size_t bytes) {
 
 }  // namespace
 
+// One sweep of substitution with the triangle A, given the inverses W of its diagonal blocks:
+// panels solved a strip of columns per CTA, the other rows updated once per panel. 8192 x 1024:
+// 2.92 ms (3.81 with a product, a copy and an update of all other rows per 128-row block), 2.28 of it in
+// the updates.
+template <class T>
+int sweep(bool upper, int64_t m, int64_t n, View<const T> A, const T* W, bool w_row_major, View<T> B, cudaStream_t s,
+          const int* abort) {
+    constexpr int64_t per = kStripRows;
+    const int64_t panels = (m + per - 1) / per;
+    for (int64_t q = 0; q < panels; ++q) {
+        const int64_t p0 = (upper ? panels - 1 - q : q) * per, sz = m - p0 < per ? m - p0 : per;
+        const View<T> Bp = B.sub(p0, 0);
+        RC_TRY(strip_solve<T>(upper, sz, n, A.sub(p0, p0), W + (size_t)p0 * NB, w_row_major, Bp, s, abort));
+        const int64_t from = upper ? 0 : p0 + sz, rows = upper ? p0 : m - from;
+        if (rows > 0)
+            RC_TRY(gemm<T>(rows, n, sz, T(-1), A.sub(from, p0), View<const T>{Bp.p, Bp.rs, Bp.cs}, T(1),
+                           B.sub(from, 0), kFull, 0, s, abort));
+    }
+    return RC_SUCCESS;
+}
+
 template <class T>
 int trsm_left(bool upper, bool unit, int64_t m, int64_t n, T alpha, View<const T> A, View<T> B, int* info,
               cudaStream_t s, const int* abort) {
     if (m <= 0 || n <= 0) return RC_SUCCESS;
     const int64_t nblk = (m + NB - 1) / NB;
     T* W = static_cast<T*>(workspace(s, (size_t)nblk * NB * NB * sizeof(T), 1));
-    T* tmp = static_cast<T*>(workspace(s, (size_t)NB * n * sizeof(T), 2));
-    if (!W || !tmp) return RC_ERR_ALLOC;
-    const View<const T> L = upper ? A.t() : A;
-    RC_TRY(set_smem(trtri_blocks<T>, kDiagSmem));
-    trtri_blocks<T><<<(unsigned)nblk, kDiagThreads, kDiagSmem, s>>>(m, L, unit, W, info, abort);
-    RC_TRY(check_launch());
+    if (!W) return RC_ERR_ALLOC;
+    RC_TRY(trtri_blocks_launch<T>(m, upper ? A.t() : A, unit, W, info, abort, s));
     if (alpha != T(1)) RC_TRY(copy2d<T, T>(m, n, alpha, View<const T>{B.p, B.rs, B.cs}, B, s, abort));
-    const View<T> Tv = colmajor(tmp, (int64_t)NB);
-    for (int64_t step = 0; step < nblk; ++step) {
-        const int64_t b = upper ? nblk - 1 - step : step;
-        const int64_t r0 = b * NB, sz = (m - r0 < NB) ? m - r0 : NB;
-        const View<const T> X = {W + (size_t)b * NB * NB, 1, NB};
-        View<T> Bb = B.sub(r0, 0);
-        RC_TRY(gemm<T>(sz, n, sz, T(1), upper ? X.t() : X, View<const T>{Bb.p, Bb.rs, Bb.cs}, T(0), Tv, kFull, 0, s,
-                       abort));
-        RC_TRY(copy2d<T, T>(sz, n, T(1), View<const T>{Tv.p, Tv.rs, Tv.cs}, Bb, s, abort));
-        const View<const T> Bc = {Bb.p, Bb.rs, Bb.cs};
-        if (!upper && r0 + sz < m)
-            RC_TRY(gemm<T>(m - r0 - sz, n, sz, T(-1), A.sub(r0 + sz, r0), Bc, T(1), B.sub(r0 + sz, 0), kFull, 0, s,
-                           abort));
-        if (upper && r0 > 0) RC_TRY(gemm<T>(r0, n, sz, T(-1), A.sub(0, r0), Bc, T(1), B, kFull, 0, s, abort));
-    }
-    return RC_SUCCESS;
+    return trsm_preinv<T>(upper, m, n, A, W, false, B, s, abort);
 }
 
 template <class T>
-int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s) {
+int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s, T* Winv) {
     if (!info) return RC_ERR_INVALID_ARGUMENT;
     if (cudaMemsetAsync(info, 0, sizeof(int), s) != cudaSuccess) return RC_ERR_CUDA;
     if (n <= 0) return RC_SUCCESS;
-    T* W = static_cast<T*>(workspace(s, (size_t)NB * NB * sizeof(T), 1));
-    if (!W) return RC_ERR_ALLOC;
-    // An in-place FP64 product runs on a DMMA tile that spans the panel's 128 columns, so one
-    // CTA owns every column of its rows and the panel solve can write in place; other types
-    // go through a buffer.
+    // Outer panels of kOuter columns: 128-column steps factor the panel's diagonal block, the rows
+    // below it are solved a strip per CTA, and the trailing matrix gets one update of depth
+    // kOuter. SPD solve n = 1024, 16 right-hand sides: 730 -> 595 us; FP32 factor and solves
+    // n = 3001: 3.09 -> 2.48 ms.
+    constexpr int64_t kOuter = kStripRows;
+    T* own = Winv ? nullptr : static_cast<T*>(workspace(s, (size_t)kOuter * NB * sizeof(T), 1));
+    if (!Winv && !own) return RC_ERR_ALLOC;
+    // An in-place FP64 product runs on a DMMA tile that spans the step's 128 columns, so one
+    // CTA owns every column of its rows; other types go through a buffer.
     constexpr bool in_place = std::is_same<T, double>::value;
     T* tmp = nullptr;
     if (!in_place) {
-        tmp = static_cast<T*>(workspace(s, (size_t)n * NB * sizeof(T), 2));
+        tmp = static_cast<T*>(workspace(s, (size_t)kOuter * NB * sizeof(T), 2));
         if (!tmp) return RC_ERR_ALLOC;
     }
     RC_TRY(set_smem(potrf_diag<T>, kDiagSmem));
-    const View<const T> Wt = {W, NB, 1};  // inv(L_jj)^T
-    // Outer panels of kOuter columns: inner 128-column blocks update only the rest of
-    // their panel, and the trailing matrix gets one update of depth kOuter per panel, so
-    // the dominant GEMM streams its C tiles kOuter / 128 times less often.
-    constexpr int64_t kOuter = 512;
     auto C_ = [](const View<T>& v) { return View<const T>{v.p, v.rs, v.cs}; };
     for (int64_t k0 = 0; k0 < n; k0 += kOuter) {
-        const int64_t w = (n - k0) < kOuter ? n - k0 : kOuter;
-        for (int64_t j0 = k0; j0 < k0 + w; j0 += NB) {
-            const int jb = (int)((k0 + w - j0) < NB ? k0 + w - j0 : NB);
+        const int64_t w = (n - k0) < kOuter ? n - k0 : kOuter, end = k0 + w;
+        T* Wp = Winv ? Winv + k0 * NB : own;
+        for (int64_t j0 = k0; j0 < end; j0 += NB) {
+            const int jb = (int)(end - j0 < NB ? end - j0 : NB);
+            T* W = Wp + (j0 - k0) * NB;
+            const View<const T> Wt = {W, NB, 1};  // inv(L_jj)^T
             potrf_diag<T><<<1, kDiagThreads, kDiagSmem, s>>>(A.sub(j0, j0), jb, j0, W, info, false);
             RC_TRY(check_launch());
-            const int64_t rows = n - j0 - jb;
+            const int64_t rows = end - j0 - jb;
             if (rows <= 0) continue;
             View<T> P = A.sub(j0 + jb, j0);
             if (in_place) {
@@ -479,15 +507,14 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s) {
                 RC_TRY(gemm<T>(rows, jb, jb, T(1), C_(P), Wt, T(0), Tv, kFull, 0, s, info));
                 RC_TRY(copy2d<T, T>(rows, jb, T(1), C_(Tv), P, s, info));
             }
-            const int64_t cw = k0 + w - (j0 + jb);
-            if (cw > 0)
-                RC_TRY(gemm<T>(rows, cw, jb, T(-1), C_(P), C_(P).t(), T(1), A.sub(j0 + jb, j0 + jb), kLower, 0, s,
-                               info));
+            RC_TRY(gemm<T>(rows, rows, jb, T(-1), C_(P), C_(P).t(), T(1), A.sub(j0 + jb, j0 + jb), kLower, 0, s,
+                           info));
         }
-        const int64_t rows = n - k0 - w;
+        const int64_t rows = n - end;
         if (rows <= 0) continue;
-        const View<T> Pk = A.sub(k0 + w, k0);
-        RC_TRY(gemm<T>(rows, rows, w, T(-1), C_(Pk), C_(Pk).t(), T(1), A.sub(k0 + w, k0 + w), kLower, 0, s, info));
+        const View<T> Pk = A.sub(end, k0);
+        RC_TRY(strip_solve<T>(false, w, rows, C_(A.sub(k0, k0)), Wp, false, Pk.t(), s, info));
+        RC_TRY(gemm<T>(rows, rows, w, T(-1), C_(Pk), C_(Pk).t(), T(1), A.sub(end, end), kLower, 0, s, info));
     }
     return RC_SUCCESS;
 }
@@ -500,24 +527,11 @@ int potrf_diag_block(View<T> A, int sz, int64_t g0, T* W, bool w_row_major, int*
 }
 
 template <class T>
-int trsm_preinv(bool trans, int64_t m, int64_t n, View<const T> L, const T* Winv, View<T> B, T* tmp, cudaStream_t s) {
+int trsm_preinv(bool upper, int64_t m, int64_t n, View<const T> A, const T* Winv, bool w_row_major, View<T> B,
+                cudaStream_t s, const int* abort) {
     if (m <= 0 || n <= 0) return RC_SUCCESS;
-    const int64_t nblk = (m + NB - 1) / NB;
-    const View<T> Tv = colmajor(tmp, (int64_t)NB);
-    const View<const T> Tc = {tmp, 1, (int64_t)NB};
-    for (int64_t step = 0; step < nblk; ++step) {
-        const int64_t b = trans ? nblk - 1 - step : step;
-        const int64_t r0 = b * NB, sz = (m - r0 < NB) ? m - r0 : NB;
-        const View<const T> X = {Winv + (size_t)b * NB * NB, NB, 1};
-        View<T> Bb = B.sub(r0, 0);
-        const View<const T> Bc = {Bb.p, Bb.rs, Bb.cs};
-        RC_TRY(gemm<T>(sz, n, sz, T(1), trans ? X.t() : X, Bc, T(0), Tv, kFull, 0, s));
-        RC_TRY(copy2d<T, T>(sz, n, T(1), Tc, Bb, s));
-        if (!trans && r0 + sz < m)
-            RC_TRY(gemm<T>(m - r0 - sz, n, sz, T(-1), L.sub(r0 + sz, r0), Bc, T(1), B.sub(r0 + sz, 0), kFull, 0, s));
-        if (trans && r0 > 0) RC_TRY(gemm<T>(r0, n, sz, T(-1), L.sub(r0, 0).t(), Bc, T(1), B, kFull, 0, s));
-    }
-    return RC_SUCCESS;
+    const bool flip = upper != w_row_major;  // an upper triangle's blocks are the transposed inverses
+    return sweep<T>(upper, m, n, A, Winv, flip, B, s, abort);
 }
 
 template <class T>
@@ -531,16 +545,14 @@ int trtri_blocks_launch(int64_t m, View<const T> L, bool unit, T* W, int* info, 
 template int trtri_blocks_launch<double>(int64_t, View<const double>, bool, double*, int*, const int*, cudaStream_t);
 template int potrf_diag_block<float>(View<float>, int, int64_t, float*, bool, int*, cudaStream_t);
 template int potrf_diag_block<double>(View<double>, int, int64_t, double*, bool, int*, cudaStream_t);
-template int trsm_preinv<float>(bool, int64_t, int64_t, View<const float>, const float*, View<float>, float*,
-                                cudaStream_t);
-template int trsm_preinv<double>(bool, int64_t, int64_t, View<const double>, const double*, View<double>, double*,
-                                 cudaStream_t);
+template int trsm_preinv<double>(bool, int64_t, int64_t, View<const double>, const double*, bool, View<double>,
+                                 cudaStream_t, const int*);
 template int trsm_left<double>(bool, bool, int64_t, int64_t, double, View<const double>, View<double>, int*,
                                cudaStream_t, const int*);
 template int trsm_left<float>(bool, bool, int64_t, int64_t, float, View<const float>, View<float>, int*,
                               cudaStream_t, const int*);
-template int potrf_lower<double>(int64_t, View<double>, int*, cudaStream_t);
-template int potrf_lower<float>(int64_t, View<float>, int*, cudaStream_t);
+template int potrf_lower<double>(int64_t, View<double>, int*, cudaStream_t, double*);
+template int potrf_lower<float>(int64_t, View<float>, int*, cudaStream_t, float*);
 
 }  // namespace rc
 
@@ -602,12 +614,16 @@ int rc_spd_solve_f64(size_t n, size_t nrhs, const double* A, size_t lda, double*
     if (!L) return RC_ERR_ALLOC;
     const rc::View<double> Lv = rc::colmajor(L, (int64_t)n);
     RC_TRY(rc::copy2d<double, double>((int64_t)n, (int64_t)n, 1.0, rc::colmajor(A, (int64_t)lda), Lv, s));
-    RC_TRY(rc::potrf_lower<double>((int64_t)n, Lv, d_info, s));
+    // The factorisation's block inverses serve both solves.
+    const int64_t nn = (int64_t)n, nblk = rc::ceil_div(n, rc::kNB);
+    double* W = static_cast<double*>(rc::workspace(s, (size_t)nblk * rc::kNB * rc::kNB * sizeof(double), 1));
+    if (!W) return RC_ERR_ALLOC;
+    RC_TRY(rc::potrf_lower<double>(nn, Lv, d_info, s, W));
     if (nrhs == 0) return RC_SUCCESS;
-    const rc::View<const double> Lc = {L, 1, (int64_t)n};
+    const rc::View<const double> Lc = {L, 1, nn};
     const rc::View<double> Bv = rc::colmajor(B, (int64_t)ldb);
-    RC_TRY(rc::trsm_left<double>(false, false, (int64_t)n, (int64_t)nrhs, 1.0, Lc, Bv, nullptr, s, d_info));
-    return rc::trsm_left<double>(true, false, (int64_t)n, (int64_t)nrhs, 1.0, Lc.t(), Bv, nullptr, s, d_info);
+    RC_TRY(rc::trsm_preinv<double>(false, nn, (int64_t)nrhs, Lc, W, false, Bv, s, d_info));
+    return rc::trsm_preinv<double>(true, nn, (int64_t)nrhs, Lc.t(), W, false, Bv, s, d_info);
 }
 
 }  // extern "C"

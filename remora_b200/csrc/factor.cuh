@@ -19,7 +19,7 @@ __device__ __forceinline__ void record_first(int* info, int v) {
     }
 }
 
-// Solves op(A) X = alpha * B in place for B (m x n), op(A) the m x m view A restricted to
+// Solves op(A) X = alpha * B in place for B (m x n, row- or column-major), op(A) the m x m view A restricted to
 // its lower (upper = false) or upper triangle. info (device, may be null): receives the
 // 1-based index of the first exactly-zero diagonal when !unit. abort (may be null): the
 // whole solve is skipped when *abort != 0 at launch time.
@@ -29,9 +29,10 @@ int trsm_left(bool upper, bool unit, int64_t m, int64_t n, T alpha, View<const T
 
 // In-place Cholesky A = L L^T of the lower triangle of the n x n view A (the strictly
 // upper part is never written). info (device, required) is set to 0 first and then to the
-// global 1-based index of the first non-positive pivot.
+// global 1-based index of the first non-positive pivot. Winv (may be null) receives the
+// inverses of the diagonal blocks, as trtri_blocks_launch stores them.
 template <class T>
-int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s);
+int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s, T* Winv = nullptr);
 
 // Factor one sz x sz (sz <= kNB) lower diagonal block of A (view offset to the block)
 // in FP64 shared memory, write L back and store inv(L) as a kNB x kNB block into W
@@ -39,11 +40,13 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s);
 template <class T>
 int potrf_diag_block(View<T> A, int sz, int64_t g0, T* W, bool w_row_major, int* info, cudaStream_t s);
 
-// Blocked triangular solve with precomputed inverses of the kNB diagonal blocks of the
-// lower-triangular L (row-major blocks, as potrf_diag_block stores them):
-// trans = false: B <- L^-1 B; trans = true: B <- L^-T B. tmp holds kNB x n elements.
+// B <- A^-1 B for the lower or upper triangle A, given the inverses of the kNB diagonal blocks
+// of the lower triangle (A, or A^T when upper), as kNB x kNB blocks column-major
+// (trtri_blocks_launch) or row-major. B is row- or column-major: the in-place products need a
+// unit stride.
 template <class T>
-int trsm_preinv(bool trans, int64_t m, int64_t n, View<const T> L, const T* Winv, View<T> B, T* tmp, cudaStream_t s);
+int trsm_preinv(bool upper, int64_t m, int64_t n, View<const T> A, const T* Winv, bool w_row_major, View<T> B,
+                cudaStream_t s, const int* abort = nullptr);
 
 // Invert every kNB x kNB diagonal block of the lower-triangular m x m view L into W
 // (column-major kNB x kNB blocks, block b at W + b * kNB * kNB); skipped when *abort != 0.

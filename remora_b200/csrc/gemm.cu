@@ -324,6 +324,7 @@ using TileS = DmmaTile<32, 32, 2, 2, 4, 5>;   // small products: latency counts
 using TileT = DmmaTile<64, 16, 4, 1, 4, 4>;   // up to 16 columns
 using TileP = DmmaTile<32, 128, 1, 4, 4, 2>;  // one CTA owns whole rows of a 128-column panel (in place)
 using TileQ = DmmaTile<128, 32, 4, 1, 4, 2>;  // one CTA owns whole columns of a 128-row block (in place)
+using TileR = DmmaTile<128, 16, 4, 1, 4, 2>;  // the same for few columns: half the serial work per CTA
 
 // Shared-memory tile of an operand with ROWS rows (the m or n direction), in the order of
 // its global layout, so that 16-byte copies keep it: K-major tiles are [row][k] with rows
@@ -557,7 +558,7 @@ int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const d
     return check_launch();
 }
 
-enum TileId { kTileM, kTileS, kTileT, kTileP, kTileQ };
+enum TileId { kTileM, kTileS, kTileT, kTileP, kTileQ, kTileR };
 
 template <bool AK, bool BK, bool V16>
 int launch_tile(TileId id, const Shape& p, double alpha, View<const double> A, View<const double> B, double beta,
@@ -567,6 +568,7 @@ int launch_tile(TileId id, const Shape& p, double alpha, View<const double> A, V
     case kTileS: return launch_dmma<AK, BK, TileS, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
     case kTileT: return launch_dmma<AK, BK, TileT, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
     case kTileP: return launch_dmma<AK, BK, TileP, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
+    case kTileR: return launch_dmma<AK, BK, TileR, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
     default: return launch_dmma<AK, BK, TileQ, V16>(p, alpha, A, B, beta, C, off, nz, s, abort);
     }
 }
@@ -584,7 +586,7 @@ void pick_tile(const Shape& p, bool c_on_a, bool c_on_b, bool may_split, TileId*
         }
     };
     if (c_on_a || c_on_b) {
-        *id = c_on_a ? kTileP : kTileQ;
+        *id = c_on_a ? kTileP : p.n <= 16 * (int64_t)sm_count() ? kTileR : kTileQ;
         *nz = 1;
         return;
     }

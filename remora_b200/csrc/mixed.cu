@@ -765,7 +765,6 @@ struct Mixed {
     double* Winv64 = nullptr;
     void* Pe[2] = {nullptr, nullptr};
     EmuPanel pe[2];
-    double* tmp64 = nullptr;
     View<const double> Av() const { return {A, 1, lda}; }
     View<float> Wv() const { return {W, ldw, 1}; }
     View<double> W64v() const { return {W64, ldw, 1}; }
@@ -851,8 +850,8 @@ struct Mixed {
         col_scale_kernel<<<g, 256, 0, st>>>(n, nrhs, sc, Rin, ldr, Zout, ldz);
         RC_TRY(check_launch());
         const View<const double> L = {W64, ldw, 1};
-        RC_TRY(trsm_preinv<double>(false, n, nrhs, L, Winv64, colmajor(Zout, ldz), tmp64, st));
-        RC_TRY(trsm_preinv<double>(true, n, nrhs, L, Winv64, colmajor(Zout, ldz), tmp64, st));
+        RC_TRY(trsm_preinv<double>(false, n, nrhs, L, Winv64, true, colmajor(Zout, ldz), st));
+        RC_TRY(trsm_preinv<double>(true, n, nrhs, L.t(), Winv64, true, colmajor(Zout, ldz), st));
         col_scale_kernel<<<g, 256, 0, st>>>(n, nrhs, sc, Zout, ldz, Zout, ldz);
         return check_launch();
     }
@@ -1131,7 +1130,6 @@ int spd_solve_mixed(int prec, int64_t n, int64_t nrhs, const double* A, int64_t 
         M.W64 = buf.take<double>((size_t)n * M.ldw);
         M.Winv64 = buf.take<double>((size_t)M.nblk * kNB * kNB);
         for (int q = 0; q < 2; ++q) M.Pe[q] = buf.take<char>(emu_panel_bytes(n, o.outer));
-        M.tmp64 = buf.take<double>((size_t)kNB * nrhs);
     } else {
         M.W = buf.take<float>((size_t)n * M.ldw);
         M.Winv = buf.take<float>((size_t)M.nblk * kNB * kNB);
