@@ -685,14 +685,12 @@ int mixed_workspace_bytes(int64_t n, int64_t nrhs, int prec, int outer, size_t* 
         add((size_t)nblk * kNB * kNB * sizeof(double));  // diagonal-block inverses (FP64)
         add(emu_panel_bytes(n, ow));                     // digit splits of two outer panels
         add(emu_panel_bytes(n, ow));
-        add((size_t)kNB * nrhs * sizeof(double));        // TRSM tile buffer
     } else {
         add((size_t)n * ldw * sizeof(float));           // W
         add((size_t)nblk * kNB * kNB * sizeof(float));  // diagonal-block inverses
         if (prec == RC_PREC_BF16) {
             add((size_t)n * ((ow + 63) / 64 * 64) * 2);  // BF16 outer panels (two)
             add((size_t)n * ((ow + 63) / 64 * 64) * 2);
-            add((size_t)n * kNB * 2);                    // BF16 128-column block
         }
         const size_t chunked = (size_t)ldw * ((nrhs + RHS - 1) / RHS) * RHS;  // 64-column chunks, ld ldw
         add(chunked * sizeof(float));                    // FP32 right-hand side of the preconditioner
@@ -717,20 +715,23 @@ int mixed_workspace_bytes(int64_t n, int64_t nrhs, int prec, int outer, size_t* 
 
 namespace {
 
-// One high-priority non-blocking stream per device for the factorisation's look-ahead
-// (kept for the life of the process).
-cudaStream_t lookahead_stream() {
-    static cudaStream_t streams[64] = {};
+// Two high-priority non-blocking streams per device for the factorisation's look-ahead (kept for
+// the life of the process): 0 its products, 1 the chain of its diagonal blocks.
+cudaStream_t lookahead_stream(int which = 0) {
+    static cudaStream_t streams[2][64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    if (!streams[dev]) {
+    if (!streams[which][dev]) {
         int lo = 0, hi = 0;
         if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess) return nullptr;
         cudaStream_t st = nullptr;
-        if (cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, hi) != cudaSuccess) return nullptr;
-        streams[dev] = st;
+        // A diagonal block needs a whole SM's shared memory, which it gets only ahead of the look-ahead's
+        // other kernels.
+        const int priority = which == 0 && hi + 1 < lo ? hi + 1 : hi;
+        if (cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, priority) != cudaSuccess) return nullptr;
+        streams[which][dev] = st;
     }
-    return streams[dev];
+    return streams[which][dev];
 }
 
 struct Mixed {
@@ -742,7 +743,6 @@ struct Mixed {
     float* W;
     float* Winv;
     void* Pb[2];  // BF16 outer panels, alternating
-    void* Pi;     // BF16 128-column block of the panel steps
     int64_t ldpb;
     double* sc;
     double* colsum;
@@ -760,7 +760,7 @@ struct Mixed {
     bool use_oz = false;
     int* errw = nullptr;  // the library's device error word (a timed-out wait sets it)
     // RC_PREC_EMU64: the FP64 working copy, its FP64 diagonal-block inverses (row-major),
-    // the digit splits of two outer panels and the TRSM tile buffer of the preconditioner.
+    // and the digit splits of two outer panels.
     double* W64 = nullptr;
     double* Winv64 = nullptr;
     void* Pe[2] = {nullptr, nullptr};
@@ -769,26 +769,83 @@ struct Mixed {
     View<float> Wv() const { return {W, ldw, 1}; }
     View<double> W64v() const { return {W64, ldw, 1}; }
 
-    // The 128-column steps of one outer panel [k0, k0 + w) of the FP64 working copy, on
-    // stream st: factor (and invert, row-major) the diagonal block, solve the rows below it
-    // in place with that inverse on the 128 x 128 FP64 DMMA tile (one CTA owns every column
-    // of a row block), update the rest of the panel's columns in FP64.
-    int panel_chain64(int64_t k0, int64_t w, int* info, cudaStream_t st) {
-        const View<double> Wm = W64v();
-        for (int64_t j0 = k0; j0 < k0 + w; j0 += kNB) {
-            const int jb = (int)((k0 + w - j0) < kNB ? k0 + w - j0 : kNB);
-            double* Wb = Winv64 + (size_t)(j0 / kNB) * kNB * kNB;
-            RC_TRY(potrf_diag_block<double>(Wm.sub(j0, j0), jb, j0, Wb, true, info, st));
-            const int64_t rows = n - j0 - jb;
-            if (rows <= 0) continue;
-            const View<double> Pj = Wm.sub(j0 + jb, j0);
-            const View<const double> Pc = {Pj.p, Pj.rs, Pj.cs};
-            RC_TRY(gemm<double>(rows, jb, jb, 1.0, Pc, View<const double>{Wb, 1, kNB}, 0.0, Pj, kFull, 0, st, info));
-            const int64_t cw = k0 + w - (j0 + jb);
-            if (cw <= 0) continue;
-            RC_TRY(gemm<double>(rows, cw, jb, -1.0, Pc, Pc.t(), 1.0, Wm.sub(j0 + jb, j0 + jb), kLower, 0, st, info));
+    // Events of a factorisation's streams, destroyed with it.
+    struct Events {
+        cudaEvent_t fork = nullptr, packed = nullptr, t2 = nullptr, join = nullptr;
+        cudaEvent_t diag = nullptr, next = nullptr, updated = nullptr;  // panel_steps
+        int create() {
+            for (cudaEvent_t* e : {&fork, &packed, &t2, &join, &diag, &next, &updated})
+                if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return RC_ERR_CUDA;
+            return RC_SUCCESS;
+        }
+        ~Events() {
+            for (cudaEvent_t e : {fork, packed, t2, join, diag, next, updated})
+                if (e) cudaEventDestroy(e);
+        }
+    };
+
+    // The 128-column steps of one outer panel [k0, k0 + w), left-looking, on two streams. On dg the
+    // dependent chain: the diagonal block's factor and inverse, the solve of the next block's rows
+    // alone and the update of that block's diagonal. On la, beside the diagonal block's factor: the
+    // block column's update by the panel's columns before it, then the solve of the rows below.
+    //   dg: diag(j) -> rec(diag) -> wait(updated(j)) -> solve(j, next block) -> rec(next) -> update(diagonal j + 1)
+    //   la: wait(next(j - 1)) -> update(j, below) -> rec(updated) -> wait(diag) -> solve(j, rows below the next block)
+    // la has waited for all of dg's work at the end.
+    // On one stream, right-looking, a step was the sum of its parts, 45 us of them the diagonal
+    // block: solve n = 32768 80.7 -> 78.0 ms, emulated-FP64 solve n = 16384 37.9 -> 36.3.
+    // (Right-looking on two streams: half of that, its updates rewrite the panel at 2 TB/s.)
+    // diag(j0, jb, st), solve(row, j0, jb, rows, st), update(row, col, k columns, rows, cols, st) with the
+    // panel's first k columns: see panel_chain.
+    template <class Diag, class Solve, class Update>
+    int panel_steps(int64_t k0, int64_t w, cudaStream_t la, const Events& ev, Diag diag, Solve solve, Update update) {
+        cudaStream_t dg = lookahead_stream(1);
+        if (!dg) return RC_ERR_CUDA;
+        auto ok = [](cudaError_t e) { return e == cudaSuccess ? RC_SUCCESS : RC_ERR_CUDA; };
+        const int64_t end = k0 + w;
+        RC_TRY(ok(cudaEventRecord(ev.updated, la)));
+        RC_TRY(ok(cudaStreamWaitEvent(dg, ev.updated, 0)));
+        for (int64_t j0 = k0; j0 < end; j0 += kNB) {
+            const int jb = (int)(end - j0 < kNB ? end - j0 : kNB);
+            const int64_t j1 = j0 + jb;                                        // the next block
+            const int64_t nx = end - j1 < kNB ? end - j1 : kNB, j2 = j1 + nx;  // its width; the rows below it
+            RC_TRY(diag(j0, jb, dg));
+            RC_TRY(ok(cudaEventRecord(ev.diag, dg)));
+            if (j0 > k0) {
+                RC_TRY(ok(cudaStreamWaitEvent(la, ev.next, 0)));
+                if (n > j1) RC_TRY(update(j1, j0, j0 - k0, n - j1, jb, la));
+                RC_TRY(ok(cudaEventRecord(ev.updated, la)));
+            }
+            RC_TRY(ok(cudaStreamWaitEvent(la, ev.diag, 0)));
+            if (n > j2) RC_TRY(solve(j2, j0, jb, n - j2, la));
+            if (nx == 0) continue;
+            RC_TRY(ok(cudaStreamWaitEvent(dg, ev.updated, 0)));
+            RC_TRY(solve(j1, j0, jb, nx, dg));
+            RC_TRY(ok(cudaEventRecord(ev.next, dg)));
+            RC_TRY(update(j1, j1, j1 - k0, nx, nx, dg));
         }
         return RC_SUCCESS;
+    }
+
+    // panel_steps on the FP64 working copy: the solves in place on a DMMA tile that owns its rows'
+    // 128 columns, the updates in FP64.
+    int panel_chain64(int64_t k0, int64_t w, int* info, cudaStream_t la, const Events& ev) {
+        const View<double> Wm = W64v();
+        auto inv = [&](int64_t j0) { return Winv64 + (size_t)(j0 / kNB) * kNB * kNB; };
+        auto C_ = [](const View<double>& v) { return View<const double>{v.p, v.rs, v.cs}; };
+        return panel_steps(
+            k0, w, la, ev,
+            [&](int64_t j0, int jb, cudaStream_t st) {
+                return potrf_diag_block<double>(Wm.sub(j0, j0), jb, j0, inv(j0), true, info, st);
+            },
+            [&](int64_t r, int64_t j0, int jb, int64_t rows, cudaStream_t st) {
+                const View<double> P = Wm.sub(r, j0);
+                return gemm<double>(rows, jb, jb, 1.0, C_(P), View<const double>{inv(j0), 1, kNB}, 0.0, P, kFull, 0, st,
+                                    info);
+            },
+            [&](int64_t r, int64_t c, int64_t k, int64_t rows, int64_t cols, cudaStream_t st) {
+                return gemm<double>(rows, cols, k, -1.0, C_(Wm.sub(r, k0)), C_(Wm.sub(c, k0)).t(), 1.0, Wm.sub(r, c),
+                                    r == c ? kLower : kFull, 0, st, info);
+            });
     }
 
     // The look-ahead schedule of factor() with an FP64 working copy: each factored outer
@@ -799,20 +856,12 @@ struct Mixed {
     int factor_emu(int outer, int* info) {
         cudaStream_t la = lookahead_stream();
         if (!la) return RC_ERR_CUDA;
-        cudaEvent_t ev_fork, ev_packed, ev_t2, ev_join;
-        if (cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_packed, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_t2, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)
-            return RC_ERR_CUDA;
-        struct Events {
-            cudaEvent_t e[4];
-            ~Events() { for (cudaEvent_t x : e) cudaEventDestroy(x); }
-        } guard{{ev_fork, ev_packed, ev_t2, ev_join}};
+        Events ev;
+        RC_TRY(ev.create());
         auto ok = [](cudaError_t e) { return e == cudaSuccess ? RC_SUCCESS : RC_ERR_CUDA; };
-        RC_TRY(ok(cudaEventRecord(ev_fork, s)));
-        RC_TRY(ok(cudaStreamWaitEvent(la, ev_fork, 0)));
-        RC_TRY(panel_chain64(0, n < outer ? n : outer, info, la));
+        RC_TRY(ok(cudaEventRecord(ev.fork, s)));
+        RC_TRY(ok(cudaStreamWaitEvent(la, ev.fork, 0)));
+        RC_TRY(panel_chain64(0, n < outer ? n : outer, info, la, ev));
         bool t2_pending = false;
         for (int64_t p = 0, k0 = 0; k0 < n; ++p, k0 += outer) {
             const int64_t w = (n - k0 < outer) ? n - k0 : outer;
@@ -821,26 +870,26 @@ struct Mixed {
             EmuPanel& pn = pe[p & 1];
             RC_TRY(emu_panel_layout(rows, w, Pe[p & 1], &pn));
             RC_TRY(emu_slice_panel(pn, W64 + k1 * ldw + k0, ldw, la));
-            RC_TRY(ok(cudaEventRecord(ev_packed, la)));
-            if (t2_pending) RC_TRY(ok(cudaStreamWaitEvent(la, ev_t2, 0)));
+            RC_TRY(ok(cudaEventRecord(ev.packed, la)));
+            if (t2_pending) RC_TRY(ok(cudaStreamWaitEvent(la, ev.t2, 0)));
             const int64_t w1 = rows < outer ? rows : outer;  // width of panel p + 1
             // T1: rows [k1, n) x columns [k1, k1 + w1) on the look-ahead stream
             RC_TRY(emu_update(pn, 0, 0, rows, w1, -1.0, 1.0, W64 + k1 * ldw + k1, ldw, true, la, info));
             // T2: rows and columns [k1 + w1, n) on the main stream
             const int64_t r2 = rows - w1;
             if (r2 > 0) {
-                RC_TRY(ok(cudaStreamWaitEvent(s, ev_packed, 0)));
+                RC_TRY(ok(cudaStreamWaitEvent(s, ev.packed, 0)));
                 RC_TRY(emu_update(pn, w1, w1, r2, r2, -1.0, 1.0, W64 + (k1 + w1) * ldw + (k1 + w1), ldw, true, s,
                                   info));
-                RC_TRY(ok(cudaEventRecord(ev_t2, s)));
+                RC_TRY(ok(cudaEventRecord(ev.t2, s)));
                 t2_pending = true;
             } else {
                 t2_pending = false;
             }
-            RC_TRY(panel_chain64(k1, w1, info, la));
+            RC_TRY(panel_chain64(k1, w1, info, la, ev));
         }
-        RC_TRY(ok(cudaEventRecord(ev_join, la)));
-        return ok(cudaStreamWaitEvent(s, ev_join, 0));
+        RC_TRY(ok(cudaEventRecord(ev.join, la)));
+        return ok(cudaStreamWaitEvent(s, ev.join, 0));
     }
 
     // Zout = M^-1 Rin = S L^-T L^-1 S Rin, all in FP64, on st: block forward and backward
@@ -856,33 +905,25 @@ struct Mixed {
         return check_launch();
     }
 
-    // The 128-column steps of one outer panel [k0, k0 + w), on stream st: factor (and
-    // invert) the diagonal block in FP64, solve the rows below it with that inverse on the
-    // TF32 tensor cores, update the rest of the panel's columns.
-    int panel_chain(int64_t k0, int64_t w, int* info, cudaStream_t st) {
+    // panel_steps on the FP32 working copy: the diagonal block in FP64, solves and updates on the
+    // tcgen05 kernels in TF32 (bound by memory, so BF16 would gain nothing here).
+    int panel_chain(int64_t k0, int64_t w, int* info, cudaStream_t la, const Events& ev) {
         const View<float> Wm = Wv();
-        for (int64_t j0 = k0; j0 < k0 + w; j0 += kNB) {
-            const int jb = (int)((k0 + w - j0) < kNB ? k0 + w - j0 : kNB);
-            float* Wb = Winv + (size_t)(j0 / kNB) * kNB * kNB;
-            RC_TRY(potrf_diag_block<float>(Wm.sub(j0, j0), jb, j0, Wb, true, info, st));
-            const int64_t rows = n - j0 - jb;
-            if (rows <= 0) continue;
-            View<float> Pj = Wm.sub(j0 + jb, j0);
-            // Panel solve in place: P <- P inv(L_jj)^T (TF32 tensor cores, one column tile).
-            RC_TRY(gemm_tc_kmajor(false, rows, jb, jb, 1.f, Pj.p, ldw, Wb, kNB, 0.f, Pj, kFull, 0, st, info, 128));
-            const int64_t cw = k0 + w - (j0 + jb);
-            if (cw <= 0) continue;
-            const void* op = Pj.p;
-            int64_t ldo = ldw;
-            if (prec == RC_PREC_BF16) {
-                RC_TRY(pack_kmajor(rows, jb, View<const float>{Pj.p, Pj.rs, Pj.cs}, Pi, kNB, true, st));
-                op = Pi;
-                ldo = kNB;
-            }
-            RC_TRY(gemm_tc_kmajor(prec == RC_PREC_BF16, rows, cw, jb, -1.f, op, ldo, op, ldo, 1.f,
-                                  Wm.sub(j0 + jb, j0 + jb), kLower, 0, st, info));
-        }
-        return RC_SUCCESS;
+        auto inv = [&](int64_t j0) { return Winv + (size_t)(j0 / kNB) * kNB * kNB; };
+        return panel_steps(
+            k0, w, la, ev,
+            [&](int64_t j0, int jb, cudaStream_t st) {
+                return potrf_diag_block<float>(Wm.sub(j0, j0), jb, j0, inv(j0), true, info, st);
+            },
+            [&](int64_t r, int64_t j0, int jb, int64_t rows, cudaStream_t st) {
+                // in place: P <- P inv(L_jj)^T, one column tile
+                const View<float> P = Wm.sub(r, j0);
+                return gemm_tc_kmajor(false, rows, jb, jb, 1.f, P.p, ldw, inv(j0), kNB, 0.f, P, kFull, 0, st, info, 128);
+            },
+            [&](int64_t r, int64_t c, int64_t k, int64_t rows, int64_t cols, cudaStream_t st) {
+                return gemm_tc_kmajor(false, rows, cols, k, -1.f, Wm.sub(r, k0).p, ldw, Wm.sub(c, k0).p, ldw, 1.f,
+                                      Wm.sub(r, c), r == c ? kLower : kFull, 0, st, info);
+            });
     }
 
     // Blocked right-looking factorisation with a look-ahead of one outer panel. With panel
@@ -898,20 +939,12 @@ struct Mixed {
         const View<float> Wm = Wv();
         cudaStream_t la = lookahead_stream();
         if (!la) return RC_ERR_CUDA;
-        cudaEvent_t ev_fork, ev_packed, ev_t2, ev_join;
-        if (cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_packed, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_t2, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess)
-            return RC_ERR_CUDA;
-        struct Events {
-            cudaEvent_t e[4];
-            ~Events() { for (cudaEvent_t x : e) cudaEventDestroy(x); }
-        } guard{{ev_fork, ev_packed, ev_t2, ev_join}};
+        Events ev;
+        RC_TRY(ev.create());
         auto ok = [](cudaError_t e) { return e == cudaSuccess ? RC_SUCCESS : RC_ERR_CUDA; };
-        RC_TRY(ok(cudaEventRecord(ev_fork, s)));
-        RC_TRY(ok(cudaStreamWaitEvent(la, ev_fork, 0)));
-        RC_TRY(panel_chain(0, n < outer ? n : outer, info, la));
+        RC_TRY(ok(cudaEventRecord(ev.fork, s)));
+        RC_TRY(ok(cudaStreamWaitEvent(la, ev.fork, 0)));
+        RC_TRY(panel_chain(0, n < outer ? n : outer, info, la, ev));
         bool t2_pending = false;
         for (int64_t p = 0, k0 = 0; k0 < n; ++p, k0 += outer) {
             const int64_t w = (n - k0 < outer) ? n - k0 : outer;
@@ -926,8 +959,8 @@ struct Mixed {
                 ldo = ldpb;
                 RC_TRY(pack_kmajor(rows, w, View<const float>{Pk.p, Pk.rs, Pk.cs}, Pb[p & 1], ldpb, true, la));
             }
-            RC_TRY(ok(cudaEventRecord(ev_packed, la)));
-            if (t2_pending) RC_TRY(ok(cudaStreamWaitEvent(la, ev_t2, 0)));
+            RC_TRY(ok(cudaEventRecord(ev.packed, la)));
+            if (t2_pending) RC_TRY(ok(cudaStreamWaitEvent(la, ev.t2, 0)));
             const int64_t w1 = rows < outer ? rows : outer;  // width of panel p + 1
             // T1: rows [k1, n) x columns [k1, k1 + w1) on the look-ahead stream
             RC_TRY(gemm_tc_kmajor(bf16, rows, w1, w, -1.f, op, ldo, op, ldo, 1.f, Wm.sub(k1, k1), kLower, 0, la, info));
@@ -936,19 +969,19 @@ struct Mixed {
             if (r2 > 0) {
                 const size_t esz = bf16 ? 2 : 4;
                 const void* op2 = static_cast<const char*>(op) + (size_t)w1 * ldo * esz;
-                RC_TRY(ok(cudaStreamWaitEvent(s, ev_packed, 0)));
+                RC_TRY(ok(cudaStreamWaitEvent(s, ev.packed, 0)));
                 // Two SMs stay free of pair CTAs for the look-ahead's diagonal blocks.
                 RC_TRY(gemm_tc_pair_kmajor(bf16, r2, r2, w, -1.f, op2, ldo, op2, ldo, 1.f, Wm.sub(k1 + w1, k1 + w1),
                                            kLower, 0, s, info, 2, true));
-                RC_TRY(ok(cudaEventRecord(ev_t2, s)));
+                RC_TRY(ok(cudaEventRecord(ev.t2, s)));
                 t2_pending = true;
             } else {
                 t2_pending = false;
             }
-            RC_TRY(panel_chain(k1, w1, info, la));
+            RC_TRY(panel_chain(k1, w1, info, la, ev));
         }
-        RC_TRY(ok(cudaEventRecord(ev_join, la)));
-        return ok(cudaStreamWaitEvent(s, ev_join, 0));
+        RC_TRY(ok(cudaEventRecord(ev.join, la)));
+        return ok(cudaStreamWaitEvent(s, ev.join, 0));
     }
 
     // Zout = M^-1 Rin = S L^-T L^-1 S Rin (FP64 in/out, FP32 triangular solves), on st.
@@ -1125,7 +1158,7 @@ int spd_solve_mixed(int prec, int64_t n, int64_t nrhs, const double* A, int64_t 
     M.ldpb = (o.outer + 63) / 64 * 64;
     M.W = nullptr;
     M.Winv = M.T32 = M.T32b = M.T32s = M.tmp = M.Y = M.Tinv = nullptr;
-    M.Pb[0] = M.Pb[1] = M.Pi = nullptr;
+    M.Pb[0] = M.Pb[1] = nullptr;
     if (emu) {
         M.W64 = buf.take<double>((size_t)n * M.ldw);
         M.Winv64 = buf.take<double>((size_t)M.nblk * kNB * kNB);
@@ -1135,7 +1168,6 @@ int spd_solve_mixed(int prec, int64_t n, int64_t nrhs, const double* A, int64_t 
         M.Winv = buf.take<float>((size_t)M.nblk * kNB * kNB);
         for (int q = 0; q < 2; ++q)
             M.Pb[q] = prec == RC_PREC_BF16 ? static_cast<void*>(buf.take<uint16_t>((size_t)n * M.ldpb)) : nullptr;
-        M.Pi = prec == RC_PREC_BF16 ? static_cast<void*>(buf.take<uint16_t>((size_t)n * kNB)) : nullptr;
         M.T32 = buf.take<float>((size_t)M.ldv * ((nrhs + RHS - 1) / RHS) * RHS);
         M.T32b = buf.take<float>((size_t)M.ldv * ((nrhs + RHS - 1) / RHS) * RHS);
         M.T32s = buf.take<float>((size_t)M.ldv * 2 * RHS);
