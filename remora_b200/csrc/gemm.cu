@@ -537,7 +537,9 @@ int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const d
                 View<double> C, int64_t off, int nz, cudaStream_t s, const int* abort) {
     constexpr size_t smem = dmma_smem<AK, BK, Tile>();
     auto kernel = gemm_dmma_f64<AK, BK, Tile, V16>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    // 48 KB need no leave; the call is a share of a small product's time
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return RC_ERR_CUDA;
     dim3 grid(ceil_div(p.n, Tile::BN), ceil_div(p.m, Tile::BM));
     if (nz > 1) {

@@ -32,19 +32,22 @@ from ._lib import call, key_array
 _FP = {torch.float64: "f64", torch.float32: "f32"}
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+# Pointers and streams go to the C-ABI as plain integers and the stream is asked for without a
+# Stream object: a small product's time is its call (12.4 -> 8.2 us for 61 x 37 x 53).
+def _stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
-def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
 
 
 def layout(X: torch.Tensor) -> tuple[int, int]:
     """(trans, ld) with X = op_trans(M), M column-major with leading dimension ld."""
-    if X.dim() != 2:
+    shape = X.shape
+    if len(shape) != 2:
         raise ValueError("expected a matrix")
-    r, c = X.shape
+    r, c = shape
     s0, s1 = X.stride()
     if s0 == 1 and (c <= 1 or s1 >= max(r, 1)):
         return 0, max(s1 if c > 1 else r, 1)
@@ -59,9 +62,13 @@ def is_row_major(X: torch.Tensor) -> bool:
 
 def _sfx(*ts: torch.Tensor) -> str:
     dt = ts[0].dtype
-    if any(t.dtype != dt for t in ts) or dt not in _FP:
+    sfx = _FP.get(dt)
+    for t in ts:
+        if t.dtype != dt:
+            sfx = None
+    if sfx is None:
         raise TypeError("arguments must share one element type, float32 or float64")
-    return _FP[dt]
+    return sfx
 
 
 def gemm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, alpha: float = 1.0, beta: float = 1.0,
