@@ -117,12 +117,12 @@ int trsm_backward(bool trans, int64_t n, int64_t nrhs, View<const double> L, Vie
     return gemm<double>(n, n, nrhs, -1.0, X, Bb.t(), 1.0, Lbar, kLower, 0, s);
 }
 
-// 1/2 (L^-T L^-1 - a a^T): the inverse is built in row panels of kPanel, X = L^-1, and each
-// finished panel is added to L^-T L^-1 at once. Columns right of a panel's diagonal block are
-// zero and never touched, so both products together do 2/3 n^3 operations; through the adjoint
-// of the factorisation (one masked product, two triangular solves with n columns) they were
-// 3 n^3. Likelihood and gradient at n = 8192, d = 16: 90.2 -> 27.5 ms, and Kbar's error against
-// a 64-bit library result 7.2e-15 -> 2.5e-15.
+// 1/2 (L^-T L^-1 - a a^T): the inverse X = L^-1 is built in row panels of kPanel, whose columns
+// right of the diagonal block are zero and never touched, and multiplied by itself from each
+// tile's diagonal on: 2/3 n^3 operations; through the adjoint of the factorisation (one masked
+// product, two triangular solves with n columns) they were 3 n^3. Likelihood and gradient at
+// n = 8192, d = 16: 90.2 -> 26.4 ms (27.5 with X^T X a panel at a time), and Kbar's error against a 64-bit
+// library result 7.2e-15 -> 3.1e-15.
 int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> Kbar, cudaStream_t s) {
     if (n <= 0) return RC_SUCCESS;
     constexpr int64_t kPanel = kStripRows;  // trailing updates as deep as the factorisation's
@@ -131,10 +131,7 @@ int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> K
     if (!w || !W) return RC_ERR_ALLOC;
     const View<double> X = colmajor(w, n);
     auto C_ = [](const View<double>& v) { return View<const double>{v.p, v.rs, v.cs}; };
-    if (cudaMemsetAsync(w, 0, (size_t)n * n * sizeof(double), s) != cudaSuccess ||
-        cudaMemset2DAsync(Kbar.p, (size_t)Kbar.cs * sizeof(double), 0, (size_t)n * sizeof(double), (size_t)n, s) !=
-            cudaSuccess)
-        return RC_ERR_CUDA;
+    if (cudaMemsetAsync(w, 0, (size_t)n * n * sizeof(double), s) != cudaSuccess) return RC_ERR_CUDA;
     identity_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, X);
     RC_TRY(check_launch());
     RC_TRY(trtri_blocks_launch<double>(n, L, false, W, nullptr, nullptr, s));
@@ -142,10 +139,10 @@ int nll_adjoint(int64_t n, View<const double> L, const double* a, View<double> K
         const int64_t pe = n - p < kPanel ? n : p + kPanel;
         RC_TRY(strip_solve<double>(false, pe - p, pe, L.sub(p, p), W + p * kNB, false, X.sub(p, 0), s, nullptr));
         const View<const double> Xp = C_(X.sub(p, 0));
-        RC_TRY(gemm<double>(pe, pe, pe - p, 0.5, Xp.t(), Xp, 1.0, Kbar, kLower, 0, s));
         if (pe < n)
             RC_TRY(gemm<double>(n - pe, pe, pe - p, -1.0, L.sub(pe, p), Xp, 1.0, X.sub(pe, 0), kFull, 0, s));
     }
+    RC_TRY(gemm<double>(n, n, n, 0.5, C_(X).t(), C_(X), 0.0, Kbar, kLowerTri, 0, s));
     const unsigned nt = ceil_div(n, 32);
     nll_adjoint_kernel<<<dim3(nt, nt), 256, 0, s>>>(n, a, Kbar);
     return check_launch();

@@ -408,7 +408,14 @@ __global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
     const int64_t first = lin / per * kGroupM, rest = (int64_t)gridDim.y - first;
     const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
     const int64_t m0 = (first + r % gsz) * BM, n0 = r / gsz * BN;
+    const bool tri = mask == kLowerTri;
+    if (tri) mask = kLower;
     if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
+    if (tri && m0 < k) {
+        A = A.sub(0, m0);
+        B = B.sub(m0, 0);
+        k -= m0;
+    }
     if (gridDim.z > 1) {  // K slice of a split-K product
         const int64_t kz = (int64_t)blockIdx.z * kchunk;
         A = A.sub(0, kz);
@@ -668,9 +675,10 @@ __global__ void scale_masked(int64_t m, int64_t n, T beta, View<T> C, Mask mask,
 }  // namespace
 
 template <class T>
-int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T> B, T beta, View<T> C, Mask mask,
+int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T> B, T beta, View<T> C, Mask asked,
          int64_t off, cudaStream_t s, const int* abort) {
     if (m <= 0 || n <= 0) return RC_SUCCESS;
+    const Mask mask = asked == kLowerTri ? kLower : asked;  // of the kernels that multiply the zeros
     if (k <= 0 || alpha == T(0)) {
         if (beta == T(1)) return RC_SUCCESS;
         dim3 grid(ceil_div(m, 256) < 1024u ? ceil_div(m, 256) : 1024u, n < 65535 ? (unsigned)n : 65535u);
@@ -681,7 +689,7 @@ int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T
     if ((a_k || a_m) && (b_k || b_n)) {
         auto run = [&](auto ak, auto bk) {
             if constexpr (std::is_same<T, double>::value)
-                return gemm_dmma<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+                return gemm_dmma<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, asked, off, s, abort);
             else
                 return sgemm<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
         };

@@ -7,7 +7,9 @@ namespace rc {
 // Which part of C a (masked) GEMM may write: kFull writes every element; kLower writes
 // C(i, j) only when i - j >= off; kUpper only when i - j <= off. Tiles that lie entirely
 // outside the mask are skipped, which turns a masked GEMM into SYRK's triangle schedule.
-enum Mask { kFull = 0, kLower = 1, kUpper = 2 };
+// kLowerTri is kLower with off = 0 for an A that is upper triangular (A(i, k) = 0 for k < i):
+// the FP64 tiles leave out the k before their first row.
+enum Mask { kFull = 0, kLower = 1, kUpper = 2, kLowerTri = 3 };
 
 // C <- alpha * A * B + beta * C (A m x k, B k x n, C m x n, arbitrary strided views).
 // beta == 0 does not read C. abort (device int, may be null): when *abort != 0 at launch
