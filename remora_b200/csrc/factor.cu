@@ -17,7 +17,6 @@
 #include "diag.cuh"
 #include "gemm.cuh"
 #include "strip.cuh"
-#include <type_traits>
 
 namespace rc {
 namespace {
@@ -472,20 +471,12 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s, T* Winv) {
     if (cudaMemsetAsync(info, 0, sizeof(int), s) != cudaSuccess) return RC_ERR_CUDA;
     if (n <= 0) return RC_SUCCESS;
     // Outer panels of kOuter columns: 128-column steps factor the panel's diagonal block, the rows
-    // below it are solved a strip per CTA, and the trailing matrix gets one update of depth
-    // kOuter. SPD solve n = 1024, 16 right-hand sides: 730 -> 595 us; FP32 factor and solves
-    // n = 3001: 3.09 -> 2.48 ms.
+    // below it are solved a strip per CTA (and so are those of a step inside the block), and the
+    // trailing matrix gets one update of depth kOuter. SPD solve n = 1024, 16 right-hand sides:
+    // 730 -> 568 us; FP32 factor and solves n = 3001: 3.09 -> 2.38 ms.
     constexpr int64_t kOuter = kStripRows;
     T* own = Winv ? nullptr : static_cast<T*>(workspace(s, (size_t)kOuter * NB * sizeof(T), 1));
     if (!Winv && !own) return RC_ERR_ALLOC;
-    // An in-place FP64 product runs on a DMMA tile that spans the step's 128 columns, so one
-    // CTA owns every column of its rows; other types go through a buffer.
-    constexpr bool in_place = std::is_same<T, double>::value;
-    T* tmp = nullptr;
-    if (!in_place) {
-        tmp = static_cast<T*>(workspace(s, (size_t)kOuter * NB * sizeof(T), 2));
-        if (!tmp) return RC_ERR_ALLOC;
-    }
     RC_TRY(set_smem(potrf_diag<T>, kDiagSmem));
     auto C_ = [](const View<T>& v) { return View<const T>{v.p, v.rs, v.cs}; };
     for (int64_t k0 = 0; k0 < n; k0 += kOuter) {
@@ -494,19 +485,12 @@ int potrf_lower(int64_t n, View<T> A, int* info, cudaStream_t s, T* Winv) {
         for (int64_t j0 = k0; j0 < end; j0 += NB) {
             const int jb = (int)(end - j0 < NB ? end - j0 : NB);
             T* W = Wp + (j0 - k0) * NB;
-            const View<const T> Wt = {W, NB, 1};  // inv(L_jj)^T
             potrf_diag<T><<<1, kDiagThreads, kDiagSmem, s>>>(A.sub(j0, j0), jb, j0, W, info, false);
             RC_TRY(check_launch());
             const int64_t rows = end - j0 - jb;
             if (rows <= 0) continue;
-            View<T> P = A.sub(j0 + jb, j0);
-            if (in_place) {
-                RC_TRY(gemm<T>(rows, jb, jb, T(1), C_(P), Wt, T(0), P, kFull, 0, s, info));
-            } else {
-                const View<T> Tv = colmajor(tmp, rows);
-                RC_TRY(gemm<T>(rows, jb, jb, T(1), C_(P), Wt, T(0), Tv, kFull, 0, s, info));
-                RC_TRY(copy2d<T, T>(rows, jb, T(1), C_(Tv), P, s, info));
-            }
+            const View<T> P = A.sub(j0 + jb, j0);
+            RC_TRY(strip_solve<T>(false, jb, rows, C_(A.sub(j0, j0)), W, false, P.t(), s, info));
             RC_TRY(gemm<T>(rows, rows, jb, T(-1), C_(P), C_(P).t(), T(1), A.sub(j0 + jb, j0 + jb), kLower, 0, s,
                            info));
         }

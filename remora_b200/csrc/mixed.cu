@@ -9,9 +9,9 @@
 //     ill-conditioned A (Higham & Pranesh 2021, diagonal scaling + shift).
 //  2. Factor W = L L^T, blocked right-looking: outer panels of `outer` columns, inner
 //     128-column blocks whose diagonal block is factored (and inverted) in FP64 shared
-//     memory; the panel below is solved with that inverse on the TF32 tensor cores; the
-//     updates inside the panel and the trailing update run on the tcgen05 tensor cores in
-//     TF32 or BF16 with FP32 accumulation (BF16 operands are packed per panel).
+//     memory; the panel below is solved with that inverse and updated inside the panel on
+//     the TF32 tensor cores; the trailing update runs on the tcgen05 tensor cores in TF32
+//     or BF16 with FP32 accumulation (BF16 operands are packed per panel).
 //  3. Refine in FP64: x0 = M^-1 b with M = S^-1 L L^T S^-1, then preconditioned conjugate
 //     gradients on A (FP64 vectors, the FP32 factor as preconditioner), one independent
 //     CG recurrence per right-hand side. The CG products A p and the starting residual
@@ -38,6 +38,7 @@
 #include "mixed.cuh"
 #include "ozaki.cuh"
 #include "ozaki_digits.cuh"
+#include "strip.cuh"
 #include "tc_gemm.cuh"
 
 namespace cg = cooperative_groups;
@@ -839,6 +840,8 @@ struct Mixed {
             },
             [&](int64_t r, int64_t j0, int jb, int64_t rows, cudaStream_t st) {
                 const View<double> P = Wm.sub(r, j0);
+                if (rows <= kNB)  // the next block's, on the chain: 16 small CTAs
+                    return strip_solve<double>(false, jb, rows, C_(Wm.sub(j0, j0)), inv(j0), true, P.t(), st, info);
                 return gemm<double>(rows, jb, jb, 1.0, C_(P), View<const double>{inv(j0), 1, kNB}, 0.0, P, kFull, 0, st,
                                     info);
             },
