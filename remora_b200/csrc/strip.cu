@@ -177,14 +177,14 @@ __global__ void __launch_bounds__(kStripThreads, 1)
 template <class T, int COLS, bool AKM, bool WKM>
 int launch_strip(bool upper, int64_t m, int64_t n, View<const T> A, const T* W, View<T> B, cudaStream_t s,
                  const int* abort) {
-    const int64_t rows = (m + SB - 1) / SB * SB;
-    const size_t smem = (size_t)(rows + SB) * (COLS + 2) * sizeof(double);
+    auto smem = [](int64_t rows) { return (size_t)(rows + SB) * (COLS + 2) * sizeof(double); };
+    // always the limit of the tallest panel: threads and captured launches share the attribute
     if (cudaFuncSetAttribute(strip_kernel<T, COLS, AKM, WKM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
+                             (int)smem(kStripRows)) != cudaSuccess)
         return RC_ERR_CUDA;
     const bool vec = reinterpret_cast<uintptr_t>(A.p) % (2 * sizeof(T)) == 0 && (AKM ? A.rs : A.cs) % 2 == 0;
-    strip_kernel<T, COLS, AKM, WKM><<<ceil_div(n, COLS), kStripThreads, smem, s>>>(upper, (int)m, n, A, W, B, vec,
-                                                                                   abort);
+    strip_kernel<T, COLS, AKM, WKM><<<ceil_div(n, COLS), kStripThreads, smem((m + SB - 1) / SB * SB), s>>>(
+        upper, (int)m, n, A, W, B, vec, abort);
     return check_launch();
 }
 

@@ -46,3 +46,35 @@ def test_potrf_across_panels(cuda, dtype, n, row, pad):
     L = torch.tril(A).double()
     ref = torch.linalg.cholesky(S.double())
     assert torch.linalg.norm(L - ref) <= TOL[dtype] * torch.linalg.norm(ref)
+
+
+def test_threads_solve_panels_of_different_heights(cuda):
+    """Solves of 128 and of 512 rows from several host threads, each on a stream of its own."""
+    import threading
+
+    wrong = []
+
+    def work(m):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            g = torch.Generator(device="cuda").manual_seed(m)
+            A = torch.rand((m, m), generator=g, device="cuda", dtype=torch.float64)
+            A.diagonal().add_(m)
+            B = torch.rand((m, 8), generator=g, device="cuda", dtype=torch.float64)
+            ref = torch.linalg.solve_triangular(A, B, upper=False)
+            for _ in range(200):
+                X = B.clone()
+                try:
+                    ops.trsm(A, X)
+                except Exception as e:  # noqa: BLE001
+                    wrong.append(e)
+                    return
+            if not torch.linalg.norm(X - ref) <= 1e-13 * torch.linalg.norm(ref):
+                wrong.append(m)
+
+    threads = [threading.Thread(target=work, args=(m,)) for m in (128, 512, 256, 512)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
