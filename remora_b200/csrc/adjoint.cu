@@ -225,7 +225,7 @@ __device__ __forceinline__ void rbf_points(RbfShared& sh, int64_t n, int d, cons
     for (int e = threadIdx.x; e < 2 * kRbfTile * d; e += 256) {
         const int side = e / (kRbfTile * d), r = e % (kRbfTile * d) / d, q = e % d;
         const int64_t i = (side ? j0 : i0) + r;
-        sh.x[side][q][r] = i < n ? X[i * d + q] : 0.0;
+        sh.x[side][q][r] = X[(i < n ? i : n - 1) * d + q];  // beyond the end the last point, at weight 0
     }
 }
 

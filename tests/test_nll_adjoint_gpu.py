@@ -57,3 +57,14 @@ def test_rbf_matrix_and_gradient(cuda, n, d):
     terms = (Kbar * ref)[:, :, None] * (X[:, None, :] - X[None, :, :]) ** 2
     scale = np.abs(terms).sum((0, 1)) / np.abs(ls * ls * ls)
     assert np.all(np.abs(g.cpu().numpy() - terms.sum((0, 1)) / (ls * ls * ls)) <= 4 * U * (n * n + 200) * scale)
+
+
+def test_gradient_of_equal_points_far_out(cuda):
+    """Distances are zero wherever the points lie, also beside the unused part of a tile."""
+    X = torch.full((5, 2), 1e200, dtype=torch.float64, device="cuda")
+    ls, Kbar = torch.ones(2, dtype=torch.float64, device="cuda"), torch.ones((5, 5), dtype=torch.float64, device="cuda")
+    g = torch.empty(2, dtype=torch.float64, device="cuda")
+    call("rc_rbf_lengthscale_grad_f64", 5, 2, X.data_ptr(), ls.data_ptr(), Kbar.data_ptr(), 5, g.data_ptr(),
+         torch.cuda.current_stream().cuda_stream)
+    assert torch.all(g == 0)
+    assert torch.all(ops.rbf_kernel(X, ls, 0.0) == 1)
