@@ -341,9 +341,12 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // P (row stride kClLd). The panel is walked in 16-column strips, whose rows are in registers,
 // rotated so that a[0] is the column to eliminate. Per column every CTA sends its candidate
 // (largest |a[0]|, the lowest row among equals) and that row into every CTA's shared memory by
-// st.async and waits for theirs on its own mbarrier (two in turn, by the column's parity: what is
-// sent for a column is sent after its sender has read all of the column before last); then all
-// agree on the pivot, the two rows swap within the strip, and every row is divided and updated. Per strip, the swaps of the panel's other columns
+// st.async and waits for theirs on its own mbarrier. All that a column writes for other warps or
+// CTAs to read (the warps' candidates, their rows, row c, the exchanged keys and rows, the mbarrier)
+// exists twice, by the column's parity: a wait ends once one warp of every CTA has sent, so a warp may
+// be a column ahead of the others of its CTA, but not two, as the barrier between its candidate and
+// its sending lies in between; and what is sent for a column is sent after its reader has read all of
+// the column before last. Then all agree on the pivot, the two rows swap within the strip, and every row is divided and updated. Per strip, the swaps of the panel's other columns
 // (and of the strip's own finished ones) are gathered through distributed shared memory, the
 // strip's 16 rows of U are solved, and the columns to the right are updated on DMMA. Each element
 // sees the pivot, division and update order of getrf_panel_kernel, a strip's sixteen products
@@ -363,10 +366,10 @@ struct ClusterSmem {
     uint64_t bar[2];
     int late;                       // a wait ran out
     int from_all[2 * kStrip], from_strip[2 * kStrip][kStrip], dest[2 * kStrip];
-    T mine[8][kStrip], top[kStrip];  // the warps' candidate rows; row c
+    T mine[2][8][kStrip], top[2][kStrip];  // by column parity: the warps' candidate rows; row c
     T U[kStrip][kLuNB];
-    unsigned whi[8], wlo[8];
-    int widx[8];
+    unsigned whi[2][8], wlo[2][8];  // by column parity: the warps' candidates
+    int widx[2][8];
     int pivots[kStrip];
     // the inverse of L11 (read and written in pairs)
     alignas(16) double L[kLuNB * kClLd];
@@ -375,6 +378,7 @@ struct ClusterSmem {
     alignas(16) double T32[32 * 36];
     double rd[kLuNB];
 };
+static_assert(sizeof(ClusterSmem<double>) <= 227 * 1024, "a CTA's shared memory");
 
 // Largest (hi, lo), the smallest idx among equals, over a warp; lanes without a candidate have
 // hi = 0 and idx = INT_MAX.
@@ -480,30 +484,30 @@ __global__ void __launch_bounds__(kClThreads, 1)
             int idx = valid ? row : INT_MAX;
             warp_best(hi, lo, idx);
             if (lane == 0) {
-                sm.whi[warp] = hi;
-                sm.wlo[warp] = lo;
-                sm.widx[warp] = idx;
+                sm.whi[par][warp] = hi;
+                sm.wlo[par][warp] = lo;
+                sm.widx[par][warp] = idx;
             }
             if (row == idx) {
 #pragma unroll
-                for (int q = 0; q < kStrip; ++q) sm.mine[warp][q] = a[q];
+                for (int q = 0; q < kStrip; ++q) sm.mine[par][warp][q] = a[q];
             }
             if (row == c) {
 #pragma unroll
-                for (int q = 0; q < kStrip; ++q) sm.top[q] = a[q];
+                for (int q = 0; q < kStrip; ++q) sm.top[par][q] = a[q];
             }
             __syncthreads();
-            hi = lane < 8 ? sm.whi[lane] : 0u;
-            lo = lane < 8 ? sm.wlo[lane] : 0u;
-            idx = lane < 8 ? sm.widx[lane] : INT_MAX;
+            hi = lane < 8 ? sm.whi[par][lane] : 0u;
+            lo = lane < 8 ? sm.wlo[par][lane] : 0u;
+            idx = lane < 8 ? sm.widx[par][lane] : INT_MAX;
             warp_best(hi, lo, idx);
             const int from_warp = idx == INT_MAX ? 0 : (idx - base) >> 5;
             {  // thread (dest, e) sends element e to CTA dest
                 const int dest = tid / kStrip, e = tid % kStrip;
                 if (dest < G) {
                     const uint32_t bar = peer_address(&sm.bar[par], dest);
-                    send(peer_address(&sm.cand_row[par][rank][e], dest), sm.mine[from_warp][e], bar);
-                    if (rank == 0) send(peer_address(&sm.crow[par][e], dest), sm.top[e], bar);
+                    send(peer_address(&sm.cand_row[par][rank][e], dest), sm.mine[par][from_warp][e], bar);
+                    if (rank == 0) send(peer_address(&sm.crow[par][e], dest), sm.top[par][e], bar);
                     if (e == 0) send(peer_address(&sm.cand_key[par][rank][0], dest), (uint64_t)hi << 32 | lo, bar);
                     if (e == 1) send(peer_address(&sm.cand_key[par][rank][1], dest), (uint64_t)idx, bar);
                 }
