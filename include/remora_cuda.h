@@ -47,11 +47,13 @@ unsigned long long rc_allocation_count(void);
 /* Free every cached workspace of the current device (synchronises the device). */
 int rc_release_workspaces(void);
 /* Failure detection. Every device-side wait (the mbarrier phases of the tensor-core
- * pipelines, the grid barriers of the cooperative getrf panel) is bounded: by the SM's cycle counter, 2 cycles per nanosecond of the limit
+ * pipelines, the grid barriers and the cluster exchange of the getrf panels) is bounded: by
+ * the SM's cycle counter, 2 cycles per nanosecond of the limit
  * set here (default 2 s), i.e. at least that long at SM clocks up to 2 GHz. A wait that
  * runs out records RC_ERR_TIMEOUT and where it happened (kernel * 100 + role * 10 + CTA
  * rank in its cluster; kernels 1 = tcgen05 GEMM, 2 = CTA-pair GEMM, 3 = int8 product,
- * 4 = int8 digit-product trailing update, 5 = getrf panel grid barrier (site 500),
+ * 4 = int8 digit-product trailing update, 5 = getrf panel (site 500: grid barrier; 501:
+ * cluster exchange, which goes on beyond its limit and gives up 2 s later),
  * 9 = self-test; roles 0 = loads, 1 = MMAs, 2 = epilogue) in a per-device error word and
  * its kernel returns, leaving the context usable. The word is sticky: while it is set,
  * every tensor-core kernel returns at once and waits in flight give up, and
@@ -214,7 +216,8 @@ int rc_potrf_f32(int upper, size_t n, float* A, size_t lda, int* d_info, void* s
  * row_major = 1): A = P L U, L unit lower below the diagonal, U on and above it.
  * d_piv (device, n ints): the row swapped with row i at step i, 0-based, applied in the
  * order i = 0, 1, ... (Remora's permutation_matrix). d_info (device): 0, or the 1-based
- * column of the first zero pivot, where the factorisation stops (the reference throws).
+ * column of the first zero pivot, where the factorisation stops (the reference throws); where
+ * a panel's wait gave up, the panel's first column, and rc_device_status has the reason.
  * Replaces kernels::getrf (include/remora/kernels/getrf.hpp:50-59; CPU algorithm
  * kernels/default/getrf.hpp:41-181). */
 int rc_getrf_f64(int row_major, size_t n, double* A, size_t lda, int* d_piv, int* d_info, void* stream);

@@ -346,16 +346,26 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // exists twice, by the column's parity: a wait ends once one warp of every CTA has sent, so a warp may
 // be a column ahead of the others of its CTA, but not two, as the barrier between its candidate and
 // its sending lies in between; and what is sent for a column is sent after its reader has read all of
-// the column before last. Then all agree on the pivot, the two rows swap within the strip, and every row is divided and updated. Per strip, the swaps of the panel's other columns
-// (and of the strip's own finished ones) are gathered through distributed shared memory, the
-// strip's 16 rows of U are solved, and the columns to the right are updated on DMMA. Each element
-// sees the pivot, division and update order of getrf_panel_kernel, a strip's sixteen products
-// summed before they are subtracted.
+// the column before last. Then all agree on the pivot, the two rows swap within the strip, and
+// every row is divided and updated. Per strip, the swaps of the panel's other columns (and of the
+// strip's own finished ones) are gathered through distributed shared memory, the strip's 16 rows
+// of U are solved, and the columns to the right are updated on DMMA. Each element sees the pivot,
+// division and update order of getrf_panel_kernel, a strip's sixteen products summed before they
+// are subtracted.
 // Bound by latency: of a column's ~2400 cycles (8 CTAs) the two-level search for the candidate
 // takes ~1000, sending and waiting ~600 (cluster barriers instead: 860, with 16 CTAs 1400
 // instead of 720), the agreed pivot, the division and the update ~700. 2048 x 64: 104 us (385 on
 // the cooperative grid, whose columns cost a grid barrier and two round trips through L2).
+//
+// Every way out of the column loop is taken by all threads of a CTA at the same barrier, and the
+// panel's end by all CTAs at the same cluster barrier, so that none leaves while another writes or
+// reads its shared memory: what ends the panel (a zero pivot, a message that does not come) is set
+// down in every CTA and looked at after the strip. A wait beyond its limit alone ends nothing: the
+// panel goes on, and the error word tells of it.
 constexpr int kClThreads = 256, kStrip = 16, kClLd = kLuNB + 4, kClMax = 16;
+constexpr int kZeroPivot = 1, kGaveUp = 2;
+constexpr long long kClGrace = 4000000000ll;  // cycles beyond its limit after which a wait gives up
+constexpr long long kClDrain = 1ll << 20;     // cycles in which a message under way arrives
 
 template <class T>
 struct ClusterSmem {
@@ -364,7 +374,9 @@ struct ClusterSmem {
     T crow[2][kStrip];              // row c before the swap
     uint64_t cand_key[2][kClMax][2];  // (hi, lo) of |a[0]|; the row
     uint64_t bar[2];
-    int late;                       // a wait ran out
+    int late;     // a wait took longer than its limit
+    int stop[2];  // by column parity: this CTA's column work ends (kZeroPivot or kGaveUp)
+    int ends;     // why the cluster's panel ends early, 0 if it does not
     int from_all[2 * kStrip], from_strip[2 * kStrip][kStrip], dest[2 * kStrip];
     T mine[2][8][kStrip], top[2][kStrip];  // by column parity: the warps' candidate rows; row c
     T U[kStrip][kLuNB];
@@ -414,8 +426,9 @@ __device__ __forceinline__ void send(uint32_t to, float v, uint32_t bar) {
                  "r"(__float_as_uint(v)), "r"(bar)
                  : "memory");
 }
-// Whether phase `parity` of the mbarrier completed within `limit` cycles.
-__device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity, long long limit) {
+// Waits for phase `parity` of the mbarrier. 0: it completed within `limit` cycles, 1: later, 2: not
+// within kClGrace more.
+__device__ __forceinline__ int wait_phase(uint64_t* bar, unsigned parity, long long limit) {
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
     const long long t0 = clock64();
     while (true) {
@@ -425,8 +438,9 @@ __device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity, long 
             : "=r"(ok)
             : "r"(b), "r"(parity)
             : "memory");
-        if (ok) return true;
-        if (clock64() - t0 > limit) return false;
+        const long long over = clock64() - t0 - limit;
+        if (ok) return over > 0;
+        if (over > kClGrace) return 2;
     }
 }
 
@@ -442,13 +456,18 @@ __global__ void __launch_bounds__(kClThreads, 1)
     if (*(volatile int*)info != 0) return;  // the same for the whole cluster
     const int m = (int)(n - k0);             // rows of the panel; rows are numbered from k0 here
     const int base = rank * kClThreads, row = base + tid;
-    const long long limit = (long long)(limit_ns * 2u);
+    const long long limit = (long long)(limit_ns < 1ull << 61 ? limit_ns * 2u : 1ull << 62);
     if (tid == 0) {
         for (int q = 0; q < 2; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&sm.bar[q])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        sm.late = 0;
+        sm.late = sm.stop[0] = sm.stop[1] = sm.ends = 0;
     }
+    auto end_panel = [&](int par, int why) {  // by whole warps
+        if (lane != 0) return;
+        sm.stop[par] = why;
+        for (int q = 0; q < G; ++q) atomicMax(&cluster.map_shared_rank(&sm, q)->ends, why);
+    };
     T* const prow_mem = sm.P + tid * kClLd;
     if (A.cs == 1) {  // rows contiguous: lanes along the columns
         for (int r = warp; r < kClThreads; r += 8)
@@ -461,6 +480,10 @@ __global__ void __launch_bounds__(kClThreads, 1)
     cluster.sync();  // every CTA runs before any writes to another's shared memory
     const unsigned bytes = (unsigned)(G * (kStrip * sizeof(T) + 16) + kStrip * sizeof(T));  // sent to a CTA per column
     unsigned turn = 0;                                                                     // columns so far
+    int zero_at = 0;  // the zero pivot's column, on the thread that records it
+    auto report_late = [&] {
+        if (tid == 0 && sm.late && err && atomicCAS(err, 0, RC_ERR_TIMEOUT) == 0) atomicExch(err + 1, 501);
+    };
     for (int j0 = 0; j0 < nb; j0 += kStrip) {
         const int w = nb - j0 < kStrip ? nb - j0 : kStrip;
         T a[kStrip];
@@ -497,9 +520,11 @@ __global__ void __launch_bounds__(kClThreads, 1)
                 for (int q = 0; q < kStrip; ++q) sm.top[par][q] = a[q];
             }
             __syncthreads();
+            const int stop = sm.stop[par ^ 1];  // set in the column before, by any warp
             hi = lane < 8 ? sm.whi[par][lane] : 0u;
             lo = lane < 8 ? sm.wlo[par][lane] : 0u;
             idx = lane < 8 ? sm.widx[par][lane] : INT_MAX;
+            if (stop != 0) break;
             warp_best(hi, lo, idx);
             const int from_warp = idx == INT_MAX ? 0 : (idx - base) >> 5;
             {  // thread (dest, e) sends element e to CTA dest
@@ -512,23 +537,26 @@ __global__ void __launch_bounds__(kClThreads, 1)
                     if (e == 1) send(peer_address(&sm.cand_key[par][rank][1], dest), (uint64_t)idx, bar);
                 }
             }
-            if (!wait_phase(&sm.bar[par], turn >> 1 & 1, limit)) sm.late = 1;
+            const int waited = wait_phase(&sm.bar[par], turn >> 1 & 1, limit);
+            if (waited != 0) sm.late = 1;
+            if (__any_sync(0xffffffffu, waited == 2)) {  // what was sent is not read
+                end_panel(par, kGaveUp);
+                continue;
+            }
             hi = lane < G ? (unsigned)(sm.cand_key[par][lane][0] >> 32) : 0u;
             lo = lane < G ? (unsigned)sm.cand_key[par][lane][0] : 0u;
             idx = lane < G ? (int)sm.cand_key[par][lane][1] : INT_MAX;
             warp_best(hi, lo, idx);
-            if (idx != INT_MAX && (idx < c || idx >= m)) idx = INT_MAX;  // after a late wait only
             const int p = idx == INT_MAX ? c : idx;  // nothing but NaN: the row itself
             const T* pr = idx == INT_MAX ? sm.crow[par] : sm.cand_row[par][p / kClThreads];
             const double pv = (double)pr[0];
             if (pv == 0.0) {  // also all-zero columns: the first row is the pivot, value 0
                 if (rank == 0 && tid == 0) {
                     piv[k0 + c] = (int)(k0 + c);
-                    record_first(info, (int)(k0 + c + 1));
+                    zero_at = (int)(k0 + c + 1);
                 }
-                if (sm.late && err && atomicCAS(err, 0, RC_ERR_TIMEOUT) == 0) atomicExch(err + 1, 501);
-                cluster.sync();
-                return;  // the whole cluster
+                end_panel(par, kZeroPivot);
+                continue;
             }
             if (tid == 0) {
                 sm.pivots[jj] = p;
@@ -557,6 +585,15 @@ __global__ void __launch_bounds__(kClThreads, 1)
             }
         }
         cluster.sync();  // P's strip and the pivots are final everywhere
+        if (sm.ends != 0) {  // the same in every CTA
+            if (sm.ends == kGaveUp) {  // the messages that are under way arrive while their CTA is there
+                for (const long long t0 = clock64(); clock64() - t0 < kClDrain;) {}
+                zero_at = rank == 0 && tid == 0 ? (int)(k0 + 1) : 0;  // stops the later kernels: piv is not whole
+            }
+            if (zero_at != 0) record_first(info, zero_at);
+            report_late();
+            return;
+        }
         // The swaps of the other columns, and of the strip's own columns by the later pivots
         // (entries right of a row's diagonal were swapped in registers): destination rows are
         // j0 .. j0 + w and the pivots beyond them; each traces its content back through the swaps.
@@ -658,7 +695,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         __syncthreads();
     }
     cluster.sync();  // no CTA leaves while its shared memory may be read
-    if (tid == 0 && sm.late && err && atomicCAS(err, 0, RC_ERR_TIMEOUT) == 0) atomicExch(err + 1, 501);
+    report_late();
     if (A.cs == 1) {
         for (int r = warp; r < kClThreads; r += 8)
             for (int col = lane; col < nb; col += 32)
