@@ -150,7 +150,8 @@ struct CoopScratch {  // indexed by column j; the barrier words live separately
 // and a wait so that work can run in between: bar[0] counts arrivals, bar[1] is the
 // generation. The wait is bounded by the SM's cycle counter (2 cycles per ns of the
 // library's wait limit); a timeout records RC_ERR_TIMEOUT in the error word and the caller
-// leaves.
+// leaves, with the panel's first column in the status word: piv is not whole, and the later kernels
+// would swap by it.
 __device__ void grid_arrive(unsigned* bar, unsigned nblocks, unsigned gen) {
     __syncthreads();  // every thread's stores before the arrival
     if (threadIdx.x == 0) {
@@ -231,6 +232,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         }
         block_argmax(best, bi, sv, si);
     };
+    auto gave_up = [&] {
+        if (threadIdx.x == 0) record_first(info, (int)(k0 + 1));
+    };
     unsigned gen = 0;
     {  // column 0 needs no update first
         double best;
@@ -238,7 +242,10 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         local_argmax(0, best, bi);
         publish(0, best, bi);
         grid_arrive(bar, (unsigned)G, gen);
-        if (!grid_wait(bar, gen, limit_ns, err, pass)) return;
+        if (!grid_wait(bar, gen, limit_ns, err, pass)) {
+            gave_up();
+            return;
+        }
     }
     for (int j = 0; j < nb; ++j) {
         const int64_t c = k0 + j;
@@ -306,7 +313,10 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
             const T l = row[j];
             for (int col = j + 2; col < nb; ++col) row[col] -= l * (T)prow[col];
         }
-        if (!grid_wait(bar, gen, limit_ns, err, pass)) return;
+        if (!grid_wait(bar, gen, limit_ns, err, pass)) {
+            gave_up();
+            return;
+        }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < myrows * nb; e += kCoopThreads) {
