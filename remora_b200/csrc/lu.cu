@@ -25,7 +25,6 @@
 // columns. piv as for getrf (identity where no swap happened); the rank goes to *rank.
 #include <cooperative_groups.h>
 
-#include <atomic>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -33,6 +32,7 @@
 #include "diag.cuh"
 #include "factor.cuh"
 #include "gemm.cuh"
+#include "per_device.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -926,15 +926,15 @@ void cluster_config(int G, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
 }
 
 // CTAs of the cluster that holds a panel of `rows` rows, 0 where none does: more than 4096 rows,
-// or a device that cannot run such a cluster (asked once per size).
+// or a device that cannot run such a cluster. The kernel's attributes on the device are set with the
+// question.
 template <class T>
 int cluster_size(int64_t rows) {
-    static std::atomic<int> fits[5];  // 0: not asked, 1: yes, 2: no
-    int g = 1, lg = 0;
+    static PerDevice<5> fits;  // by the cluster's size, 1 to 16
+    int g = 1, lg = 0, dev = 0;
     for (; g < kClMax && (int64_t)g * kClThreads < rows; g *= 2) ++lg;
-    if ((int64_t)g * kClThreads < rows) return 0;
-    int f = fits[lg].load(std::memory_order_relaxed);
-    if (f == 0) {
+    if ((int64_t)g * kClThreads < rows || cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const bool fit = fits.get(dev, lg, [&] {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr;
         cluster_config<T>(g, &cfg, &attr);
@@ -945,10 +945,9 @@ int cluster_size(int64_t rows) {
                         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                         cudaOccupancyMaxActiveClusters(&num, kernel, &cfg) == cudaSuccess && num > 0;
         if (!ok) cudaGetLastError();
-        f = ok ? 1 : 2;
-        fits[lg].store(f, std::memory_order_relaxed);
-    }
-    return f == 1 ? g : 0;
+        return ok;
+    });
+    return fit ? g : 0;
 }
 
 // The panel on a cooperative grid of about 256 rows per CTA (a grid barrier costs more the
@@ -971,8 +970,10 @@ int getrf_panel(int64_t n, View<T> A, int64_t k0, int nb, int* piv, int* info, T
         cluster_config<T>(cl, &cfg, &attr);
         cfg.stream = s;
         if (cudaLaunchKernelEx(&cfg, getrf_panel_cluster_kernel<T>, n, A, k0, nb, piv, info, linv, error_word(),
-                               wait_limit_ns()) != cudaSuccess)
+                               wait_limit_ns()) != cudaSuccess) {
+            cudaGetLastError();
             return RC_ERR_CUDA;
+        }
         RC_TRY(check_launch());
         *have_inv = true;
         return RC_SUCCESS;
