@@ -36,6 +36,21 @@ __device__ __forceinline__ bool in_mask(Mask mask, int64_t off, int64_t i, int64
     return true;
 }
 
+// First row and column of this CTA's BM x BN tile of an m x n product, all tiles along grid.x (the
+// other extents end at 65535, too few for the row tiles of a tall product). Grouped order:
+// consecutive CTAs take a group of row tiles (1024 rows) of one column tile before the next
+// column tile, so that a wave holds a few A row blocks and B column blocks in L2 instead of
+// streaming all of B once per row of tiles.
+template <int BM, int BN>
+__device__ __forceinline__ void tile_origin(int64_t m, int64_t n, int64_t* m0, int64_t* n0) {
+    constexpr int64_t kGroupM = 1024 / BM;
+    const int64_t rows = (m + BM - 1) / BM, per = kGroupM * ((n + BN - 1) / BN), lin = blockIdx.x;
+    const int64_t first = lin / per * kGroupM, rest = rows - first;
+    const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
+    *m0 = (first + r % gsz) * BM;
+    *n0 = r / gsz * BN;
+}
+
 // ------------------------------------------------------------------------------------
 // Generic SIMT kernel.
 template <class T>
@@ -178,11 +193,8 @@ __global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
     using LB = SimtLoader<B_KMAJOR, BN, Tile::THREADS, V16>;
     __shared__ __align__(16) float sA[2][BK * LDA];
     __shared__ __align__(16) float sB[2][BK * LDB];
-    constexpr int64_t kGroupM = 1024 / BM;  // grouped tile order, as gemm_dmma_f64
-    const int64_t lin = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, per = kGroupM * gridDim.x;
-    const int64_t first = lin / per * kGroupM, rest = (int64_t)gridDim.y - first;
-    const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
-    const int64_t m0 = (first + r % gsz) * BM, n0 = r / gsz * BN;
+    int64_t m0, n0;
+    tile_origin<BM, BN>(m, n, &m0, &n0);
     if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tm = (warp / Tile::WARPS_N) * 16 + (lane >> 3) * 4, tn = (warp % Tile::WARPS_N) * 32 + (lane & 7) * 4;
@@ -400,14 +412,8 @@ __global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
     extern __shared__ __align__(16) double dsmem[];
     double* sA = dsmem;
     double* sB = dsmem + ST * TA::SIZE;
-    // Grouped tile order: consecutive CTAs take a group of row tiles (1024 rows) of one
-    // column tile before the next column tile, so that a wave holds a few A row blocks and
-    // B column blocks in L2 instead of streaming all of B once per row of tiles.
-    constexpr int64_t kGroupM = 1024 / BM;
-    const int64_t lin = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, per = kGroupM * gridDim.x;
-    const int64_t first = lin / per * kGroupM, rest = (int64_t)gridDim.y - first;
-    const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
-    const int64_t m0 = (first + r % gsz) * BM, n0 = r / gsz * BN;
+    int64_t m0, n0;
+    tile_origin<BM, BN>(m, n, &m0, &n0);
     const bool tri = mask == kLowerTri;
     if (tri) mask = kLower;
     if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
@@ -520,6 +526,14 @@ struct Shape {
     Mask mask;
 };
 
+// The grid of a product's tiles (tile_origin); false where there are more than a grid holds.
+template <class Tile>
+bool tile_grid(const Shape& p, dim3* grid) {
+    const int64_t tiles = ((p.m + Tile::BM - 1) / Tile::BM) * ((p.n + Tile::BN - 1) / Tile::BN);
+    *grid = dim3((unsigned)tiles);
+    return tiles <= INT32_MAX;
+}
+
 // Cycles a product takes with a tile, per the model behind the choice of tiles: an SM works
 // on up to OCC tiles at a time, a k-step of which takes the pipe BM BN / 4 cycles each (it
 // reaches 94% of that with 64 x 64 tiles, 80% with the small ones), but never less than one
@@ -528,7 +542,6 @@ struct Shape {
 template <class Tile>
 double tile_cycles(const Shape& s, int nz) {
     const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
-    if (tm > 65535) return 1e200;  // more row tiles than grid.y holds
     double tiles = (double)tm * tn;
     if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));  // of a square, tm (tm + 1) / 2 tiles run
     const double per_sm = ceil(tiles * nz / sm_count());
@@ -548,7 +561,8 @@ int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const d
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return RC_ERR_CUDA;
-    dim3 grid(ceil_div(p.n, Tile::BN), ceil_div(p.m, Tile::BM));
+    dim3 grid;
+    if (!tile_grid<Tile>(p, &grid)) return RC_ERR_NOT_SUPPORTED;
     if (nz > 1) {
         const int64_t kchunk = ((p.k + nz - 1) / nz + DK - 1) / DK * DK;
         nz = (int)((p.k + kchunk - 1) / kchunk);
@@ -628,7 +642,6 @@ int gemm_dmma(int64_t m, int64_t n, int64_t k, double alpha, View<const double> 
 template <class Tile>
 double simt_cycles(const Shape& s, double eff, double chain) {
     const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
-    if (tm > 65535) return 1e200;
     double tiles = (double)tm * tn;
     if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));
     const double per_sm = ceil(tiles / sm_count()), work = Tile::BM * Tile::BN * Tile::BK / 128.0 / eff;
@@ -641,7 +654,8 @@ template <bool AK, bool BK, class Tile>
 int launch_sgemm(const Shape& p, float alpha, View<const float> A, View<const float> B, float beta, View<float> C,
                  int64_t off, cudaStream_t s, const int* abort) {
     auto aligned = [](const float* q, int64_t ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 4 == 0; };
-    const dim3 grid(ceil_div(p.n, Tile::BN), ceil_div(p.m, Tile::BM));
+    dim3 grid;
+    if (!tile_grid<Tile>(p, &grid)) return RC_ERR_NOT_SUPPORTED;
     if (aligned(A.p, AK ? A.rs : A.cs) && aligned(B.p, BK ? B.cs : B.rs))
         sgemm_simt<AK, BK, Tile, true><<<grid, Tile::THREADS, 0, s>>>(p.m, p.n, p.k, alpha, A, B, beta, C, p.mask, off,
                                                                       abort);
