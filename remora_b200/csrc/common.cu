@@ -59,6 +59,22 @@ void* workspace(cudaStream_t stream, size_t bytes, int slot) {
     return b.ptr;
 }
 
+void* workspace_if_any(cudaStream_t stream, size_t bytes, int slot) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (capture != cudaStreamCaptureStatusNone) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+        std::lock_guard<std::mutex> lock(g_mutex);
+        const auto it = g_buffers.find(std::make_tuple(dev, stream, slot));
+        if (it == g_buffers.end() || it->second.bytes < bytes) return nullptr;
+    }
+    return workspace(stream, bytes, slot);
+}
+
 int* scratch_info(cudaStream_t stream) { return static_cast<int*>(workspace(stream, 256, 15)); }
 
 namespace {

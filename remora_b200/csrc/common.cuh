@@ -49,6 +49,10 @@ int sm_count();
 // on allocation failure. `slot` selects one of a few independent buffers.
 void* workspace(cudaStream_t stream, size_t bytes, int slot = 0);
 
+// The same for a caller that can do without: nullptr also where the buffer would have to grow while
+// the stream is captured into a graph, which an allocation would end.
+void* workspace_if_any(cudaStream_t stream, size_t bytes, int slot);
+
 // Device int used as a per-call status word when the caller passes none.
 int* scratch_info(cudaStream_t stream);
 

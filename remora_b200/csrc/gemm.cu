@@ -15,6 +15,7 @@
 // Both honour a triangle mask (SYRK writes one triangle; whole tiles outside it exit at
 // once) and an abort word (a failed Cholesky pivot stops the trailing updates).
 #include "gemm.cuh"
+#include "gemm_plan.cuh"
 #include "tc_gemm.cuh"
 #include <cmath>
 #include <type_traits>
@@ -310,33 +311,11 @@ __global__ void __launch_bounds__(Tile::THREADS, Tile::OCC)
 // FP64 DMMA kernel. Tiles of BM x BN by a k-step of 16 staged through a cp.async ring, one
 // warp tile of 16 MI x 8 NI per warp. The pipe does 64 FMA per SM and cycle (36.9 TFLOP/s
 // measured on registers alone), so what a shape reaches depends on how evenly its tiles
-// load the SMs and on what a tile spends outside its k loop; pick_tile weighs both.
+// load the SMs and on what a tile spends outside its k loop; pick_tile (gemm_plan.cuh) weighs both.
 // gridDim.z > 1 splits K: slice z covers [z * kchunk, (z + 1) * kchunk) and writes its
 // partial product (alpha = 1, beta = 0) to Cz + z * zstride; a second kernel then reduces
 // the slices into C.
-constexpr int DK = 16;
 constexpr int DKP = DK + 4;  // row stride of a K-major tile (doubles)
-
-template <int BM_, int BN_, int WARPS_M_, int WARPS_N_, int STAGES_, int OCC_>
-struct DmmaTile {
-    static constexpr int BM = BM_, BN = BN_, WARPS_M = WARPS_M_, WARPS_N = WARPS_N_, STAGES = STAGES_;
-    static constexpr int OCC = OCC_;  // CTAs per SM, by shared memory and registers
-    static constexpr int THREADS = 32 * WARPS_M * WARPS_N;
-    static constexpr int WM = BM / WARPS_M, WN = BN / WARPS_N;
-    static constexpr int MI = WM / 16, NI = WN / 8;
-};
-// 64 x 64 with three CTAs per SM is the fastest at every size that fills the GPU: the CTAs'
-// barriers, fills and drains fall at different times, so the pipe always has work. 4096^3:
-// 4.08-4.12 ms (33.7 TFLOP/s), against 4.47-4.72 for one 128 x 128 CTA of 8 warps per SM,
-// 4.10-4.14 for two 128 x 64 of 4 warps, 4.17-4.26 for four 64 x 64 with a two-stage ring
-// and 4.71-4.88 for 32 x 32. Below about one tile per SM the smaller tiles win: 512^3 takes
-// 16.5 us with 32 x 32 and 32.8 us with 64 x 64.
-using TileM = DmmaTile<64, 64, 2, 2, 3, 3>;
-using TileS = DmmaTile<32, 32, 2, 2, 4, 5>;   // small products: latency counts
-using TileT = DmmaTile<64, 16, 4, 1, 4, 4>;   // up to 16 columns
-using TileP = DmmaTile<32, 128, 1, 4, 4, 2>;  // one CTA owns whole rows of a 128-column panel (in place)
-using TileQ = DmmaTile<128, 32, 4, 1, 4, 2>;  // one CTA owns whole columns of a 128-row block (in place)
-using TileR = DmmaTile<128, 16, 4, 1, 4, 2>;  // the same for few columns: half the serial work per CTA
 
 // Shared-memory tile of an operand with ROWS rows (the m or n direction), in the order of
 // its global layout, so that 16-byte copies keep it: K-major tiles are [row][k] with rows
@@ -521,9 +500,9 @@ __global__ void splitk_reduce(int64_t m, int64_t n, int nz, const double* P, int
         }
 }
 
-struct Shape {
-    int64_t m, n, k;
+struct Shape : Problem {
     Mask mask;
+    Shape(int64_t m_, int64_t n_, int64_t k_, Mask mask_) : Problem{m_, n_, k_, mask_ != kFull}, mask(mask_) {}
 };
 
 // The grid of a product's tiles (tile_origin); false where there are more than a grid holds.
@@ -532,24 +511,6 @@ bool tile_grid(const Shape& p, dim3* grid) {
     const int64_t tiles = ((p.m + Tile::BM - 1) / Tile::BM) * ((p.n + Tile::BN - 1) / Tile::BN);
     *grid = dim3((unsigned)tiles);
     return tiles <= INT32_MAX;
-}
-
-// Cycles a product takes with a tile, per the model behind the choice of tiles: an SM works
-// on up to OCC tiles at a time, a k-step of which takes the pipe BM BN / 4 cycles each (it
-// reaches 94% of that with 64 x 64 tiles, 80% with the small ones), but never less than one
-// warp's own chain (its MMAs and ~400 cycles of barrier and fragment loads: 512^3 on 64 x 64
-// tiles, one per SM); a round of tiles pays a fixed fill and drain.
-template <class Tile>
-double tile_cycles(const Shape& s, int nz) {
-    const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
-    double tiles = (double)tm * tn;
-    if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));  // of a square, tm (tm + 1) / 2 tiles run
-    const double per_sm = ceil(tiles * nz / sm_count());
-    const double work = Tile::BM * Tile::BN / 4.0 / (Tile::MI * Tile::NI >= 8 ? 0.94 : 0.80);
-    const double chain = Tile::MI * Tile::NI * 4 * 32 + 400.0, ksteps = ceil((double)s.k / nz / DK);
-    const double full = floor(per_sm / Tile::OCC), rest = per_sm - full * Tile::OCC;
-    auto round = [&](double c) { return c <= 0 ? 0.0 : ksteps * (c * work > chain ? c * work : chain) + 3000.0; };
-    return full * round(Tile::OCC) + round(rest);
 }
 
 template <bool AK, bool BK, class Tile, bool V16>
@@ -563,12 +524,13 @@ int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const d
         return RC_ERR_CUDA;
     dim3 grid;
     if (!tile_grid<Tile>(p, &grid)) return RC_ERR_NOT_SUPPORTED;
-    if (nz > 1) {
+    const int64_t zstride = p.m * p.n;
+    // Without room for the partial products (or a capture under way, in which none can be made) the
+    // same tiles take all of K.
+    double* P = nz > 1 ? static_cast<double*>(workspace_if_any(s, (size_t)nz * zstride * sizeof(double), 7)) : nullptr;
+    if (P) {
         const int64_t kchunk = ((p.k + nz - 1) / nz + DK - 1) / DK * DK;
         nz = (int)((p.k + kchunk - 1) / kchunk);
-        const int64_t zstride = p.m * p.n;
-        double* P = static_cast<double*>(workspace(s, (size_t)nz * zstride * sizeof(double), 7));
-        if (!P) return RC_ERR_ALLOC;
         grid.z = nz;
         kernel<<<grid, Tile::THREADS, smem, s>>>(p.m, p.n, p.k, 1.0, A, B, 0.0, colmajor(P, p.m), kFull, 0, abort,
                                                  kchunk, zstride);
@@ -580,8 +542,6 @@ int launch_dmma(const Shape& p, double alpha, View<const double> A, View<const d
     kernel<<<grid, Tile::THREADS, smem, s>>>(p.m, p.n, p.k, alpha, A, B, beta, C, p.mask, off, abort, p.k, 0);
     return check_launch();
 }
-
-enum TileId { kTileM, kTileS, kTileT, kTileP, kTileQ, kTileR };
 
 template <bool AK, bool BK, bool V16>
 int launch_tile(TileId id, const Shape& p, double alpha, View<const double> A, View<const double> B, double beta,
@@ -596,40 +556,13 @@ int launch_tile(TileId id, const Shape& p, double alpha, View<const double> A, V
     }
 }
 
-// The tile and K split of least modelled time. A product that writes over one of its own
-// operands (C on A with n <= 128, or on B with m <= 128) takes a tile that spans that
-// operand's rows or columns: each CTA has then read all of what it overwrites.
-void pick_tile(const Shape& p, bool c_on_a, bool c_on_b, bool may_split, TileId* id, int* nz) {
-    double best = 1e300;
-    auto look = [&](TileId t, double cycles, int z) {
-        if (cycles < best) {
-            best = cycles;
-            *id = t;
-            *nz = z;
-        }
-    };
-    if (c_on_a || c_on_b) {
-        *id = c_on_a ? kTileP : p.n <= 16 * (int64_t)sm_count() ? kTileR : kTileQ;
-        *nz = 1;
-        return;
-    }
-    // A split pays a second launch and two passes over its partial products.
-    const int zmax = may_split ? 8 : 1;
-    for (int z = 1; z <= zmax && (z == 1 || (int64_t)z * 512 <= p.k); ++z) {
-        const double extra = z > 1 ? 6000.0 + 16.0 * z * p.m * p.n / 2500.0 : 0.0;
-        look(kTileM, tile_cycles<TileM>(p, z) + extra, z);
-        look(kTileS, tile_cycles<TileS>(p, z) + extra, z);
-        if (p.n <= 16) look(kTileT, tile_cycles<TileT>(p, z) + extra, z);
-    }
-}
-
 template <bool AK, bool BK>
 int gemm_dmma(int64_t m, int64_t n, int64_t k, double alpha, View<const double> A, View<const double> B, double beta,
               View<double> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
-    const Shape p{m, n, k, mask};
+    const Shape p(m, n, k, mask);
     TileId id = kTileM;
     int nz = 1;
-    pick_tile(p, C.p == A.p, C.p == B.p, mask == kFull && k >= 2048, &id, &nz);
+    pick_tile(p, C.p == A.p, C.p == B.p, mask == kFull && k >= 2048, sm_count(), &id, &nz);
     auto even = [](const double* q, int64_t ld) { return reinterpret_cast<uintptr_t>(q) % 16 == 0 && ld % 2 == 0; };
     if (even(A.p, AK ? A.rs : A.cs) && even(B.p, BK ? B.cs : B.rs))
         return launch_tile<AK, BK, true>(id, p, alpha, A, B, beta, C, off, nz, s, abort);
@@ -643,7 +576,7 @@ template <class Tile>
 double simt_cycles(const Shape& s, double eff, double chain) {
     const int64_t tm = (s.m + Tile::BM - 1) / Tile::BM, tn = (s.n + Tile::BN - 1) / Tile::BN;
     double tiles = (double)tm * tn;
-    if (s.mask != kFull) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));
+    if (s.triangle) tiles = 0.5 * (tiles + (tm > tn ? tm : tn));
     const double per_sm = ceil(tiles / sm_count()), work = Tile::BM * Tile::BN * Tile::BK / 128.0 / eff;
     const double ksteps = ceil((double)s.k / Tile::BK), full = floor(per_sm / Tile::OCC), rest = per_sm - full * Tile::OCC;
     auto round = [&](double c) { return c <= 0 ? 0.0 : ksteps * (c * work > chain ? c * work : chain) + 3000.0; };
@@ -668,7 +601,7 @@ int launch_sgemm(const Shape& p, float alpha, View<const float> A, View<const fl
 template <bool AK, bool BK>
 int sgemm(int64_t m, int64_t n, int64_t k, float alpha, View<const float> A, View<const float> B, float beta,
           View<float> C, Mask mask, int64_t off, cudaStream_t s, const int* abort) {
-    const Shape p{m, n, k, mask};
+    const Shape p(m, n, k, mask);
     // A product that writes over one of its own operands (C on B with m <= 128, on A with n <= 64)
     // takes the tile that spans that operand's rows or columns, as in pick_tile.
     const bool in_place = C.p == A.p || C.p == B.p;
