@@ -398,7 +398,9 @@ template <class T>
 int launch_plain(const Plan& p, Config c, cudaStream_t s) {
     const size_t smem = BatchedSmem::bytes(*std::max_element(p.sizes.begin(), p.sizes.end()));
     auto fn = kernel_for<T>(c);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    // always the limit of the tallest batch: kept plans and other threads share the attribute
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BatchedSmem::bytes(kMaxN)) !=
+        cudaSuccess)
         return RC_ERR_CUDA;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * c.warps, smem) != cudaSuccess || per_sm < 1)
