@@ -114,8 +114,9 @@ __device__ __forceinline__ double rsqrt_normal(double d) {
 // 16 x 16 block to factor and the 16 rows below it): a becomes L's row, column j of L goes to
 // Lt + j * kLTD, L(j, j) to ld and its reciprocal to rd; arrive(h) is called once columns
 // 8 h .. 8 h + 7 are there. flags[0] = 1 + column of the first non-positive (or NaN)
-// pivot, 0 if there is none; after one the values are void. flags[1] = 1 where a pivot is too
-// small for rsqrt_normal, and the result is void.
+// pivot, 0 if there is none; after one the values are void. flags[1] = 1 where any pivot is below
+// 1e-300, negative ones included, and so perhaps too small for rsqrt_normal: the pivots after it may
+// be infinite or NaN whatever the matrix, so the result is void, the failing column included.
 template <class Arrive>
 __device__ __forceinline__ void factor_sub_block(double (&a)[kDB], double* Lt, double* ld, double* rd, int lane,
                                                  volatile int* flags, Arrive arrive) {
@@ -143,7 +144,7 @@ __device__ __forceinline__ void factor_sub_block(double (&a)[kDB], double* Lt, d
             r = rsqrt_normal(d);
         } else if (lane == 0) {
             flags[0] = bad;
-            flags[1] = tiny && bad == 0;
+            flags[1] = tiny;
         }
         __syncwarp();
         if (j % 8 == 7) arrive(j / 8);
