@@ -20,7 +20,7 @@
 //    substitution walks the panels with the kept inverses;
 //  * a failing pivot records its 1-based index in info[i] and the CTA moves on.
 // The warps per CTA are chosen per (precision, size bucket) by a small autotuner that times
-// every candidate on the caller's batch once and caches the winner.
+// every candidate on the caller's batch, loaded and warm, and caches the winner.
 //
 // 1024 systems of 16 to 512 rows: 1.04 ms in FP64, 1.00 ms in FP32 (12.3 and 10.4 ms with FMA
 // tiles over a right-looking update and one barrier per column), 11.9 GFLOP of which the DMMA
@@ -413,7 +413,9 @@ int launch_plain(const Plan& p, Config c, cudaStream_t s) {
 }
 
 // Time each candidate once on the caller's batch (the factorisations happen in place, so
-// the caller's matrices are first saved and restored around the tuning runs).
+// the caller's matrices are first saved and restored around the tuning runs). A first run of all
+// is not timed: it loads the kernels, which takes longer than they run and by chance differs
+// between them (1 process of 6 kept 4 warps, 1.47 ms for 1024 systems, where 8 take 1.04).
 template <class T>
 int autotune(Plan& p, cudaStream_t s) {
     const auto key = std::make_pair((int)sizeof(T), size_bucket(p.sizes));
@@ -454,6 +456,8 @@ int autotune(Plan& p, cudaStream_t s) {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
+    for (const Config& c : kCandidates) launch_plain<T>(p, c, s);  // (the later ones on what the first left)
+    copy_all(false);
     for (const Config& c : kCandidates) {
         cudaEventRecord(e0, s);
         const int st = launch_plain<T>(p, c, s);
