@@ -11,6 +11,7 @@
 // indices (the reference writes past the matrix when cols % 64 != 0, :172, :186), and
 // threads that keep their place along the contiguous direction and walk the other one.
 #include "common.cuh"
+#include "sincos_2pi.cuh"
 #include <cmath>
 
 namespace rc {
@@ -57,7 +58,7 @@ __device__ __forceinline__ float uniform1(uint32_t x, float low, float range) {
 }
 
 // The fills are bound by instruction issue, so the normal transform's functions cover just the
-// arguments it has. 2^28 normals (16384 x 16384, row-major): 705 -> 449 us; the general
+// arguments it has. 2^28 normals (16384 x 16384, row-major): 705 -> 457 us; the general
 // library functions branch around cases that do not occur here.
 
 // Bit pattern of nextafter(unit_float(x), 0): one less than the float's for x > 0, else 0.
@@ -90,22 +91,6 @@ __device__ __forceinline__ float sqrt_m2log(int bits) {
     const float r = t * y;
     const float root = __fmaf_rn(__fmaf_rn(-r, r, t), 0.5f * y, r);
     return bits == 0 ? __int_as_float(0x7f800000) : root;
-}
-
-// Sine and cosine of q = 2 pi u rounded to a float, 0 <= u < 1: q less the nearest multiple of pi / 2
-// (in two parts, Cody and Waite), then polynomials on [-pi/4, pi/4] fitted as above: within 1.5
-// ulp.
-__device__ __forceinline__ void sincos_2pi(float u, float* sine, float* cosine) {
-    const float q = (2.0f * 3.14159265358979323846f) * u;
-    const float biased = __fmaf_rn(u, 4.0f, 12582912.0f), kf = biased - 12582912.0f;
-    const int k = __float_as_int(biased);
-    const float r = __fmaf_rn(-kf, -0x1.777a5cp-25f, __fmaf_rn(-kf, 0x1.921fb6p+0f, q)), z = r * r;
-    const float ps = __fmaf_rn(__fmaf_rn(-0x1.994386p-13f, z, 0x1.11073ap-7f), z, -0x1.555546p-3f);
-    const float pc = __fmaf_rn(__fmaf_rn(0x1.99eb4ap-16f, z, -0x1.6c0c32p-10f), z, 0x1.55554ap-5f);
-    const float s = __fmaf_rn(ps * z, r, r), c = __fmaf_rn(z, __fmaf_rn(z, pc, -0.5f), 1.0f);
-    const bool odd = k & 1;
-    *sine = __int_as_float(__float_as_int(odd ? c : s) ^ ((k << 30) & 0x80000000));
-    *cosine = __int_as_float(__float_as_int(odd ? s : c) ^ (((k + 1) << 30) & 0x80000000));
 }
 
 enum Kind { kBits = 0, kUniform = 1, kNormal = 2, kDiscreteF = 3, kDiscreteI = 4 };
