@@ -4,14 +4,12 @@
 // (include/remora/hip/cublas_backend.hpp:121-166, :389-431, called from
 // include/remora/kernels/hip/gemm.hpp:46-112 and kernels/hip/syrk.hpp:44-85).
 //
-// Three kernels:
+// Two kernels:
 //  * gemm_dmma_f64: the FP64 tensor-core path (DMMA, mma.sync m16n8k4 f64), a family of
 //    CTA tiles from 128 x 128 down to 32 x 32 over one kernel template. Operand tiles are
 //    staged by 16-byte cp.async (8-byte where the alignment asks for it) in the order of
 //    their global layout, so all four transpose combinations run at the same rate.
 //  * sgemm_simt: FP32 on the FMA units, register tiles of packed pairs.
-//  * gemm_simt: a generic strided kernel (64x64x16 tiles, 4x4 outer products per thread) for
-//    operands with no unit stride.
 // Both honour a triangle mask (SYRK writes one triangle; whole tiles outside it exit at
 // once) and an abort word (a failed Cholesky pivot stops the trailing updates).
 #include "gemm.cuh"
@@ -50,62 +48,6 @@ __device__ __forceinline__ void tile_origin(int64_t m, int64_t n, int64_t* m0, i
     const int64_t gsz = rest < kGroupM ? rest : kGroupM, r = lin % per;
     *m0 = (first + r % gsz) * BM;
     *n0 = r / gsz * BN;
-}
-
-// ------------------------------------------------------------------------------------
-// Generic SIMT kernel.
-template <class T>
-__global__ void __launch_bounds__(256) gemm_simt(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A,
-                                                 View<const T> B, T beta, View<T> C, Mask mask, int64_t off,
-                                                 const int* abort) {
-    constexpr int BM = 64, BN = 64, BK = 16;
-    __shared__ T sA[BK][BM + 1];
-    __shared__ T sB[BK][BN + 1];
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-    if (aborted(abort) || tile_outside(mask, off, m0, n0, BM, BN)) return;
-    const int tid = threadIdx.x;
-    const int tm = tid / 16, tn = tid % 16;  // 16 x 16 threads, 4 x 4 each
-    T acc[4][4] = {};
-    for (int64_t k0 = 0; k0 < k; k0 += BK) {
-        for (int e = tid; e < BM * BK; e += 256) {
-            // A tile: consecutive threads walk the unit-stride direction when there is one.
-            int mm, kk;
-            if (A.rs == 1) { mm = e % BM; kk = e / BM; } else { kk = e % BK; mm = e / BK; }
-            const int64_t gi = m0 + mm, gk = k0 + kk;
-            sA[kk][mm] = (gi < m && gk < k) ? A(gi, gk) : T(0);
-            int nn, kb;
-            if (B.cs == 1) { nn = e % BN; kb = e / BN; } else { kb = e % BK; nn = e / BK; }
-            const int64_t gj = n0 + nn, gk2 = k0 + kb;
-            sB[kb][nn] = (gj < n && gk2 < k) ? B(gk2, gj) : T(0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            T a[4], b[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = sA[kk][tm + 16 * r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = sB[kk][tn + 16 * c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int64_t i = m0 + tm + 16 * r;
-        if (i >= m) continue;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t j = n0 + tn + 16 * c;
-            if (j >= n || !in_mask(mask, off, i, j)) continue;
-            T v = alpha * acc[r][c];
-            if (beta != T(0)) v = fma(beta, C(i, j), v);
-            C(i, j) = v;
-        }
-    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -633,21 +575,17 @@ int gemm(int64_t m, int64_t n, int64_t k, T alpha, View<const T> A, View<const T
         return check_launch();
     }
     const bool a_k = A.cs == 1, a_m = A.rs == 1, b_k = B.rs == 1, b_n = B.cs == 1;
-    if ((a_k || a_m) && (b_k || b_n)) {
-        auto run = [&](auto ak, auto bk) {
-            if constexpr (std::is_same<T, double>::value)
-                return gemm_dmma<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, asked, off, s, abort);
-            else
-                return sgemm<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
-        };
-        if (a_k && b_k) return run(std::true_type{}, std::true_type{});
-        if (a_k) return run(std::true_type{}, std::false_type{});
-        if (b_k) return run(std::false_type{}, std::true_type{});
-        return run(std::false_type{}, std::false_type{});
-    }
-    dim3 grid(ceil_div(n, 64), ceil_div(m, 64));
-    gemm_simt<T><<<grid, 256, 0, s>>>(m, n, k, alpha, A, B, beta, C, mask, off, abort);
-    return check_launch();
+    if (!(a_k || a_m) || !(b_k || b_n)) return RC_ERR_NOT_SUPPORTED;
+    auto run = [&](auto ak, auto bk) {
+        if constexpr (std::is_same<T, double>::value)
+            return gemm_dmma<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, asked, off, s, abort);
+        else
+            return sgemm<ak.value, bk.value>(m, n, k, alpha, A, B, beta, C, mask, off, s, abort);
+    };
+    if (a_k && b_k) return run(std::true_type{}, std::true_type{});
+    if (a_k) return run(std::true_type{}, std::false_type{});
+    if (b_k) return run(std::false_type{}, std::true_type{});
+    return run(std::false_type{}, std::false_type{});
 }
 
 template int gemm<double>(int64_t, int64_t, int64_t, double, View<const double>, View<const double>, double,

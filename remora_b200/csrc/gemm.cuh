@@ -11,7 +11,8 @@ namespace rc {
 // the FP64 tiles leave out the k before their first row.
 enum Mask { kFull = 0, kLower = 1, kUpper = 2, kLowerTri = 3 };
 
-// C <- alpha * A * B + beta * C (A m x k, B k x n, C m x n, arbitrary strided views).
+// C <- alpha * A * B + beta * C (A m x k and B k x n row- or column-major, C m x n any strided view;
+// RC_ERR_NOT_SUPPORTED for an operand without a unit stride).
 // beta == 0 does not read C. abort (device int, may be null): when *abort != 0 at launch
 // time the kernel returns without touching C (used after a failed Cholesky pivot).
 template <class T>
