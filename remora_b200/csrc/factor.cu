@@ -4,12 +4,14 @@
 // trsm.hpp:45-107 -> cublas trsm; include/remora/kernels/hip/potrf.hpp:41-141, a
 // recursive split whose 16x16 leaves are factored by a single thread). Here:
 //  * TRSM: every 128x128 diagonal block of the triangle is inverted at once (one CTA
-//    per block, FP64 in shared memory); the solve then walks the block rows, each step
-//    one GEMM with the inverted block and one GEMM update of the remaining rows, so
-//    nearly all flops run in the tensor-core GEMM.
-//  * POTRF: per 128-wide panel, one CTA factors the diagonal block in FP64 shared
-//    memory (and inverts it), the panel below is solved by a GEMM with that inverse,
-//    and the trailing matrix is updated by a lower-masked GEMM (the SYRK schedule).
+//    per block, FP64 in shared memory); the solve then walks panels of 512 rows, each
+//    solved in strips of a few right-hand sides per CTA (strip.cu) and followed by one
+//    GEMM update of the remaining rows, where nearly all flops are.
+//  * POTRF: panels of 512 columns. Inside a panel's diagonal block, per 128 columns, one
+//    CTA factors the diagonal block in FP64 shared memory (and inverts it), the rows below
+//    it are solved in strips and the rest of the block is updated; then the rows below the
+//    panel are solved in strips through all of its 128-column steps, and the trailing
+//    matrix is updated by a lower-masked GEMM of depth 512 (the SYRK schedule).
 //    A non-positive pivot writes its global index to the status word and every later
 //    kernel of the factorization returns at once.
 #include "factor.cuh"

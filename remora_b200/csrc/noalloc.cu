@@ -4,9 +4,10 @@
 // whose device memory is reserved up front by their own pool allocator (a cudaMalloc
 // from the library would fail or escape their accounting), and latency-bound loops in
 // which cudaMalloc/cudaFree, which can synchronise the whole device, are not allowed.
-// For them this entry point runs the same Cholesky factorisation and the same two
-// triangular solves as rc_spd_solve_f64, on scratch that lives in one file-scope
-// __device__ array instead of the library's cached workspaces.
+// For them this entry point factors and solves on scratch that lives in one file-scope
+// __device__ array instead of the library's cached workspaces. It takes 128-column steps: the
+// diagonal block of rc_spd_solve_f64, then products with its inverse and updates of all that
+// follows, a launch each (rc_spd_solve_f64 solves its panels in strips, strip.cu, which are faster).
 //
 // The array holds 9.19 MiB: the n x n copy of A (n <= 1024), the inverse of one
 // diagonal block for the factorisation and of the eight diagonal blocks for the solves,
@@ -56,7 +57,8 @@ double* scratch_address() {
 }
 
 // B <- L^-1 B (upper = false) or L^-T B (upper = true) with the diagonal-block inverses
-// already in Winv (column-major blocks); the same block loop as the allocating solve.
+// already in Winv (column-major blocks): per block row the product with its inverse into the
+// tile, the copy back and the update of all other rows.
 int solve_with_inverses(bool upper, int64_t n, int64_t nrhs, View<const double> L, const double* Winv,
                         View<double> B, double* tile, cudaStream_t s, const int* abort) {
     const int64_t nblk = (n + kNB - 1) / kNB;

@@ -5,11 +5,11 @@
 // stream is the reference's, bit for bit: same counter per (row, 4-column group)
 // (:167, :181), same key schedule including the reference's third key injection
 // (:102-106), same float transforms (:110-132) with the multiply-adds fused as nvcc
-// compiles them. The layout differs: one thread per 4-element group, threads laid out
-// along the storage's contiguous direction so each warp store is one or four 128-byte
-// segments (16-byte vector stores for aligned row-major rows), a bounds check on both
-// indices (the reference writes past the matrix when cols % 64 != 0, :172, :186), and
-// threads that keep their place along the contiguous direction and walk the other one.
+// compiles them. The layout differs: a thread keeps its place along the storage's
+// contiguous direction (a 4-column group, or a row) and walks the other one, a 4-element
+// group a step, so each warp store is one or four 128-byte segments (16-byte vector stores
+// for aligned row-major rows), with a bounds check on both indices (the reference writes
+// past the matrix when cols % 64 != 0, :172, :186).
 #include "common.cuh"
 #include "sincos_2pi.cuh"
 #include <cmath>
