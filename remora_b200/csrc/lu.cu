@@ -370,8 +370,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // Every way out of the column loop is taken by all threads of a CTA at the same barrier, and the
 // panel's end by all CTAs at the same cluster barrier, so that none leaves while another writes or
 // reads its shared memory: what ends the panel (a zero pivot, a message that does not come) is set
-// down in every CTA and looked at after the strip. A wait beyond its limit alone ends nothing: the
-// panel goes on, and the error word tells of it.
+// down in every CTA and looked at after the strip. (It is set down behind the loop: a way back into
+// the loop would keep two places for every a[q], 5% of a panel's time.) A wait beyond its limit alone
+// ends nothing: the panel goes on, and the error word tells of it.
 constexpr int kClThreads = 256, kStrip = 16, kClLd = kLuNB + 4, kClMax = 16;
 constexpr int kZeroPivot = 1, kGaveUp = 2;
 constexpr long long kClGrace = 4000000000ll;  // cycles beyond its limit after which a wait gives up
@@ -502,8 +503,9 @@ __global__ void __launch_bounds__(kClThreads, 1)
 #pragma unroll
             for (int q = 0; q < kStrip; ++q) a[q] = src[q];
         }
+        int jj = 0, ends = 0;
 #pragma unroll 1
-        for (int jj = 0; jj < w; ++jj, ++turn) {
+        for (; jj < w; ++jj, ++turn) {
             const int c = j0 + jj, par = turn & 1;
             if (tid == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
@@ -550,8 +552,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
             const int waited = wait_phase(&sm.bar[par], turn >> 1 & 1, limit);
             if (waited != 0) sm.late = 1;
             if (__any_sync(0xffffffffu, waited == 2)) {  // what was sent is not read
-                end_panel(par, kGaveUp);
-                continue;
+                ends = kGaveUp;
+                break;
             }
             hi = lane < G ? (unsigned)(sm.cand_key[par][lane][0] >> 32) : 0u;
             lo = lane < G ? (unsigned)sm.cand_key[par][lane][0] : 0u;
@@ -565,8 +567,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
                     piv[k0 + c] = (int)(k0 + c);
                     zero_at = (int)(k0 + c + 1);
                 }
-                end_panel(par, kZeroPivot);
-                continue;
+                ends = kZeroPivot;
+                break;
             }
             if (tid == 0) {
                 sm.pivots[jj] = p;
@@ -593,6 +595,10 @@ __global__ void __launch_bounds__(kClThreads, 1)
                 for (int q = 0; q + 1 < kStrip; ++q)
                     if (jj + 1 + q < w) prow_mem[c + 1 + q] = a[q];
             }
+        }
+        if (ends != 0) {
+            end_panel(turn & 1, ends);
+            if (jj + 1 < w) __syncthreads();  // the other warps' next column, where they look at stop
         }
         cluster.sync();  // P's strip and the pivots are final everywhere
         if (sm.ends != 0) {  // the same in every CTA
