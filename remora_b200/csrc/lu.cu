@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // are subtracted.
 // Bound by latency: of a column's ~2400 cycles (8 CTAs) the two-level search for the candidate
 // takes ~1000, sending and waiting ~600 (cluster barriers instead: 860, with 16 CTAs 1400
-// instead of 720), the agreed pivot, the division and the update ~700. 2048 x 64: 104 us (385 on
+// instead of 720), the agreed pivot, the division and the update ~700. 2048 x 64: about 105 us (385 on
 // the cooperative grid, whose columns cost a grid barrier and two round trips through L2).
 //
 // Every way out of the column loop is taken by all threads of a CTA at the same barrier, and the
