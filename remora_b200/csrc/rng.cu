@@ -139,8 +139,9 @@ __global__ void __launch_bounds__(256) fill_rowmajor(typename Out<K>::type* __re
          g += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t j = 4 * g;
         const uint32_t cz = (uint32_t)(j & 0xffffu), cw = (uint32_t)(j >> 32);
-        T* out = A + blockIdx.y * ld + j;
-        for (uint64_t i = blockIdx.y; i < rows; i += gridDim.y, out += gridDim.y * ld) {
+        const uint64_t first = (uint64_t)blockIdx.y * blockDim.y + threadIdx.y, step = (uint64_t)gridDim.y * blockDim.y;
+        T* out = A + first * ld + j;
+        for (uint64_t i = first; i < rows; i += step, out += step * ld) {
             T v[4];
             transform<K>(threefry(make_uint4((uint32_t)(i & 0xffffu), (uint32_t)(i >> 32), cz, cw), key), a, b, ia, N,
                          v);
@@ -168,8 +169,9 @@ __global__ void __launch_bounds__(256) fill_colmajor(typename Out<K>::type* __re
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t cx = (uint32_t)(i & 0xffffu), cy = (uint32_t)(i >> 32);
-        T* out = A + i + 4 * blockIdx.y * ld;
-        for (uint64_t g = blockIdx.y; g < groups; g += gridDim.y, out += 4 * gridDim.y * ld) {
+        const uint64_t first = (uint64_t)blockIdx.y * blockDim.y + threadIdx.y, step = (uint64_t)gridDim.y * blockDim.y;
+        T* out = A + i + 4 * first * ld;
+        for (uint64_t g = first; g < groups; g += step, out += 4 * step * ld) {
             const uint64_t j = 4 * g;
             T v[4];
             transform<K>(threefry(make_uint4(cx, cy, (uint32_t)(j & 0xffffu), (uint32_t)(j >> 32)), key), a, b, ia, N,
@@ -198,19 +200,24 @@ int launch_fill(const uint32_t key[4], size_t rows, size_t cols, void* Av, size_
     T* A = static_cast<T*>(Av);
     const uint4 k = make_uint4(key[0], key[1], key[2], key[3]);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // Along x a block covers the contiguous direction; along y, threads of as many blocks as fill
-    // the SMs four times over share the steps of the other one: enough that the last ones to
-    // finish cost little, few enough that their prologues do.
+    // Along x a block covers the contiguous direction, several steps of the other one where that is
+    // short (2^20 x 64 normals, row-major: 278 us with a step per block); along y, threads of as many
+    // blocks as fill the SMs four times over share the steps: enough that the last ones to finish
+    // cost little, few enough that their prologues do.
     constexpr unsigned threads = 256;
     const uint64_t groups = (cols + 3) / 4, along = row_major ? groups : rows, steps = row_major ? rows : groups;
-    const unsigned gx = ceil_div(along, threads) < 65535u ? ceil_div(along, threads) : 65535u;
-    const uint64_t share = ceil_div((uint64_t)sm_count() * 32, gx);
-    const dim3 grid(gx, (unsigned)(steps < share ? steps : share));
+    unsigned bx = 1;
+    while (bx < threads && bx < along) bx *= 2;
+    const dim3 block(bx, threads / bx);
+    const uint64_t blocks = (uint64_t)sm_count() * 32, whole = (along + bx - 1) / bx;
+    const unsigned gx = (unsigned)(whole < blocks ? whole : blocks);
+    const uint64_t share = ceil_div(blocks, gx), most = (steps + block.y - 1) / block.y;
+    const dim3 grid(gx, (unsigned)(most < share ? most : share));
     if (row_major) {
         const bool vec_ok = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (ld % 4 == 0);
-        fill_rowmajor<K><<<grid, threads, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N, vec_ok);
+        fill_rowmajor<K><<<grid, block, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N, vec_ok);
     } else {
-        fill_colmajor<K><<<grid, threads, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N);
+        fill_colmajor<K><<<grid, block, 0, s>>>(A, ld, rows, cols, k, a, b, ia, N);
     }
     return check_launch();
 }
