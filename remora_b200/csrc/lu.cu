@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         for (int col = 0; col < kLuNB; ++col)
             if (col < nb) A(k0 + row, k0 + col) = prow_mem[col];
     }
-    if (rank != 0) return;
+    if (rank != 0 || m == nb) return;  // nothing right of the last panel
     // inv(L11), unit lower (the identity beyond nb), for U12 = inv(L11) A12 right of the panel:
     // 16-blocks by a warp each, then merges (diag.cuh)
 #pragma unroll 8
