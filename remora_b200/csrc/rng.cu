@@ -58,7 +58,7 @@ __device__ __forceinline__ float uniform1(uint32_t x, float low, float range) {
 }
 
 // The fills are bound by instruction issue, so the normal transform's functions cover just the
-// arguments it has. 2^28 normals (16384 x 16384, row-major): 705 -> 457 us; the general
+// arguments it has. 2^28 normals (16384 x 16384, row-major): 705 -> 451 us; the general
 // library functions branch around cases that do not occur here.
 
 // Bit pattern of nextafter(unit_float(x), 0): one less than the float's for x > 0, else 0.
@@ -201,7 +201,7 @@ int launch_fill(const uint32_t key[4], size_t rows, size_t cols, void* Av, size_
     const uint4 k = make_uint4(key[0], key[1], key[2], key[3]);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Along x a block covers the contiguous direction, several steps of the other one where that is
-    // short (2^20 x 64 normals, row-major: 278 us with a step per block); along y, threads of as many
+    // short (2^20 x 64 normals, row-major: 114 us, 278 with a step per block); along y, threads of as many
     // blocks as fill the SMs four times over share the steps: enough that the last ones to finish
     // cost little, few enough that their prologues do.
     constexpr unsigned threads = 256;

@@ -5,7 +5,7 @@ namespace rc {
 
 // Sine and cosine of q = 2 pi u rounded to a float, 0 <= u < 1: q less the nearest multiple of pi / 2
 // (in three parts, Cody and Waite: at u = 3/4 what is left of q is 1.2e-8, and two parts leave 5.8 ulp
-// of error in the cosine; the third takes 8 of a fill's 457 us), then polynomials on [-pi/4, pi/4] fitted as the logarithm's:
+// of error in the cosine; the third takes 8 of a fill's 451 us), then polynomials on [-pi/4, pi/4] fitted as the logarithm's:
 // within 1.5 ulp.
 __device__ __forceinline__ void sincos_2pi(float u, float* sine, float* cosine) {
     const float q = (2.0f * 3.14159265358979323846f) * u;
